@@ -95,10 +95,6 @@ struct tbsla_matrix {
   // items (long rows and chunks of huge rows), huge rows, chunk partials
   int *short_rows = nullptr;
   int n_short = 0;
-  // the first n_tiny entries of short_rows hold every short row of at most
-  // kTinyRow entries (empty ones included), when there are many of them:
-  // reducing epilogues (PageRank sweeps) run them in warp tiles
-  int n_tiny = 0;
   int64_t short_nnz = 0;  // entries of the short rows
   int short_max = 0;      // entries of the longest short row (<= kTinyRow, all rows
                           // short and in order: the tiny-row warp tiles)
@@ -151,6 +147,11 @@ struct tbsla_matrix {
   // PageRank workspace built on first use (pagerank.cu)
   void *pr_work = nullptr;
   void (*pr_work_free)(void *) = nullptr;
+  bool pr_dmask_stale = false;       // the values changed since pr_work's dangling mask
+  unsigned char *col_pattern = nullptr;  // columns without a stored entry (column_mask.cuh)
+  // row classes of the PageRank solver (pagerank.cu; the row structure only)
+  void *pr_plan = nullptr;
+  void (*pr_plan_free)(void *) = nullptr;
   unsigned char *dangling = nullptr;
   double *pr_scratch = nullptr;
   // PageRank on a relabelled copy (pr_relabel.cu): vertices in decreasing

@@ -131,7 +131,7 @@ __device__ __forceinline__ Acc row_sum_thread(const int *__restrict__ colidx, co
 }
 
 // short rows: rows [0, n_rows) when `rows` is NULL, else rows[0..n_rows);
-// grid-stride (one row per thread unless the epilogue caps the grid)
+// one row per thread
 template <typename V, typename XT, typename Epi>
 __global__ void __launch_bounds__(256) csr_short_kernel(const int *__restrict__ rows, int n_rows,
                                                        const int *__restrict__ rowptr,
@@ -140,42 +140,13 @@ __global__ void __launch_bounds__(256) csr_short_kernel(const int *__restrict__ 
                                                        const XT *__restrict__ x, int f_col, XKeep x_keep,
                                                        Epi epi) {
   using Acc = typename Epi::Acc;
-  if (!epi.active()) return;
-  typename Epi::State es{};
   const uint64_t keep = policy_keep(x_keep, x);
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if constexpr (!Epi::kReduces) {
-    // one row per thread (uncapped grid)
-    for (; t < n_rows; t += stride) {
-      const int r = rows ? __ldg(rows + t) : (int)t;
-      const int a = __ldg(rowptr + r), b = __ldg(rowptr + r + 1);
-      epi.emit(r, row_sum_thread<V, XT, Acc>(colidx, values, x, f_col, a, b, keep), es);
-    }
-  } else {
-    // the next row's bounds are loaded before the current row is summed, so
-    // their latency overlaps the sum (capped grids give a thread many rows)
-    int r = 0, a = 0, b = 0;
-    if (t < n_rows) {
-      r = rows ? __ldg(rows + t) : (int)t;
-      a = __ldg(rowptr + r);
-      b = __ldg(rowptr + r + 1);
-    }
-    for (; t < n_rows; t += stride) {
-      const int64_t tn = t + stride;
-      int rn = 0, an = 0, bn = 0;
-      if (tn < n_rows) {
-        rn = rows ? __ldg(rows + tn) : (int)tn;
-        an = __ldg(rowptr + rn);
-        bn = __ldg(rowptr + rn + 1);
-      }
-      epi.emit(r, row_sum_thread<V, XT, Acc>(colidx, values, x, f_col, a, b, keep), es);
-      r = rn;
-      a = an;
-      b = bn;
-    }
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n_rows; t += stride) {
+    const int r = rows ? __ldg(rows + t) : (int)t;
+    const int a = __ldg(rowptr + r), b = __ldg(rowptr + r + 1);
+    epi.emit(r, row_sum_thread<V, XT, Acc>(colidx, values, x, f_col, a, b, keep));
   }
-  epi.block_done(es, blockIdx.x);
 }
 
 // Short rows, two adjacent lanes per row: the row's aligned groups (of eight
@@ -209,8 +180,6 @@ __global__ void __launch_bounds__(256) csr_pair_kernel(const int *__restrict__ r
                                                       const XT *__restrict__ x, int f_col, XKeep x_keep,
                                                       Epi epi) {
   using Acc = typename Epi::Acc;
-  if (!epi.active()) return;
-  typename Epi::State es{};
   const uint64_t keep = policy_keep(x_keep, x);
   const int half = threadIdx.x & 1;
   const unsigned pair = 3u << ((threadIdx.x & 31) & ~1);  // both lanes of a pair always run together
@@ -220,9 +189,8 @@ __global__ void __launch_bounds__(256) csr_pair_kernel(const int *__restrict__ r
     const int a = __ldg(rowptr + r), b = __ldg(rowptr + r + 1);
     const Acc mine = row_half<V, XT, Acc>(colidx, values, x, f_col, a, b, half, keep);
     const Acc other = __shfl_xor_sync(pair, mine, 1);
-    if (!half) epi.emit(r, mine + other, es);
+    if (!half) epi.emit(r, mine + other);
   }
-  epi.block_done(es, blockIdx.x);
 }
 
 // Tiny rows: every row in order and at most T entries (T = 2 or 4).  A warp
@@ -242,8 +210,6 @@ __global__ void __launch_bounds__(256) csr_tiny_kernel(int n_rows, const int *__
                                                       Epi epi) {
   using Acc = typename Epi::Acc;
   constexpr int R = 8 / T;
-  if (!epi.active()) return;
-  typename Epi::State es{};
   const int64_t base = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32 * (32 * R);
   if (base < n_rows) {
     const uint64_t keep = policy_keep(x_keep, x);
@@ -280,82 +246,9 @@ __global__ void __launch_bounds__(256) csr_tiny_kernel(int n_rows, const int *__
       #pragma unroll
       for (int t = 0; t < T; ++t)
         if (a[q] + t < b[q]) acc = fma_acc(to_acc(v[q][t], Acc()), xv[q][t], acc);
-      if (r0 + 32 * q < n_rows) epi.emit(r0 + 32 * q, acc, es);
+      if (r0 + 32 * q < n_rows) epi.emit(r0 + 32 * q, acc);
     }
   }
-  epi.block_done(es, blockIdx.x);
-}
-
-// Tiny rows from a list: rows[0..n) each hold at most T entries (empty ones
-// included), in any order.  As csr_tiny_kernel, a warp takes 32 R list
-// entries, lane l entries l, l + 32, ..., with the bounds, entries and
-// gathers of its R rows in flight together, but grid-stride over tiles, so
-// that a reducing epilogue's capped grid covers the list; one thread per row
-// would wait on each row's load chain in turn (PageRank sweeps on R-MAT:
-// four fifths of the rows).  Each row is summed in stored order, one FMA per
-// entry: the one-thread-per-row arithmetic.
-constexpr int kTinyListRows = 2;  // R: rows per lane
-inline int tiny_list_grid(int n, bool reduces) {
-  const int g = (int)(((int64_t)n + 256 * kTinyListRows - 1) / (256 * kTinyListRows));
-  return std::max(1, reduces ? std::min(g, 152 * 16) : g);
-}
-
-template <typename V, typename XT, typename Epi>
-__global__ void __launch_bounds__(256) csr_tiny_list_kernel(const int *__restrict__ rows, int n,
-                                                           const int *__restrict__ rowptr,
-                                                           const int *__restrict__ colidx,
-                                                           const V *__restrict__ values,
-                                                           const XT *__restrict__ x, int f_col, XKeep x_keep,
-                                                           Epi epi) {
-  using Acc = typename Epi::Acc;
-  constexpr int R = kTinyListRows, T = kTinyRow;
-  if (!epi.active()) return;
-  typename Epi::State es{};
-  const uint64_t keep = policy_keep(x_keep, x);
-  const int lane = threadIdx.x & 31;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t base = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (32 * R); base < n;
-       base += nwarps * (32 * R)) {
-    int r[R], a[R], b[R];
-    #pragma unroll
-    for (int q = 0; q < R; ++q) {
-      const int64_t idx = base + lane + 32 * q;
-      r[q] = idx < n ? __ldg(rows + idx) : -1;
-    }
-    #pragma unroll
-    for (int q = 0; q < R; ++q) {
-      a[q] = r[q] >= 0 ? __ldg(rowptr + r[q]) : 0;
-      b[q] = r[q] >= 0 ? __ldg(rowptr + r[q] + 1) : 0;
-    }
-    V v[R][T];
-    int c[R][T];
-    #pragma unroll
-    for (int q = 0; q < R; ++q) {
-      #pragma unroll
-      for (int t = 0; t < T; ++t) {
-        const int k = a[q] + t;
-        const bool in = k < b[q];
-        c[q][t] = in ? ld_ell<false>(colidx + k) : f_col;
-        v[q][t] = in ? ld_ell<false>(values + k) : V(0);
-      }
-    }
-    Acc xv[R][T];
-    #pragma unroll
-    for (int q = 0; q < R; ++q) {
-      #pragma unroll
-      for (int t = 0; t < T; ++t)
-        xv[q][t] = a[q] + t < b[q] ? to_acc(ld_keep(x + (c[q][t] - f_col), keep), Acc()) : Acc(0);
-    }
-    #pragma unroll
-    for (int q = 0; q < R; ++q) {
-      Acc acc = 0;
-      #pragma unroll
-      for (int t = 0; t < T; ++t)
-        if (a[q] + t < b[q]) acc = fma_acc(to_acc(v[q][t], Acc()), xv[q][t], acc);
-      if (r[q] >= 0) epi.emit(r[q], acc, es);
-    }
-  }
-  epi.block_done(es, blockIdx.x);
 }
 
 // sum of entries [a, b) by a group of L lanes of one warp (L a power of two
@@ -388,8 +281,6 @@ __global__ void __launch_bounds__(256) csr_group_kernel(const int4 *__restrict__
                                                        const XT *__restrict__ x, int f_col, XKeep x_keep,
                                                        typename Epi::Acc *__restrict__ partials, Epi epi) {
   using Acc = typename Epi::Acc;
-  if (!epi.active()) return;
-  typename Epi::State es{};
   const uint64_t keep = policy_keep(x_keep, x);
   const int64_t ng = ((int64_t)gridDim.x * blockDim.x) / L;
   // every lane of a group sees the same item sequence (same trip count)
@@ -400,12 +291,11 @@ __global__ void __launch_bounds__(256) csr_group_kernel(const int4 *__restrict__
     const int4 nx = g + ng < n_items ? items[g + ng] : make_int4(0, 0, 0, -1);
     const Acc s = range_sum_group<L, V, XT, Acc>(colidx, values, x, f_col, it.y, it.z, keep);
     if ((threadIdx.x & (L - 1)) == 0) {
-      if (it.w < 0) epi.emit(it.x, s, es);
+      if (it.w < 0) epi.emit(it.x, s);
       else partials[it.w] = s;
     }
     it = nx;
   }
-  epi.block_done(es, blockIdx.x);
 }
 
 // ---------------------------------------------------------------- staged
@@ -486,8 +376,6 @@ __global__ void __launch_bounds__(kStageWarps * 32) csr_stage_kernel(int rows, c
                                                                     XKeep x_keep, int cap, Epi epi) {
   using Acc = typename Epi::Acc;
   extern __shared__ __align__(16) unsigned char stage_smem[];
-  if (!epi.active()) return;
-  typename Epi::State es{};
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   V *sv = reinterpret_cast<V *>(stage_smem) + (size_t)wib * cap;
   int *sc = reinterpret_cast<int *>(stage_smem + (size_t)kStageWarps * cap * sizeof(V)) + (size_t)wib * cap;
@@ -522,10 +410,9 @@ __global__ void __launch_bounds__(kStageWarps * 32) csr_stage_kernel(int rows, c
     }
     __syncwarp();
     const Acc acc = stage_row_sum<V, XT, Acc>(sv, sc, lo - e0, hi - e0, x, f_col, keep);
-    if ((t << 5) + lane < rows) epi.emit((t << 5) + lane, acc, es);
+    if ((t << 5) + lane < rows) epi.emit((t << 5) + lane, acc);
     __syncwarp();  // the next tile's copies overwrite the slots
   }
-  epi.block_done(es, blockIdx.x);
 }
 
 // y[row] = sum of the row's chunk partials in chunk order;
@@ -534,16 +421,13 @@ template <typename Epi>
 __global__ void csr_chunk_fixup_kernel(const int2 *__restrict__ huge, int n_huge,
                                        const typename Epi::Acc *__restrict__ partials, Epi epi) {
   using Acc = typename Epi::Acc;
-  if (!epi.active()) return;
   const int h = blockIdx.x * blockDim.x + threadIdx.x;
-  typename Epi::State es{};
   if (h < n_huge) {
     const int row = huge[h].x, first = huge[h].y, last = huge[h + 1].y;
     Acc s = partials[first];
     for (int c = first + 1; c < last; ++c) s += partials[c];
-    epi.emit(row, s, es);
+    epi.emit(row, s);
   }
-  epi.fixup_done(es, blockIdx.x);
 }
 
 
@@ -563,10 +447,8 @@ __global__ void __launch_bounds__(256) csr_sell_kernel(const int *__restrict__ c
                                                       int64_t stride, int width, const XT *__restrict__ x,
                                                       int f_col, int rows, XKeep x_keep, Epi epi) {
   using Acc = typename Epi::Acc;
-  if (!epi.active()) return;
   const int64_t base = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32 * (32 * R);
   const int lane = threadIdx.x & 31;
-  typename Epi::State es{};
   if (base < rows) {
     const uint64_t keep = policy_keep(x_keep, x);
     const int r0 = (int)base + lane;
@@ -589,9 +471,8 @@ __global__ void __launch_bounds__(256) csr_sell_kernel(const int *__restrict__ c
     }
     #pragma unroll
     for (int q = 0; q < R; ++q)
-      if (r0 + 32 * q < rows) epi.emit(r0 + 32 * q, a[q], es);
+      if (r0 + 32 * q < rows) epi.emit(r0 + 32 * q, a[q]);
   }
-  epi.block_done(es, blockIdx.x);
 }
 
 // the sliced copy of one array: entry rowptr[r] + j to slot j * stride + r

@@ -62,7 +62,6 @@ __global__ void __launch_bounds__(kRowsNT, 3) csr_rows_kernel(const RowBlock *__
   int *s_wsum = s_seg + kRowsMax + 1;
   Acc *s_part = s_val;                // segment sums, after the staged data is consumed
 
-  if (!epi.active()) return;
   const RowBlock d = blocks[blockIdx.x];
   const int r0 = d.x, r1 = d.y, j0 = d.z, huge = d.w;
   const int nrows = r1 - r0;
@@ -113,7 +112,6 @@ __global__ void __launch_bounds__(kRowsNT, 3) csr_rows_kernel(const RowBlock *__
     }
   }
   __syncthreads();
-  typename Epi::State es{};
 
   if (huge >= 0) {
     // one chunk of a huge row: segments of kSeg, summed in order by thread 0
@@ -129,7 +127,6 @@ __global__ void __launch_bounds__(kRowsNT, 3) csr_rows_kernel(const RowBlock *__
       for (int t = 1; t < nseg; ++t) s += s_part[t];
       partials[huge] = s;
     }
-    epi.block_done(es, blockIdx.x);
     return;
   }
 
@@ -201,10 +198,9 @@ __global__ void __launch_bounds__(kRowsNT, 3) csr_rows_kernel(const RowBlock *__
       const int b0 = s_seg[i], b1 = s_seg[i + 1];
       Acc s = s_part[b0];
       for (int t = b0 + 1; t < b1; ++t) s += s_part[t];
-      epi.emit(r0 + i, s, es);
+      epi.emit(r0 + i, s);
     }
   }
-  epi.block_done(es, blockIdx.x);
 }
 
 // y[row] = sum of the row's chunk partials, in chunk order
@@ -212,16 +208,13 @@ template <typename Epi>
 __global__ void csr_huge_fixup_kernel(const int2 *__restrict__ huge_rows, int n_huge,
                                       const typename Epi::Acc *__restrict__ partials, Epi epi) {
   using Acc = typename Epi::Acc;
-  if (!epi.active()) return;
   const int h = blockIdx.x * blockDim.x + threadIdx.x;
-  typename Epi::State es{};
   if (h < n_huge) {
     const int row = huge_rows[h].x, first = huge_rows[h].y, last = huge_rows[h + 1].y;
     Acc s = partials[first];
     for (int c = first + 1; c < last; ++c) s += partials[c];
-    epi.emit(row, s, es);
+    epi.emit(row, s);
   }
-  epi.fixup_done(es, blockIdx.x);
 }
 
 }  // namespace tbsla

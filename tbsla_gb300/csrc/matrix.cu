@@ -7,6 +7,7 @@
 #include <new>
 #include <vector>
 
+#include "column_mask.cuh"
 #include "common.cuh"
 #include "product.cuh"
 
@@ -243,6 +244,7 @@ static void free_handle(tbsla_matrix *A) {
   if (!A) return;
   cudaSetDevice(A->device);
   if (A->pr_work && A->pr_work_free) A->pr_work_free(A->pr_work);
+  if (A->pr_plan && A->pr_plan_free) A->pr_plan_free(A->pr_plan);
   if (A->ppr_plan && A->ppr_plan_free) A->ppr_plan_free(A->ppr_plan);
   if (A->pr_relabel) free_handle(A->pr_relabel);
   if (A->transpose) free_handle(A->transpose);
@@ -251,7 +253,7 @@ static void free_handle(tbsla_matrix *A) {
                   A->short_rows, A->warp_items, A->chunk_rows, A->chunk_partials, A->chunk_partials32,
                   A->tile_start, A->tile_head_row, A->tile_head_val,
                   A->tile_tail_val, A->tile_emitted, A->tile_head_val32, A->tile_tail_val32,
-                  A->dangling, A->pr_scratch, A->d_x, A->d_y, A->d_t, A->d_err, A->pr_newid, A->pr_out,
+                  A->dangling, A->pr_scratch, A->col_pattern, A->d_x, A->d_y, A->d_t, A->d_err, A->pr_newid, A->pr_out,
                   A->transpose_perm, A->coo_rowptr, A->sell_cols, A->sell_vals[0], A->sell_vals[1],
                   A->sell_vals[2]};
   for (void *p : ptrs) if (p) cudaFree(p);
@@ -259,20 +261,6 @@ static void free_handle(tbsla_matrix *A) {
   for (auto &e : A->pending_events) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
   for (auto &e : A->free_events) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
   delete A;
-}
-
-// The short-row list back in row order, without the tiny head: for copies
-// whose rows are already grouped by length (the degree-relabelled PageRank
-// graph), where the one-thread-per-row kernel over the whole list measured
-// faster (R-MAT 2^24 FP64 solve 44.7 ms against 47.4 ms with the split).
-tbsla_status_t csr_unsplit_tiny(tbsla_matrix *A) {
-  if (A->n_tiny == 0 || !A->short_rows) return TBSLA_OK;
-  std::vector<int> rows((size_t)A->n_short);
-  TB_CUDA(cudaMemcpy(rows.data(), A->short_rows, rows.size() * sizeof(int), cudaMemcpyDeviceToHost));
-  std::sort(rows.begin(), rows.end());
-  TB_CUDA(cudaMemcpy(A->short_rows, rows.data(), rows.size() * sizeof(int), cudaMemcpyHostToDevice));
-  A->n_tiny = 0;
-  return TBSLA_OK;
 }
 
 tbsla_matrix *new_matrix(int format) { return new_handle(format); }
@@ -376,6 +364,34 @@ tbsla_status_t axpy_inplace(double *y, const double *x, int64_t n, cudaStream_t 
   if (n <= 0) return TBSLA_OK;
   axpy_kernel<<<grid_for(n, 256), 256, 0, s>>>(y, x, n);
   TB_CUDA(cudaGetLastError());
+  return TBSLA_OK;
+}
+
+// --------------------------------------------------------- column pattern
+__global__ void __launch_bounds__(256) mask_start_kernel(const unsigned char *__restrict__ pattern, int n_col,
+                                                         const int *zeros, unsigned char *mask) {
+  const bool all = *zeros != 0;
+  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < n_col; c += (int64_t)gridDim.x * blockDim.x)
+    mask[c] = all ? (unsigned char)1 : pattern[c];
+}
+
+tbsla_status_t column_pattern(tbsla_matrix *A, const unsigned char **pattern) {
+  if (!A->col_pattern) {
+    unsigned char *p = nullptr;
+    const size_t n = (size_t)std::max(A->n_col, 1);
+    TB_TRY(dev_alloc(A, (void **)&p, n));
+    cudaError_t e = cudaMemset(p, 1, n);
+    if (e == cudaSuccess && A->stored)
+      column_mark_kernel<float><<<mask_grid(A->stored), 256>>>(A->idx1, nullptr, A->stored, A->f_col, A->n_col,
+                                                               nullptr, p);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+    if (e != cudaSuccess) {
+      cudaFree(p);
+      TB_CUDA(e);
+    }
+    A->col_pattern = p;
+  }
+  *pattern = A->col_pattern;
   return TBSLA_OK;
 }
 
@@ -494,18 +510,6 @@ tbsla_status_t csr_bins(tbsla_matrix *A, const std::vector<int> &rp) {
       int cap = 0;
       for (int r = 0; r < rows; r += 32) cap = std::max(cap, rp[std::min(r + 32, rows)] - rp[r]);
       A->stage_cap = std::max(16, (cap + 15) / 16 * 16);
-    }
-    // Rows of at most kTinyRow entries first, when they are a large part of
-    // the short rows (power-law graphs: R-MAT 2^22 has 52 % empty rows and
-    // 27 % of 1-4 entries); the order within each part is the rows' order.
-    A->n_tiny = 0;
-    if (!all_short && !shorts.empty()) {
-      int64_t tiny = 0;
-      for (int r : shorts) tiny += rp[r + 1] - rp[r] <= kTinyRow;
-      if (tiny >= 1024 && 8 * tiny >= (int64_t)shorts.size()) {
-        std::stable_partition(shorts.begin(), shorts.end(), [&](int r) { return rp[r + 1] - rp[r] <= kTinyRow; });
-        A->n_tiny = (int)tiny;
-      }
     }
     if (!all_short && !shorts.empty()) {
       TB_TRY(alloc_n(A, &A->short_rows, (int64_t)shorts.size()));
@@ -905,8 +909,7 @@ tbsla_status_t tbsla_matrix_set_values(tbsla_matrix_t *A, tbsla_dtype_t type, co
   TB_TRY(transpose_refresh(A, s));
   TB_CUDA(cudaStreamSynchronize(s));
   // PageRank state derived from the values: rebuilt on next use
-  if (A->pr_work && A->pr_work_free) A->pr_work_free(A->pr_work);
-  A->pr_work = nullptr;
+  A->pr_dmask_stale = true;
   if (A->pr_relabel) free_handle(A->pr_relabel);
   A->pr_relabel = nullptr;
   if (A->pr_newid) cudaFree(A->pr_newid);

@@ -39,6 +39,7 @@
 #include <vector>
 
 #include "anderson.cuh"
+#include "column_mask.cuh"
 #include "product.cuh"
 
 namespace tbsla {
@@ -549,14 +550,6 @@ __global__ void __launch_bounds__(256) ppr_load_kernel(int n, const double *__re
   if (partials) block_columns<KT, 1, NV>(part, partials, blockIdx.x);
 }
 
-// dmask[j] = 1 when column j holds no nonzero value
-template <typename T>
-__global__ void ppr_dangling_kernel(const int *__restrict__ colidx, const T *__restrict__ values, int64_t nnz,
-                                    unsigned char *dmask) {
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nnz; k += (int64_t)gridDim.x * blockDim.x)
-    if (values[k] != T(0)) dmask[colidx[k]] = 0;
-}
-
 // out[v_j * n + u] = column c_j of a tile at row map(u), as FP64, for the
 // cnt (column, vector) pairs of a list
 struct PprPicks {
@@ -709,7 +702,6 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
   constexpr int NV = AA ? 5 : 2;
   constexpr int G = PprLanes<T, KT>::G;
   const int n = M->n_row;
-  const int64_t nnz = M->stored;
   const T *values = static_cast<const T *>(M->values[std::is_same<T, double>::value ? 0 : 1]);
   TB_CHECK(values, "the matrix lacks the %s value store", std::is_same<T, double>::value ? "F64" : "F32");
   const int tiles = (k + KT - 1) / KT;
@@ -756,6 +748,7 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
   unsigned *d_seeds = nullptr;
   int2 *d_pairs = nullptr;
   unsigned char *dmask = nullptr;
+  int *d_zeros = nullptr;
   double *d_inv = nullptr, *partials = nullptr;
   ColCtl *d_col = nullptr;
   ColAa *d_aa = nullptr;
@@ -786,6 +779,7 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
   alloc((void **)&d_seeds, (size_t)tiles * n * sizeof(unsigned));
   alloc((void **)&d_pairs, pairs.size() * sizeof(int2));
   alloc((void **)&dmask, (size_t)n);
+  alloc((void **)&d_zeros, sizeof(int));
   alloc((void **)&d_inv, inv.size() * sizeof(double));
   alloc((void **)&partials, (size_t)tiles * nparts * KT * NV * sizeof(double));
   alloc((void **)&d_col, (size_t)tiles * KT * sizeof(ColCtl));
@@ -831,9 +825,9 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
   up(d_aa, haa.data(), haa.size() * sizeof(ColAa));
   up(d_tile, htile.data(), htile.size() * sizeof(TileCtl));
   up(d_vec, hvec.data(), hvec.size() * sizeof(int));
-  if (e == cudaSuccess) e = cudaMemsetAsync(dmask, 1, (size_t)n, s);
   if (e != cudaSuccess) { cleanup(); return fail(TBSLA_ERR_CUDA, "batched PageRank upload: %s", cudaGetErrorString(e)); }
-  ppr_dangling_kernel<T><<<152 * 8, 256, 0, s>>>(M->idx1, values, nnz, dmask);
+  st = column_mask(const_cast<tbsla_matrix *>(M), values, dmask, d_zeros, s);
+  if (st != TBSLA_OK) { cleanup(); return st; }
   const double beta = p->beta;
   for (int t = 0; t < tiles; ++t) {
     double *pt = partials + (size_t)t * nparts * KT * NV;

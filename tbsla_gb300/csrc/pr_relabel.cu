@@ -31,8 +31,6 @@
 
 namespace tbsla {
 
-tbsla_status_t csr_unsplit_tiny(tbsla_matrix *A);
-
 namespace {
 
 constexpr int kBandSamples = 4096;
@@ -65,12 +63,6 @@ __global__ void band_sample_kernel(const int *__restrict__ rowptr, const int *__
 __global__ void column_count_kernel(const int *__restrict__ colidx, int64_t nnz, int f_col, int *deg) {
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nnz; k += (int64_t)gridDim.x * blockDim.x)
     atomicAdd(deg + (colidx[k] - f_col), 1);  // columns are in [f_col, f_col + n) (candidate())
-}
-
-// out[v] = x[newid[v]]
-__global__ void relabel_gather_kernel(const double *__restrict__ x, const int *__restrict__ newid, int n,
-                                      double *__restrict__ out) {
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) out[v] = x[newid[v]];
 }
 
 int cls_max(int maxdeg) { return 31 - __builtin_clz((unsigned)maxdeg + 1u); }
@@ -202,13 +194,6 @@ tbsla_status_t build(tbsla_matrix *A, bool check_skew, bool *built) {
   va.clear(); va.shrink_to_fit();
   tbsla_matrix_t *B = nullptr;
   TB_TRY(tbsla_csr_create(n, n, 0, n, nrp.data(), nci.data(), nva.data(), A->stores, &B));
-  // rows are grouped by length here: one thread per short row over the
-  // whole list (the tiny-row tiles measured slower on this order)
-  const tbsla_status_t su = csr_unsplit_tiny(B);
-  if (su != TBSLA_OK) {
-    tbsla_matrix_destroy(B);
-    return su;
-  }
   B->x_keep = A->x_keep;
   B->x_keep_range = A->x_keep_range;
   B->short_mode = A->short_mode;
@@ -259,13 +244,6 @@ tbsla_status_t pr_relabelled(tbsla_matrix *A, tbsla_matrix **B) {
   TB_TRY(build(A, !forced, &built));
   A->pr_relabel_state = built ? 1 : 2;
   *B = built ? A->pr_relabel : nullptr;
-  return TBSLA_OK;
-}
-
-// out[v] = x[newid[v]] for the n vertices of A, ordered on s
-tbsla_status_t pr_relabel_gather(const tbsla_matrix *A, const double *x, double *out, cudaStream_t s) {
-  relabel_gather_kernel<<<152 * 4, 256, 0, s>>>(x, A->pr_newid, A->n_row, out);
-  TB_CUDA(cudaGetLastError());
   return TBSLA_OK;
 }
 

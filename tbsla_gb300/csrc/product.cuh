@@ -1,12 +1,8 @@
 // product.cuh -- launches of the SpMV kernels of every format with an
-// epilogue functor (shared by the plain products and PageRank).
+// epilogue functor (plain products, a_axpx).
 //
-// Every epilogue provides:
-//   active()             false once its computation is finished (PageRank
-//                        sweeps after convergence): kernels return at once;
-//   emit(row, v, state)  receives each finished row exactly once;
-//   block_done / fixup_done(state, block)  per-block reduction hooks;
-//   set_part_base(k)     offset of the launch's blocks in a partials array.
+// Every epilogue provides emit(row, v), which receives each finished row
+// exactly once.
 #pragma once
 
 #include <algorithm>
@@ -18,19 +14,13 @@
 
 namespace tbsla {
 
-// grids of the grid-stride CSR kernels.  Plain products take one row (one
-// warp item) per thread (warp): the most loads in flight.  Epilogues that
-// reduce per block cap the grid at kStrideBlocks blocks, so that each
-// block's reduction covers many rows and the partials stay few.
+// grids: one row (one row item) per thread (group), the most loads in flight;
+// the staged kernel strides a grid of at most kStrideBlocks blocks
 constexpr int kStrideBlocks = 152 * 16;
-inline int short_grid(int n_short, bool reduces) {
-  const int g = (int)(((int64_t)n_short + 255) / 256);
-  return std::max(1, reduces ? std::min(g, kStrideBlocks) : g);
-}
-inline int group_grid(int n_items, int lanes, bool reduces) {
+inline int short_grid(int64_t n_short) { return (int)std::max<int64_t>(1, (n_short + 255) / 256); }
+inline int group_grid(int n_items, int lanes) {
   const int per_block = 256 / lanes;
-  const int g = (int)(((int64_t)n_items + per_block - 1) / per_block);
-  return std::max(1, reduces ? std::min(g, kStrideBlocks) : g);
+  return (int)std::max<int64_t>(1, ((int64_t)n_items + per_block - 1) / per_block);
 }
 inline int fixup_grid(int n) { return std::max(1, (n + 127) / 128); }
 
@@ -70,21 +60,6 @@ template <typename XT> inline XKeep xkeep_of(const tbsla_matrix *A) {
   return k;
 }
 
-// Reducing epilogues take the short list's tiny head (n_tiny rows of at most
-// kTinyRow entries) in warp tiles when the short-row kernel is the default.
-template <typename Epi> inline bool tiny_split(const tbsla_matrix *A) {
-  return Epi::kReduces && A->n_tiny > 0 && A->short_rows != nullptr && A->short_mode <= 0;
-}
-// the partial slots the short-row launches of a reducing epilogue write
-inline int short_parts_reducing(const tbsla_matrix *A) {
-  if (A->n_short == 0) return 0;
-  if (A->n_tiny > 0 && A->short_rows != nullptr && A->short_mode <= 0) {
-    const int rest = A->n_short - A->n_tiny;
-    return tiny_list_grid(A->n_tiny, true) + (rest > 0 ? short_grid(rest, true) : 0);
-  }
-  return short_grid(A->n_short, true);
-}
-
 // The staged kernel applies when every row is short (stage_cap > 0) and the
 // handle's stage mode (tbsla_matrix_tune) is on.
 inline bool stage_on(const tbsla_matrix *A) {
@@ -114,11 +89,11 @@ inline int sell_rows_per_thread(const tbsla_matrix *A) {
 // handle has one and plain products take it: the default short-row mode, or
 // mode 3; F64 and F32 stores (BF16 slots load 64 bytes per warp instruction:
 // cqmat 2^24 0.366 ms against 0.334 with one thread per row)
-template <typename V, typename Epi> inline const V *sell_vals_for(const tbsla_matrix *A, const V *vals) {
+template <typename V> inline const V *sell_vals_for(const tbsla_matrix *A, const V *vals) {
   if constexpr (sizeof(V) < 4) {
     return nullptr;  // BF16: the copy is not kept
   } else {
-    if (Epi::kReduces || !A->sell_width || !(A->short_mode == -1 || A->short_mode == 3)) return nullptr;
+    if (!A->sell_width || !(A->short_mode == -1 || A->short_mode == 3)) return nullptr;
     for (int k = 0; k < 2; ++k)
       if (A->values[k] == static_cast<const void *>(vals)) return static_cast<const V *>(A->sell_vals[k]);
     return nullptr;
@@ -133,8 +108,7 @@ tbsla_status_t launch_csr_direct(const tbsla_matrix *A, const int *rowptr, const
                                  const XT *x, Epi epi, cudaStream_t s) {
   using Acc = typename Epi::Acc;
   KernelTimer kt(A, s);
-  int base = 0;
-  if (const V *sv = sell_vals_for<V, Epi>(A, vals)) {
+  if (const V *sv = sell_vals_for<V>(A, vals)) {
     // every row short, the ELL-layout copy: one warp per 32 R rows
     const int R = sell_rows_per_thread(A);
     const int64_t threads = A->sell_stride / (32 * R) * 32;
@@ -152,65 +126,36 @@ tbsla_status_t launch_csr_direct(const tbsla_matrix *A, const int *rowptr, const
     return TBSLA_OK;
   }
   if (A->n_short > 0 && stage_on(A)) {
-    // all rows short: the staged kernel (reducing epilogues: the same grid as
-    // the short-row kernel, so that every partial slot is written)
+    // all rows short: the staged kernel
     const size_t smem = csr_stage_setup<V, XT, Epi>(A->stage_cap);
     const int tiles = (A->n_short + 31) / 32;
-    const int grid = Epi::kReduces ? short_grid(A->n_short, true)
-                                   : std::max(1, std::min((tiles + kStageWarps - 1) / kStageWarps, kStrideBlocks));
-    epi.set_part_base(base);
-    base += short_grid(A->n_short, Epi::kReduces);
+    const int grid = std::max(1, std::min((tiles + kStageWarps - 1) / kStageWarps, kStrideBlocks));
     csr_stage_kernel<V, XT, Epi><<<grid, kStageWarps * 32, smem, s>>>(A->n_short, rowptr, colidx, vals, x, A->f_col,
                                                                      xkeep_of<XT>(A), A->stage_cap, epi);
-  } else if (A->n_short > 0 && A->short_rows == nullptr && A->short_mode < 0 && !Epi::kReduces &&
-             A->short_max <= kTinyRow) {
+  } else if (A->n_short > 0 && A->short_rows == nullptr && A->short_mode < 0 && A->short_max <= kTinyRow) {
     // every row in order and tiny: warp tiles of 32 * 8 / T rows
     const int T = A->short_max <= 2 ? 2 : 4;
     const int64_t warps = ((int64_t)A->n_short + 32 * (8 / T) - 1) / (32 * (8 / T));
     const int grid = (int)((warps * 32 + 255) / 256);
-    epi.set_part_base(base);
-    base += short_grid(A->n_short, Epi::kReduces);
     if (T == 2)
       csr_tiny_kernel<2, V, XT, Epi><<<grid, 256, 0, s>>>(A->n_short, rowptr, colidx, vals, x, A->f_col,
                                                           xkeep_of<XT>(A), epi);
     else
       csr_tiny_kernel<4, V, XT, Epi><<<grid, 256, 0, s>>>(A->n_short, rowptr, colidx, vals, x, A->f_col,
                                                           xkeep_of<XT>(A), epi);
-  } else if (A->n_short > 0 && tiny_split<Epi>(A)) {
-    // the tiny head in warp tiles, the rest one thread per row
-    const int grid = tiny_list_grid(A->n_tiny, true);
-    epi.set_part_base(base);
-    base += grid;
-    csr_tiny_list_kernel<V, XT, Epi><<<grid, 256, 0, s>>>(A->short_rows, A->n_tiny, rowptr, colidx, vals, x,
-                                                          A->f_col, xkeep_of<XT>(A), epi);
-    const int rest = A->n_short - A->n_tiny;
-    if (rest > 0) {
-      epi.set_part_base(base);
-      base += short_grid(rest, true);
-      csr_short_kernel<V, XT, Epi><<<short_grid(rest, true), 256, 0, s>>>(
-          A->short_rows + A->n_tiny, rest, rowptr, colidx, vals, x, A->f_col, xkeep_of<XT>(A), epi);
-    }
-  } else if (A->n_short > 0 && (A->short_mode == 2 || (A->short_mode < 0 && sizeof(V) == 8 && !Epi::kReduces &&
+  } else if (A->n_short > 0 && (A->short_mode == 2 || (A->short_mode < 0 && sizeof(V) == 8 &&
                                                        A->short_nnz >= (int64_t)kPairMinRow * A->n_short))) {
-    // two lanes per row: twice the threads of the one-lane grid (reducing
-    // epilogues: the same capped grid, so every partial slot is written)
-    const int grid = Epi::kReduces ? short_grid(A->n_short, true) : short_grid(2 * A->n_short, false);
-    epi.set_part_base(base);
-    base += short_grid(A->n_short, Epi::kReduces);
-    csr_pair_kernel<V, XT, Epi><<<grid, 256, 0, s>>>(A->short_rows, A->n_short, rowptr, colidx, vals, x, A->f_col,
-                                                     xkeep_of<XT>(A), epi);
+    // two lanes per row
+    csr_pair_kernel<V, XT, Epi><<<short_grid(2 * (int64_t)A->n_short), 256, 0, s>>>(
+        A->short_rows, A->n_short, rowptr, colidx, vals, x, A->f_col, xkeep_of<XT>(A), epi);
   } else if (A->n_short > 0) {
-    epi.set_part_base(base);
-    base += short_grid(A->n_short, Epi::kReduces);
-    csr_short_kernel<V, XT, Epi><<<short_grid(A->n_short, Epi::kReduces), 256, 0, s>>>(
+    csr_short_kernel<V, XT, Epi><<<short_grid(A->n_short), 256, 0, s>>>(
         A->short_rows, A->n_short, rowptr, colidx, vals, x, A->f_col, xkeep_of<XT>(A), epi);
   }
   for (int c = 0; c < kGroupClasses; ++c) {
     const int first = A->item_class_start[c], count = A->item_class_start[c + 1] - first;
     if (count == 0) continue;
-    const int grid = group_grid(count, kGroupLanes[c], Epi::kReduces);
-    epi.set_part_base(base);
-    base += grid;
+    const int grid = group_grid(count, kGroupLanes[c]);
     const int4 *items = A->warp_items + first;
     Acc *parts = chunk_partials_of<Acc>(A);
     switch (kGroupLanes[c]) {
@@ -230,7 +175,6 @@ tbsla_status_t launch_csr_direct(const tbsla_matrix *A, const int *rowptr, const
   }
   kt.stop();
   if (A->n_chunk_rows > 0) {
-    epi.set_part_base(base);
     csr_chunk_fixup_kernel<Epi><<<fixup_grid(A->n_chunk_rows), 128, 0, s>>>(
         A->chunk_rows, A->n_chunk_rows, chunk_partials_of<Acc>(A), epi);
   }

@@ -14,7 +14,7 @@
 // DENSE is a row-major GEMV, four rows per warp.
 //
 // The products are written through an epilogue functor `Epi` that receives
-// each finished row once:  epi.emit(row, value, state).
+// each finished row once:  epi.emit(row, value).
 #pragma once
 
 #include "common.cuh"
@@ -31,38 +31,26 @@ template <typename Acc> struct Carry {
 // ------------------------------------------------------------ epilogues
 template <typename YT, typename AccT> struct StoreEpi {
   using Acc = AccT;
-  static constexpr bool kReduces = false;  // no per-block partials
-  struct State {};
   YT *y;
   int n_out;   // rows that may be written
   int shift;   // output row = row + shift (COO vect_incr)
-  __device__ __forceinline__ void emit(int row, Acc v, State &) const {
+  __device__ __forceinline__ void emit(int row, Acc v) const {
     int o = row + shift;
     if (o >= 0 && o < n_out) __stcs(y + o, (YT)v);  // streaming: keep L2 for x
   }
-  __device__ __forceinline__ bool active() const { return true; }
-  __host__ __device__ void set_part_base(int) {}
-  __device__ __forceinline__ void block_done(State &, int) const {}
-  __device__ __forceinline__ void fixup_done(State &, int) const {}
 };
 
 // y = A x + x  (the first half of Matrix::a_axpx_, Matrix.cpp:6-11)
 template <typename AccT> struct AddXEpi {
   using Acc = AccT;
-  static constexpr bool kReduces = false;
-  struct State {};
   double *y;
   const double *x;
   int n_out;
   int shift;
-  __device__ __forceinline__ void emit(int row, Acc v, State &) const {
+  __device__ __forceinline__ void emit(int row, Acc v) const {
     int o = row + shift;
     if (o >= 0 && o < n_out) __stcs(y + o, (double)v + x[o]);
   }
-  __device__ __forceinline__ bool active() const { return true; }
-  __host__ __device__ void set_part_base(int) {}
-  __device__ __forceinline__ void block_done(State &, int) const {}
-  __device__ __forceinline__ void fixup_done(State &, int) const {}
 };
 
 // --------------------------------------------------------- block helpers
@@ -103,8 +91,7 @@ __device__ __forceinline__ void resolve_tile(int tile, bool deferred, int first_
                                              typename Epi::Acc first_val, bool tile_starts_mid,
                                              typename Epi::Acc *s_tail, unsigned char *s_emit,
                                              int *s_misc, typename Epi::Acc *s_red,
-                                             Carry<typename Epi::Acc> carry, const Epi &epi,
-                                             typename Epi::State &es) {
+                                             Carry<typename Epi::Acc> carry, const Epi &epi) {
   using Acc = typename Epi::Acc;
   if (threadIdx.x == 0) s_misc[0] = -1;
   __syncthreads();
@@ -115,7 +102,7 @@ __device__ __forceinline__ void resolve_tile(int tile, bool deferred, int first_
     for (int v = u < 0 ? 0 : u; v < (int)threadIdx.x; ++v) s += s_tail[v];
     s += first_val;
     if (u >= 0 || !tile_starts_mid) {
-      epi.emit(first_row, s, es);
+      epi.emit(first_row, s);
     } else {
       s_misc[0] = first_row;
       s_red[NT / 32] = s;  // head value (slot after the reduction scratch)
@@ -166,9 +153,7 @@ __device__ __forceinline__ void stage_tile(const V *__restrict__ vals, const int
 template <typename Epi>
 __global__ void merge_fixup_kernel(int num_tiles, Carry<typename Epi::Acc> carry, Epi epi) {
   using Acc = typename Epi::Acc;
-  if (!epi.active()) return;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  typename Epi::State es{};
   if (t < num_tiles) {
     const int r = carry.head_row[t];
     if (r >= 0) {
@@ -177,10 +162,9 @@ __global__ void merge_fixup_kernel(int num_tiles, Carry<typename Epi::Acc> carry
       Acc s = 0;
       for (int v = u < 0 ? 0 : u; v < t; ++v) s += carry.tail_val[v];
       s += carry.head_val[t];
-      epi.emit(r, s, es);
+      epi.emit(r, s);
     }
   }
-  epi.fixup_done(es, blockIdx.x);
 }
 
 // --------------------------------------------------------------- COO
@@ -202,7 +186,6 @@ __global__ void __launch_bounds__(NT) coo_merge_kernel(const int *__restrict__ r
   __shared__ unsigned char s_emit[NT];
   __shared__ int s_misc[NT / 32 + 2];
 
-  if (!epi.active()) return;
   const int t = blockIdx.x;
   const int64_t e0 = (int64_t)t * TILE;
   const int n_t = (int)min((int64_t)TILE, nnz - e0);
@@ -215,7 +198,6 @@ __global__ void __launch_bounds__(NT) coo_merge_kernel(const int *__restrict__ r
   const int n_items = min(b + K, n_t) - b;
   // row of the entry after this tile (INT_MIN past the last entry)
   const int next_tile_row = (e0 + n_t < nnz) ? rowv[e0 + n_t] : INT_MIN;
-  typename Epi::State es{};
   Acc acc = 0, first_val = 0;
   bool emitted = false, deferred = false;
   int first_row = -1;
@@ -230,7 +212,7 @@ __global__ void __launch_bounds__(NT) coo_merge_kernel(const int *__restrict__ r
       const int nr = (e + 1 < n_t) ? s_row[e + 1] : next_tile_row;
       if (nr != r) {  // the row ends at entry e
         if (!emitted && starts_mid) { deferred = true; first_row = r; first_val = acc; }
-        else epi.emit(r, acc, es);
+        else epi.emit(r, acc);
         emitted = true;
         acc = 0;
       }
@@ -240,8 +222,7 @@ __global__ void __launch_bounds__(NT) coo_merge_kernel(const int *__restrict__ r
   s_emit[threadIdx.x] = emitted;
   const bool tile_starts_mid = n_t > 0 && prev_row == s_row[0];
   resolve_tile<NT, Epi>(t, deferred, first_row, first_val, tile_starts_mid, s_tail, s_emit, s_misc,
-                        s_red, carry, epi, es);
-  epi.block_done(es, t);
+                        s_red, carry, epi);
 }
 
 // --------------------------------------------------------------- ELL
@@ -309,9 +290,7 @@ __global__ void __launch_bounds__(256) ell_kernel(const int *__restrict__ cols,
                                                   const XT *__restrict__ x, int f_col, int rows,
                                                   int rows_pad, int max_col, XKeep x_keep, Epi epi) {
   using Acc = typename Epi::Acc;
-  if (!epi.active()) return;
   const int r0 = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
-  typename Epi::State es{};
   if (r0 < rows) {
     const uint64_t keep = policy_keep(x_keep, x);
     Acc a[4] = {0, 0, 0, 0};
@@ -330,9 +309,8 @@ __global__ void __launch_bounds__(256) ell_kernel(const int *__restrict__ cols,
     }
     #pragma unroll
     for (int q = 0; q < 4; ++q)
-      if (r0 + q < rows) epi.emit(r0 + q, a[q], es);
+      if (r0 + q < rows) epi.emit(r0 + q, a[q]);
   }
-  epi.block_done(es, blockIdx.x);
 }
 
 // Warp tiles of 128 rows: lane l of a warp sums rows base + l + 32 q
@@ -376,10 +354,8 @@ __global__ void __launch_bounds__(256) ell_warp_kernel(const int *__restrict__ c
                                                        const XT *__restrict__ x, int f_col, int rows,
                                                        int rows_pad, int max_col, XKeep x_keep, Epi epi) {
   using Acc = typename Epi::Acc;
-  if (!epi.active()) return;
   const int64_t base = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32 * (32 * R);
   const int lane = threadIdx.x & 31;
-  typename Epi::State es{};
   if (base < rows) {
     const uint64_t keep = policy_keep(x_keep, x);
     const int r0 = (int)base + lane;
@@ -408,9 +384,8 @@ __global__ void __launch_bounds__(256) ell_warp_kernel(const int *__restrict__ c
     }
     #pragma unroll
     for (int q = 0; q < R; ++q)
-      if (in[q]) epi.emit(r0 + 32 * q, a[q], es);
+      if (in[q]) epi.emit(r0 + 32 * q, a[q]);
   }
-  epi.block_done(es, blockIdx.x);
 }
 
 // --------------------------------------------------------------- DENSE
@@ -423,11 +398,9 @@ __global__ void __launch_bounds__(256) dense_kernel(const V *__restrict__ a,
                                                     Epi epi) {
   using Acc = typename Epi::Acc;
   constexpr int RW = 4;
-  if (!epi.active()) return;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int r0 = warp * RW;
-  typename Epi::State es{};
   if (r0 < rows) {
     Acc acc[RW] = {0, 0, 0, 0};
     const V *rowp[RW];
@@ -444,10 +417,9 @@ __global__ void __launch_bounds__(256) dense_kernel(const V *__restrict__ a,
       Acc v = acc[q];
       #pragma unroll
       for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-      if (lane == 0 && r0 + q < rows) epi.emit(r0 + q, v, es);
+      if (lane == 0 && r0 + q < rows) epi.emit(r0 + q, v);
     }
   }
-  epi.block_done(es, blockIdx.x);
 }
 
 }  // namespace tbsla

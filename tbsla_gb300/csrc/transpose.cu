@@ -128,7 +128,7 @@ tbsla_status_t grad_values(const tbsla_matrix *A, const T *a, const T *b, T scal
   for (int c = 0; c < kGroupClasses; ++c) {
     const int first = A->item_class_start[c], count = A->item_class_start[c + 1] - first;
     if (count == 0) continue;
-    const int grid = group_grid(count, kGroupLanes[c], false);
+    const int grid = group_grid(count, kGroupLanes[c]);
     const int4 *items = A->warp_items + first;
     switch (kGroupLanes[c]) {
     case 4: grad_group_kernel<4, T><<<grid, 256, 0, s>>>(items, count, A->idx1, A->f_col, a, b, scale, out); break;
