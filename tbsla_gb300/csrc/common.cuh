@@ -165,6 +165,7 @@ struct tbsla_matrix {
   double *pr_out = nullptr;          // result in the original labels (device)
   // transposed copy (transpose.cu), built on first use: entry k' of the copy
   // holds entry transpose_perm[k'] of this matrix
+  int *seg_row = nullptr;  // values gradient: the row of every 128th entry
   tbsla_matrix *transpose = nullptr;
   int *transpose_perm = nullptr;
   // batched PageRank tile width chosen by tbsla_autotune_ppr (F64, F32); 0: none

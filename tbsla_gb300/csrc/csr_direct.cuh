@@ -11,12 +11,13 @@
 //     barrier are involved.  The row is summed in
 //     its stored order with one FMA per nonzero (the order of
 //     MatrixCSR::Ax, src/cpp/matrix/MatrixCSR.cpp:133-139).
-//   long (<= kChunk): a group of L lanes per row, L = 4, 8, 16 or 32 by
-//     length class (kGroupLimit), lanes striding the row, partial sums
-//     combined with a fixed shuffle tree inside the group.
-//   huge (> kChunk): the row is cut into chunks of kChunk nonzeros, 32 lanes
+//   long (<= kChunk): a group of L lanes per row, L = 4, 8, 32 or a block of
+//     256 by length class (kGroupLimit), lanes striding the row, partial sums
+//     combined in a fixed order inside the group.
+//   huge (> kChunk): the row is cut into chunks of kChunk nonzeros, a block
 //     per chunk writing a partial; csr_chunk_fixup_kernel adds the partials of
 //     each row in chunk order.
+// Matrices with long rows run all of it in one launch (csr_mixed_kernel).
 // The groups exist for the FP64 pipe (2 lane-operations per clock per SM on
 // GB300; a warp instruction costs the same with 1 or 32 lanes active): one
 // warp per row would spend ~10 FP64 warp instructions per row on its
@@ -38,7 +39,7 @@ constexpr int kChunk = 8192;
 // kGroupLimit[c] entries with kGroupLanes[c] lanes each (chunks: class 3)
 constexpr int kGroupClasses = 4;
 constexpr int kGroupLimit[kGroupClasses] = {96, 256, 1024, kChunk};
-constexpr int kGroupLanes[kGroupClasses] = {4, 8, 16, 32};
+constexpr int kGroupLanes[kGroupClasses] = {4, 8, 32, 256};
 
 __device__ __forceinline__ float bf16_lo(unsigned w) { return __bfloat162float(__ushort_as_bfloat16((unsigned short)(w & 0xffffu))); }
 __device__ __forceinline__ float bf16_hi(unsigned w) { return __bfloat162float(__ushort_as_bfloat16((unsigned short)(w >> 16))); }
@@ -130,10 +131,9 @@ __device__ __forceinline__ Acc row_sum_thread(const int *__restrict__ colidx, co
   return row_groups<2, V, XT, Acc>(colidx, values, x, f_col, a, b, keep);
 }
 
-// short rows: rows [0, n_rows) when `rows` is NULL, else rows[0..n_rows);
-// one row per thread
+// every row short: one row per thread
 template <typename V, typename XT, typename Epi>
-__global__ void __launch_bounds__(256) csr_short_kernel(const int *__restrict__ rows, int n_rows,
+__global__ void __launch_bounds__(256) csr_short_kernel(int n_rows,
                                                        const int *__restrict__ rowptr,
                                                        const int *__restrict__ colidx,
                                                        const V *__restrict__ values,
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(256) csr_short_kernel(const int *__restrict__ 
   const uint64_t keep = policy_keep(x_keep, x);
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n_rows; t += stride) {
-    const int r = rows ? __ldg(rows + t) : (int)t;
+    const int r = (int)t;
     const int a = __ldg(rowptr + r), b = __ldg(rowptr + r + 1);
     epi.emit(r, row_sum_thread<V, XT, Acc>(colidx, values, x, f_col, a, b, keep));
   }
@@ -173,7 +173,7 @@ __device__ __forceinline__ Acc row_half(const int *__restrict__ colidx, const V 
 }
 
 template <typename V, typename XT, typename Epi>
-__global__ void __launch_bounds__(256) csr_pair_kernel(const int *__restrict__ rows, int n_rows,
+__global__ void __launch_bounds__(256) csr_pair_kernel(int n_rows,
                                                       const int *__restrict__ rowptr,
                                                       const int *__restrict__ colidx,
                                                       const V *__restrict__ values,
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(256) csr_pair_kernel(const int *__restrict__ r
   const unsigned pair = 3u << ((threadIdx.x & 31) & ~1);  // both lanes of a pair always run together
   const int64_t stride = ((int64_t)gridDim.x * blockDim.x) >> 1;
   for (int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 1; t < n_rows; t += stride) {
-    const int r = rows ? __ldg(rows + t) : (int)t;
+    const int r = (int)t;
     const int a = __ldg(rowptr + r), b = __ldg(rowptr + r + 1);
     const Acc mine = row_half<V, XT, Acc>(colidx, values, x, f_col, a, b, half, keep);
     const Acc other = __shfl_xor_sync(pair, mine, 1);
@@ -251,50 +251,125 @@ __global__ void __launch_bounds__(256) csr_tiny_kernel(int n_rows, const int *__
   }
 }
 
-// sum of entries [a, b) by a group of L lanes of one warp (L a power of two
-// <= 32, groups aligned in the warp): lanes stride the range, fixed shuffle
-// tree within the group.  Valid in the group's first lane.
+// A lane's share of entries [a, b) of a group of L lanes: entries a + lane,
+// a + lane + L, ..., one FMA per entry in that order.  Four entries go
+// together, their gathers in flight with the next four's columns and values.
 template <int L, typename V, typename XT, typename Acc>
-__device__ __forceinline__ Acc range_sum_group(const int *__restrict__ colidx, const V *__restrict__ values,
-                                               const XT *__restrict__ x, int f_col, int a, int b, uint64_t keep) {
-  const int lane = threadIdx.x & (L - 1);
-  const unsigned mask = L == 32 ? 0xffffffffu : ((1u << (L & 31)) - 1u) << ((threadIdx.x & 31) & ~(L - 1));
+__device__ __forceinline__ Acc range_sum_lane(const int *__restrict__ colidx, const V *__restrict__ values,
+                                              const XT *__restrict__ x, int f_col, int a, int b, int lane,
+                                              uint64_t keep) {
+  constexpr int U = 4;
   Acc acc = 0;
-  #pragma unroll 4
-  for (int k = a + lane; k < b; k += L)
-    acc = fma_acc(to_acc(ld_stream(values + k), Acc()), to_acc(ld_keep(x + (ld_stream(colidx + k) - f_col), keep), Acc()), acc);
-  #pragma unroll
-  for (int o = L / 2; o > 0; o >>= 1) acc += __shfl_down_sync(mask, acc, o, L);
+  int c[U];
+  V v[U];
+  auto load = [&](int64_t k) {
+    #pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool in = k + u * L < b;
+      c[u] = in ? ld_stream(colidx + k + u * L) : -1;
+      v[u] = in ? ld_stream(values + k + u * L) : V(0);
+    }
+  };
+  load((int64_t)a + lane);
+  for (int64_t k = (int64_t)a + lane; k < b; k += L * U) {
+    Acc xv[U];
+    V vv[U];
+    bool in[U];
+    #pragma unroll
+    for (int u = 0; u < U; ++u) {
+      in[u] = c[u] >= 0;
+      vv[u] = v[u];
+      xv[u] = in[u] ? to_acc(ld_keep(x + (c[u] - f_col), keep), Acc()) : Acc(0);
+    }
+    load(k + L * U);
+    #pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (in[u]) acc = fma_acc(to_acc(vv[u], Acc()), xv[u], acc);
+  }
   return acc;
 }
 
-// Rows longer than kShortRow and chunks of huge rows, L lanes per item:
-// items[i] = (row, begin, end, partial slot or -1).  A warp holds 32/L
-// groups, so its FP64 reduction steps and the epilogue serve 32/L rows at
-// once (every FP64 warp instruction costs the same on this part whatever
-// its active lanes).  Items come in length classes, so the groups of a warp
-// take similar trip counts.
+// One long row (or chunk) by a group of L lanes of a warp, items [first,
+// first + n) dealt 256 / L to a block: items[i] = (row, begin, end, partial
+// slot or -1).  A warp holds 32/L groups, so its FP64 reduction steps and the
+// epilogue serve 32/L rows at once.
 template <int L, typename V, typename XT, typename Epi>
-__global__ void __launch_bounds__(256) csr_group_kernel(const int4 *__restrict__ items, int n_items,
-                                                       const int *__restrict__ colidx,
-                                                       const V *__restrict__ values,
+__device__ __forceinline__ void mixed_group(const int4 *__restrict__ items, int n, int block,
+                                            const int *__restrict__ colidx, const V *__restrict__ values,
+                                            const XT *__restrict__ x, int f_col, uint64_t keep, const Epi &epi) {
+  using Acc = typename Epi::Acc;
+  const int i = block * (256 / L) + (int)threadIdx.x / L, lane = threadIdx.x & (L - 1);
+  const int4 it = i < n ? __ldg(items + i) : make_int4(-1, 0, 0, -1);
+  Acc s = range_sum_lane<L, V, XT, Acc>(colidx, values, x, f_col, it.y, it.z, lane, keep);
+  #pragma unroll
+  for (int o = L / 2; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, L);
+  if (lane == 0 && it.x >= 0) epi.emit(it.x, s);
+}
+
+// Matrices with long rows, one launch: the blocks take, in this order, the
+// block-wide items (a row above 1024 entries or a chunk each), the items of
+// 32, 8 and 4 lanes, and the short rows (one lane each, or two: kPair), so
+// that the longest items start first and the small classes fill the GPU
+// together.  One launch per class left the classes one after the other
+// and walked chunks of 8192 entries with 32 lanes: a ragged FP32 matrix of
+// 600011 rows (8 million entries, 30 hub rows) took 150 us, 67 of them the 30
+// hub rows.
+struct MixedPlan {
+  const int4 *items;
+  int start[kGroupClasses + 1];  // items of class c: [start[c], start[c + 1])
+  int first[kGroupClasses + 1];  // first block of class c (3, 2, 1, 0), [kGroupClasses]: of the short rows
+  const int *rows;               // short rows
+  int n_short;
+};
+
+template <bool kPair, typename V, typename XT, typename Epi>
+__global__ void __launch_bounds__(256) csr_mixed_kernel(const MixedPlan p, const int *__restrict__ rowptr,
+                                                       const int *__restrict__ colidx, const V *__restrict__ values,
                                                        const XT *__restrict__ x, int f_col, XKeep x_keep,
                                                        typename Epi::Acc *__restrict__ partials, Epi epi) {
   using Acc = typename Epi::Acc;
+  __shared__ Acc part[256];
   const uint64_t keep = policy_keep(x_keep, x);
-  const int64_t ng = ((int64_t)gridDim.x * blockDim.x) / L;
-  // every lane of a group sees the same item sequence (same trip count)
-  int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / L;
-  int4 it = g < n_items ? items[g] : make_int4(0, 0, 0, -1);
-  for (; g < n_items; g += ng) {
-    // next item loaded ahead (its latency overlaps this item's sum)
-    const int4 nx = g + ng < n_items ? items[g + ng] : make_int4(0, 0, 0, -1);
-    const Acc s = range_sum_group<L, V, XT, Acc>(colidx, values, x, f_col, it.y, it.z, keep);
-    if ((threadIdx.x & (L - 1)) == 0) {
-      if (it.w < 0) epi.emit(it.x, s);
-      else partials[it.w] = s;
+  const int b = blockIdx.x;
+  if (b < p.first[2]) {
+    const int4 it = __ldg(p.items + p.start[3] + b);
+    part[threadIdx.x] = range_sum_lane<256, V, XT, Acc>(colidx, values, x, f_col, it.y, it.z, threadIdx.x, keep);
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      Acc s = part[threadIdx.x];
+      #pragma unroll
+      for (int u = 1; u < 8; ++u) s += part[threadIdx.x + 32 * u];
+      #pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+      if (threadIdx.x == 0) {
+        if (it.w < 0) epi.emit(it.x, s);
+        else partials[it.w] = s;
+      }
     }
-    it = nx;
+  } else if (b < p.first[1]) {
+    mixed_group<32, V, XT, Epi>(p.items + p.start[2], p.start[3] - p.start[2], b - p.first[2], colidx, values, x, f_col, keep, epi);
+  } else if (b < p.first[0]) {
+    mixed_group<8, V, XT, Epi>(p.items + p.start[1], p.start[2] - p.start[1], b - p.first[1], colidx, values, x, f_col, keep, epi);
+  } else if (b < p.first[4]) {
+    mixed_group<4, V, XT, Epi>(p.items + p.start[0], p.start[1] - p.start[0], b - p.first[0], colidx, values, x, f_col, keep, epi);
+  } else if constexpr (kPair) {
+    const int64_t t = ((int64_t)(b - p.first[4]) * 256 + threadIdx.x) >> 1;
+    const int half = threadIdx.x & 1;
+    const unsigned pair = 3u << ((threadIdx.x & 31) & ~1);  // both lanes of a pair always run together
+    if (t < p.n_short) {
+      const int r = __ldg(p.rows + t);
+      const int a = __ldg(rowptr + r), e = __ldg(rowptr + r + 1);
+      const Acc mine = row_half<V, XT, Acc>(colidx, values, x, f_col, a, e, half, keep);
+      const Acc other = __shfl_xor_sync(pair, mine, 1);
+      if (!half) epi.emit(r, mine + other);
+    }
+  } else {
+    const int64_t t = (int64_t)(b - p.first[4]) * 256 + threadIdx.x;
+    if (t < p.n_short) {
+      const int r = __ldg(p.rows + t);
+      const int a = __ldg(rowptr + r), e = __ldg(rowptr + r + 1);
+      epi.emit(r, row_sum_thread<V, XT, Acc>(colidx, values, x, f_col, a, e, keep));
+    }
   }
 }
 

@@ -230,6 +230,7 @@ tbsla_status_t alloc_carries(tbsla_matrix *A) {
 }
 
 tbsla_status_t csr_bins(tbsla_matrix *A, const std::vector<int> &rp);
+tbsla_status_t grad_segments(tbsla_matrix *A);
 
 static tbsla_matrix *new_handle(int format) {
   tbsla_matrix *A = new (std::nothrow) tbsla_matrix();
@@ -253,7 +254,7 @@ static void free_handle(tbsla_matrix *A) {
                   A->short_rows, A->warp_items, A->chunk_rows, A->chunk_partials, A->chunk_partials32,
                   A->tile_start, A->tile_head_row, A->tile_head_val,
                   A->tile_tail_val, A->tile_emitted, A->tile_head_val32, A->tile_tail_val32,
-                  A->dangling, A->pr_scratch, A->col_pattern, A->d_x, A->d_y, A->d_t, A->d_err, A->pr_newid, A->pr_out,
+                  A->dangling, A->pr_scratch, A->col_pattern, A->seg_row, A->d_x, A->d_y, A->d_t, A->d_err, A->pr_newid, A->pr_out,
                   A->transpose_perm, A->coo_rowptr, A->sell_cols, A->sell_vals[0], A->sell_vals[1],
                   A->sell_vals[2]};
   for (void *p : ptrs) if (p) cudaFree(p);
@@ -577,6 +578,7 @@ tbsla_status_t csr_bins(tbsla_matrix *A, const std::vector<int> &rp) {
   if (!blocks.empty())
     TB_CUDA(cudaMemcpy(A->row_blocks, blocks.data(), blocks.size() * sizeof(int4), cudaMemcpyHostToDevice));
   TB_CUDA(cudaMemcpy(A->huge_rows, huge.data(), huge.size() * sizeof(int2), cudaMemcpyHostToDevice));
+  if (A->format == TBSLA_FMT_CSR) TB_TRY(grad_segments(A));
   TB_CUDA(cudaDeviceSynchronize());
   return TBSLA_OK;
 }
@@ -937,8 +939,7 @@ tbsla_status_t tbsla_matrix_info(const tbsla_matrix_t *A, tbsla_matrix_info_t *i
   case TBSLA_FMT_CSR:
     if (A->rows > 0 && A->stored > 0) {
       if (A->csr_variant == 0) {
-        k = (A->n_short > 0) + (A->n_chunk_rows > 0);
-        for (int c = 0; c < kGroupClasses; ++c) k += A->item_class_start[c + 1] > A->item_class_start[c];
+        k = 1 + (A->n_chunk_rows > 0);
       }
       else k = 1 + (A->num_huge > 0);
     }
@@ -946,8 +947,7 @@ tbsla_status_t tbsla_matrix_info(const tbsla_matrix_t *A, tbsla_matrix_info_t *i
   case TBSLA_FMT_COO:
   case TBSLA_FMT_SCOO:
     if (A->stored > 0 && A->coo_rowptr && A->csr_variant == 0) {
-      k = (A->n_short > 0) + (A->n_chunk_rows > 0);
-      for (int c = 0; c < kGroupClasses; ++c) k += A->item_class_start[c + 1] > A->item_class_start[c];
+      k = 1 + (A->n_chunk_rows > 0);
     } else {
       k = A->stored > 0 ? 2 : 0;
     }

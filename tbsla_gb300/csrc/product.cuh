@@ -125,6 +125,9 @@ tbsla_status_t launch_csr_direct(const tbsla_matrix *A, const int *rowptr, const
     kt.stop();
     return TBSLA_OK;
   }
+  // two lanes per short row: asked for, or FP64 values and rows long enough
+  const bool pair = A->short_mode == 2 || (A->short_mode < 0 && sizeof(V) == 8 &&
+                                           A->short_nnz >= (int64_t)kPairMinRow * A->n_short);
   if (A->n_short > 0 && stage_on(A)) {
     // all rows short: the staged kernel
     const size_t smem = csr_stage_setup<V, XT, Epi>(A->stage_cap);
@@ -143,35 +146,34 @@ tbsla_status_t launch_csr_direct(const tbsla_matrix *A, const int *rowptr, const
     else
       csr_tiny_kernel<4, V, XT, Epi><<<grid, 256, 0, s>>>(A->n_short, rowptr, colidx, vals, x, A->f_col,
                                                           xkeep_of<XT>(A), epi);
-  } else if (A->n_short > 0 && (A->short_mode == 2 || (A->short_mode < 0 && sizeof(V) == 8 &&
-                                                       A->short_nnz >= (int64_t)kPairMinRow * A->n_short))) {
-    // two lanes per row
+  } else if (A->n_warp_items == 0 && A->n_short > 0 && pair) {
     csr_pair_kernel<V, XT, Epi><<<short_grid(2 * (int64_t)A->n_short), 256, 0, s>>>(
-        A->short_rows, A->n_short, rowptr, colidx, vals, x, A->f_col, xkeep_of<XT>(A), epi);
-  } else if (A->n_short > 0) {
-    csr_short_kernel<V, XT, Epi><<<short_grid(A->n_short), 256, 0, s>>>(
-        A->short_rows, A->n_short, rowptr, colidx, vals, x, A->f_col, xkeep_of<XT>(A), epi);
-  }
-  for (int c = 0; c < kGroupClasses; ++c) {
-    const int first = A->item_class_start[c], count = A->item_class_start[c + 1] - first;
-    if (count == 0) continue;
-    const int grid = group_grid(count, kGroupLanes[c]);
-    const int4 *items = A->warp_items + first;
-    Acc *parts = chunk_partials_of<Acc>(A);
-    switch (kGroupLanes[c]) {
-    case 4:
-      csr_group_kernel<4, V, XT, Epi><<<grid, 256, 0, s>>>(items, count, colidx, vals, x, A->f_col, xkeep_of<XT>(A), parts, epi);
-      break;
-    case 8:
-      csr_group_kernel<8, V, XT, Epi><<<grid, 256, 0, s>>>(items, count, colidx, vals, x, A->f_col, xkeep_of<XT>(A), parts, epi);
-      break;
-    case 16:
-      csr_group_kernel<16, V, XT, Epi><<<grid, 256, 0, s>>>(items, count, colidx, vals, x, A->f_col, xkeep_of<XT>(A), parts, epi);
-      break;
-    default:
-      csr_group_kernel<32, V, XT, Epi><<<grid, 256, 0, s>>>(items, count, colidx, vals, x, A->f_col, xkeep_of<XT>(A), parts, epi);
-      break;
+        A->n_short, rowptr, colidx, vals, x, A->f_col, xkeep_of<XT>(A), epi);
+  } else if (A->n_warp_items == 0 && A->n_short > 0) {
+    csr_short_kernel<V, XT, Epi><<<short_grid(A->n_short), 256, 0, s>>>(A->n_short, rowptr, colidx, vals, x, A->f_col,
+                                                                       xkeep_of<XT>(A), epi);
+  } else if (A->n_warp_items > 0) {
+    // long rows: every class and the short rows in one launch
+    MixedPlan p{};
+    p.items = A->warp_items;
+    p.rows = A->short_rows;
+    p.n_short = A->n_short;
+    for (int c = 0; c <= kGroupClasses; ++c) p.start[c] = A->item_class_start[c];
+    int blocks = 0;
+    for (int c = kGroupClasses - 1; c >= 0; --c) {
+      p.first[c] = blocks;
+      const int n = p.start[c + 1] - p.start[c];
+      if (n > 0) blocks += group_grid(n, kGroupLanes[c]);
     }
+    p.first[kGroupClasses] = blocks;
+    Acc *parts = chunk_partials_of<Acc>(A);
+    if (A->n_short > 0) blocks += short_grid((pair ? 2 : 1) * (int64_t)A->n_short);
+    if (pair)
+      csr_mixed_kernel<true, V, XT, Epi><<<blocks, 256, 0, s>>>(p, rowptr, colidx, vals, x, A->f_col, xkeep_of<XT>(A),
+                                                               parts, epi);
+    else
+      csr_mixed_kernel<false, V, XT, Epi><<<blocks, 256, 0, s>>>(p, rowptr, colidx, vals, x, A->f_col, xkeep_of<XT>(A),
+                                                                parts, epi);
   }
   kt.stop();
   if (A->n_chunk_rows > 0) {

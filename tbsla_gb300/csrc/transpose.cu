@@ -19,87 +19,69 @@ tbsla_status_t rederive_stores(tbsla_matrix *A, cudaStream_t s);
 
 namespace {
 
-// out[k] = scale * a[row] * b[col - f_col] over the short rows (one thread each)
-template <typename T>
-__global__ void __launch_bounds__(256) grad_short_kernel(const int *__restrict__ rows, int n_rows,
-                                                        const int *__restrict__ rowptr,
-                                                        const int *__restrict__ colidx, int f_col,
-                                                        const T *__restrict__ a, const T *__restrict__ b, T scale,
-                                                        T *__restrict__ out) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n_rows; t += stride) {
-    const int r = rows ? rows[t] : (int)t;
-    const T ar = scale * a[r];
-    for (int k = rowptr[r]; k < rowptr[r + 1]; ++k) out[k] = ar * b[colidx[k] - f_col];
-  }
-}
+// out[k] = scale * a[row(k)] * b[col(k) - f_col].  A warp takes segments of
+// kGradSeg consecutive entries whatever their rows, so the column loads and
+// gradient stores are coalesced and hub rows spread over warps; seg_row[s] is
+// the row of segment s's first entry.  The lanes hold the ends of the 32 rows
+// from there on, and a lane finds its entry's row by a binary search over them
+// (shuffles); a segment that leaves those 32 rows goes on with the next 32.
+// The segment's index loads, then its gathers (b with the handle's L2 policy
+// for x, TBSLA_TUNE_X_L2_KEEP), are in flight together.  One row per thread
+// for short rows and 4 to 32 lanes per long row left R-MAT 2^16 at 175 us, 120
+// of them its hub rows.
+constexpr int kGradSeg = 128;
 
-// All rows short and consecutive (b, the gathered vector, read with the
-// handle's L2 policy for x, TBSLA_TUNE_X_L2_KEEP): a warp takes 32 rows [r0, r0 + 32) and
-// strides its lanes over the segment's entries, so index loads and gradient
-// stores are coalesced; a lane finds the row of its entry by a binary search
-// over the 32 row starts held one per lane (shuffles).  Four strides of the
-// warp go together (128 entries: their index loads, then their gathers, in
-// flight at once; eight measured the same).  The entry loop runs in whole warps (inactive lanes
-// search too, then store nothing), as the full-mask shuffles require.
 template <typename T>
-__global__ void __launch_bounds__(256) grad_segment_kernel(int rows, const int *__restrict__ rowptr,
+__global__ void __launch_bounds__(256) grad_segment_kernel(int rows, int64_t nnz, const int *__restrict__ seg_row,
+                                                          const int *__restrict__ rowptr,
                                                           const int *__restrict__ colidx, int f_col,
                                                           const T *__restrict__ a, const T *__restrict__ b,
                                                           T scale, T *__restrict__ out, XKeep b_keep) {
-  constexpr int U = 4;
+  constexpr int U = kGradSeg / 32;
   const int lane = threadIdx.x & 31;
   const uint64_t keep = policy_keep(b_keep, b);
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * 32 < rows; w += nwarps) {
-    const int r0 = (int)(w * 32);
-    const int mine = min(r0 + lane, rows);
-    const int start = __ldg(rowptr + mine);                    // row start of row r0 + lane
-    const T ar = r0 + lane < rows ? scale * a[r0 + lane] : T(0);
-    const int first = __shfl_sync(0xffffffffu, start, 0);
-    const int end = __ldg(rowptr + min(r0 + 32, rows));
-    for (int e0 = first; e0 < end; e0 += 32 * U) {
-      int col[U];
-      T bv[U];
+  for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w * kGradSeg < nnz; w += nwarps) {
+    const int64_t e0 = w * kGradSeg;
+    const int n = (int)min((int64_t)kGradSeg, nnz - e0);
+    int r0 = __ldg(seg_row + w);
+    int col[U];
+    T bv[U];
+    #pragma unroll
+    for (int u = 0; u < U; ++u) col[u] = 32 * u + lane < n ? ld_stream(colidx + e0 + 32 * u + lane) : f_col;
+    #pragma unroll
+    for (int u = 0; u < U; ++u) bv[u] = 32 * u + lane < n ? ld_keep(b + (col[u] - f_col), keep) : T(0);
+    int done = 0;  // entries of the segment in rows before r0
+    while (done < n) {
+      const int r = min(r0 + lane, rows - 1);
+      // the end of row r0 + lane, relative to the segment
+      const int end = (int)min((int64_t)__ldg(rowptr + r + 1) - e0, (int64_t)kGradSeg);
+      const T ar = scale * __ldg(a + r);
+      const int last = min(__shfl_sync(0xffffffffu, end, 31), n);
       #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int e = e0 + 32 * u + lane;
-        col[u] = e < end ? ld_stream(colidx + e) : f_col;
-      }
-      #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int e = e0 + 32 * u + lane;
-        bv[u] = e < end ? ld_keep(b + (col[u] - f_col), keep) : T(0);
-      }
-      #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int e = e0 + 32 * u + lane;
-        int j = 0;  // largest lane index with start <= e
+        const int e = 32 * u + lane;
+        if (32 * u >= last || 32 * u + 32 <= done) continue;  // uniform: no entry of these rows here
+        int j = 0;  // rows that end at or before e
         #pragma unroll
         for (int step = 16; step >= 1; step >>= 1) {
-          const int cand = j + step;
-          const int v = __shfl_sync(0xffffffffu, start, cand & 31);
-          if (cand < 32 && v <= e) j = cand;
+          const int v = __shfl_sync(0xffffffffu, end, j + step - 1);
+          if (v <= e) j += step;
         }
         const T arow = __shfl_sync(0xffffffffu, ar, j);
-        if (e < end) __stcs(out + e, arow * bv[u]);
+        if (e >= done && e < last) __stcs(out + e0 + e, arow * bv[u]);
       }
+      done = last;
+      r0 += 32;
     }
   }
 }
 
-// the same over the long-row items, L lanes per item
-template <int L, typename T>
-__global__ void __launch_bounds__(256) grad_group_kernel(const int4 *__restrict__ items, int n_items,
-                                                        const int *__restrict__ colidx, int f_col,
-                                                        const T *__restrict__ a, const T *__restrict__ b, T scale,
-                                                        T *__restrict__ out) {
-  const int64_t ng = ((int64_t)gridDim.x * blockDim.x) / L;
-  const int lane = threadIdx.x & (L - 1);
-  for (int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / L; g < n_items; g += ng) {
-    const int4 it = items[g];
-    const T ar = scale * a[it.x];
-    for (int k = it.y + lane; k < it.z; k += L) out[k] = ar * b[colidx[k] - f_col];
+// seg_row[s] = the row of entry s * kGradSeg
+__global__ void grad_segments_kernel(int rows, const int *__restrict__ rowptr, int *__restrict__ seg_row) {
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
+    const int a = rowptr[r], b = rowptr[r + 1];
+    for (int64_t s = ((int64_t)a + kGradSeg - 1) / kGradSeg; s * kGradSeg < b; ++s) seg_row[s] = (int)r;
   }
 }
 
@@ -115,33 +97,25 @@ bool csr_direct(const tbsla_matrix *A) { return A && A->format == TBSLA_FMT_CSR 
 template <typename T>
 tbsla_status_t grad_values(const tbsla_matrix *A, const T *a, const T *b, T scale, T *out, cudaStream_t s) {
   if (A->stored == 0 || A->rows == 0) return TBSLA_OK;
-  if (A->short_rows == nullptr && A->n_short == A->rows) {  // every row short, in order
-    const int warps = (A->rows + 31) / 32;
-    grad_segment_kernel<T><<<(int)std::min<int64_t>(((int64_t)warps + 7) / 8, 152 * 64), 256, 0, s>>>(
-        A->rows, A->idx0, A->idx1, A->f_col, a, b, scale, out, xkeep_of<T>(A));
-    TB_CUDA(cudaGetLastError());
-    return TBSLA_OK;
-  }
-  if (A->n_short > 0)
-    grad_short_kernel<T><<<(int)(((int64_t)A->n_short + 255) / 256), 256, 0, s>>>(
-        A->short_rows, A->n_short, A->idx0, A->idx1, A->f_col, a, b, scale, out);
-  for (int c = 0; c < kGroupClasses; ++c) {
-    const int first = A->item_class_start[c], count = A->item_class_start[c + 1] - first;
-    if (count == 0) continue;
-    const int grid = group_grid(count, kGroupLanes[c]);
-    const int4 *items = A->warp_items + first;
-    switch (kGroupLanes[c]) {
-    case 4: grad_group_kernel<4, T><<<grid, 256, 0, s>>>(items, count, A->idx1, A->f_col, a, b, scale, out); break;
-    case 8: grad_group_kernel<8, T><<<grid, 256, 0, s>>>(items, count, A->idx1, A->f_col, a, b, scale, out); break;
-    case 16: grad_group_kernel<16, T><<<grid, 256, 0, s>>>(items, count, A->idx1, A->f_col, a, b, scale, out); break;
-    default: grad_group_kernel<32, T><<<grid, 256, 0, s>>>(items, count, A->idx1, A->f_col, a, b, scale, out); break;
-    }
-  }
+  const int64_t segs = (A->stored + kGradSeg - 1) / kGradSeg;
+  grad_segment_kernel<T><<<(int)std::min<int64_t>((segs + 7) / 8, 152 * 64), 256, 0, s>>>(
+      A->rows, A->stored, A->seg_row, A->idx0, A->idx1, A->f_col, a, b, scale, out, xkeep_of<T>(A));
   TB_CUDA(cudaGetLastError());
   return TBSLA_OK;
 }
 
 }  // namespace
+
+// The segments' rows of a CSR handle, at its creation (the row structure only)
+tbsla_status_t grad_segments(tbsla_matrix *A) {
+  if (A->stored == 0 || A->rows == 0) return TBSLA_OK;
+  const int64_t segs = (A->stored + kGradSeg - 1) / kGradSeg;
+  TB_TRY(dev_alloc(A, (void **)&A->seg_row, (size_t)segs * sizeof(int)));
+  grad_segments_kernel<<<(int)std::min<int64_t>(((int64_t)A->rows + 255) / 256, 152 * 16), 256>>>(A->rows, A->idx0,
+                                                                                               A->seg_row);
+  TB_CUDA(cudaGetLastError());
+  return TBSLA_OK;
+}
 
 // The transposed copy of a CSR handle, built on first use.
 tbsla_status_t ensure_transpose(tbsla_matrix *A, tbsla_matrix **T) {
