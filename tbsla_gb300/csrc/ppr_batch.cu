@@ -48,7 +48,7 @@ tbsla_status_t pr_relabelled(tbsla_matrix *A, tbsla_matrix **B);
 
 namespace {
 
-constexpr int kPprChunk = 512;
+constexpr int kPprChunkMin = 64, kPprChunkMax = 512;
 
 struct ColCtl {
   double add;    // beta * d.x + cst of the current iterate
@@ -260,6 +260,28 @@ __device__ __forceinline__ void ppr_gather_parts(const T (&res)[VW], const doubl
       for (int q = 0; q < VW; ++q) part[2 + j][q] = (double)dots[(j * VW + q) * 256 + threadIdx.x];
 }
 
+// What the kernels of one sweep need, tile t = blockIdx.y of the layout: every
+// array holds the tiles one after another.  All tiles go in one launch, so
+// that they fill the GPU together and a sweep costs as many launches as one
+// tile's.
+template <typename T>
+struct PprSweep {
+  const T *xo;               // iterates
+  T *xn;                     // outputs
+  PprRing<T> ring;
+  const T *rhs;              // added to every sweep, or NULL
+  const unsigned *seeds;
+  const unsigned char *dmask;
+  const ColCtl *col;
+  const ColAa *aa;
+  const double *inv_size;
+  T *chunks;                 // sums of the rows' chunks
+  double *partials;
+  const TileCtl *tile;
+  double beta;
+  int n, slots, nparts;      // rows, chunk slots and partial slots of a tile
+};
+
 // Resident blocks per SM the sweep kernel is compiled for (its register
 // budget, 64 registers): the sweeps are bound by the latency of their
 // gathers, and resident warps keep them in flight (R-MAT 2^22, 256 vectors,
@@ -272,22 +294,29 @@ constexpr int ppr_min_blocks() {
 // items: (row, begin, end, chunk slot or -1).  A row group of G lanes takes
 // an item, lane l its vectors l*VW .. l*VW+VW-1 (one 16-byte gather of the
 // tile row per entry); each vector's sum is one FMA per entry in stored order.
+// Items come in decreasing length (a tile row is whole lines, so their order
+// costs no coalescing): the groups of a warp walk rows of one length and the
+// longest start first.  Groups of eight lanes or more read eight entries with
+// one load per array, a lane each, and share them by shuffles; narrower ones
+// read four, every lane all of them.  Either way the step's gathers are all
+// issued before its first multiply-add, the next item ahead.
 template <typename T, int KT, bool AA>
 __global__ void __launch_bounds__(256, ppr_min_blocks<T, AA>()) ppr_spmm_kernel(const int4 *__restrict__ items, int n_items,
                                                       const int *__restrict__ colidx, const T *__restrict__ values,
-                                                      const T *__restrict__ xo, T *__restrict__ xn,
-                                                      const unsigned *__restrict__ seeds,
-                                                      const unsigned char *__restrict__ dmask,
-                                                      const ColCtl *__restrict__ col, const ColAa *__restrict__ aa,
-                                                      const double *__restrict__ inv_size, double beta,
-                                                      const T *__restrict__ rhs, PprRing<T> ring,
-                                                      T *__restrict__ chunk_partials, double *partials,
-                                                      const TileCtl *tile) {
-  if (*(volatile const int *)&tile->done) return;
+                                                      const PprSweep<T> p) {
+  const int tl = blockIdx.y;
+  if (*(volatile const int *)&p.tile[tl].done) return;
   constexpr int VW = PprLanes<T, KT>::VW, G = PprLanes<T, KT>::G, NV = AA ? 5 : 2;
   const int c = (threadIdx.x & (G - 1)) * VW;  // first vector of this lane
+  const size_t off = (size_t)tl * p.n * KT;
+  const T *__restrict__ xo = p.xo + off;
+  T *__restrict__ xn = p.xn + off;
+  const T *rhs = p.rhs ? p.rhs + off : nullptr;
+  const PprRing<T> ring{AA ? p.ring.r0 + off : nullptr, AA ? p.ring.r1 + off : nullptr,
+                        AA ? p.ring.r2 + off : nullptr};
+  const unsigned *seeds = p.seeds + (size_t)tl * p.n;
   PprCols<VW> pc;
-  ppr_cols<VW, AA>(pc, c, col, inv_size, aa);
+  ppr_cols<VW, AA>(pc, c, p.col + tl * KT, p.inv_size + tl * KT, p.aa + tl * KT);
   const int64_t ng = ((int64_t)gridDim.x * blockDim.x) / G;
   T res[VW];
   double dm[VW];
@@ -299,62 +328,89 @@ __global__ void __launch_bounds__(256, ppr_min_blocks<T, AA>()) ppr_spmm_kernel(
   __shared__ T dots[AA ? 3 * VW * 256 : 1];
   if (AA)
     for (int j = 0; j < 3 * VW; ++j) dots[j * 256 + threadIdx.x] = 0;
-  for (int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G; g < n_items; g += ng) {
-    const int4 it = items[g];
+  int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
+  int4 it = g < n_items ? __ldg(items + g) : make_int4(0, 0, 0, -1);
+  for (; g < n_items; g += ng) {
+    const int4 nx = g + ng < n_items ? __ldg(items + g + ng) : make_int4(0, 0, 0, -1);
     T acc[VW];
     #pragma unroll
     for (int q = 0; q < VW; ++q) acc[q] = 0;
-    // four entries per step, the last step predicated: a short row's
-    // gathers are all issued before its first multiply-add (R-MAT rows are
-    // mostly short, and one entry at a time chains index -> gather -> FMA)
-    for (int e = it.y; e < it.z; e += 4) {
-      const int rem = it.z - e;
-      int cj[4];
-      T vj[4], xj[4][VW];
-      #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        cj[u] = u < rem ? __ldg(colidx + e + u) : 0;
-        vj[u] = u < rem ? __ldg(values + e + u) : T(0);
-      }
-      #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (u < rem) ppr_ld<T, VW>(xo + (size_t)cj[u] * KT + c, xj[u]);
-      #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (u < rem)
+    if constexpr (G >= 8) {
+      const unsigned mask = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << ((threadIdx.x & 31) & ~(G - 1));
+      const int sl = threadIdx.x & (G - 1) & 7;
+      for (int e = it.y; e < it.z; e += 8) {
+        const int rem = it.z - e;
+        const int cm = sl < rem ? __ldg(colidx + e + sl) : 0;
+        const T vm = sl < rem ? __ldg(values + e + sl) : T(0);
+        constexpr int H = 4;  // gathers in flight (registers)
+        #pragma unroll
+        for (int h = 0; h < 8; h += H) {
+          T xj[H][VW];
           #pragma unroll
-          for (int q = 0; q < VW; ++q) acc[q] = fma(vj[u], xj[u][q], acc[q]);
+          for (int u = 0; u < H; ++u) {
+            const int cj = __shfl_sync(mask, cm, h + u, G);
+            if (h + u < rem) ppr_ld<T, VW>(xo + (size_t)cj * KT + c, xj[u]);
+          }
+          #pragma unroll
+          for (int u = 0; u < H; ++u) {
+            const T vj = __shfl_sync(mask, vm, h + u, G);
+            if (h + u < rem)
+              #pragma unroll
+              for (int q = 0; q < VW; ++q) acc[q] = fma(vj, xj[u][q], acc[q]);
+          }
+        }
+      }
+    } else {
+      for (int e = it.y; e < it.z; e += 4) {
+        const int rem = it.z - e;
+        int cj[4];
+        T vj[4], xj[4][VW];
+        #pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          cj[u] = u < rem ? __ldg(colidx + e + u) : 0;
+          vj[u] = u < rem ? __ldg(values + e + u) : T(0);
+        }
+        #pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (u < rem) ppr_ld<T, VW>(xo + (size_t)cj[u] * KT + c, xj[u]);
+        #pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (u < rem)
+            #pragma unroll
+            for (int q = 0; q < VW; ++q) acc[q] = fma(vj[u], xj[u][q], acc[q]);
+      }
     }
     if (it.w >= 0) {
-      ppr_st<T, VW>(chunk_partials + (size_t)it.w * KT + c, acc);
+      ppr_st<T, VW>(p.chunks + ((size_t)tl * p.slots + it.w) * KT + c, acc);
     } else {
       PprRowIn<T, VW, AA> in;
-      ppr_row_in<T, VW, AA>(in, it.x, KT, c, pc, xo, seeds, dmask, rhs, ring);
-      ppr_emit<T, VW, AA>(it.x, KT, c, acc, pc, in, xn, beta, rhs != nullptr, ring, res, dm, dots);
+      ppr_row_in<T, VW, AA>(in, it.x, KT, c, pc, xo, seeds, p.dmask, rhs, ring);
+      ppr_emit<T, VW, AA>(it.x, KT, c, acc, pc, in, xn, p.beta, rhs != nullptr, ring, res, dm, dots);
     }
+    it = nx;
   }
   double part[NV][VW];
   ppr_gather_parts<T, VW, NV, AA>(res, dm, dots, part);
-  block_columns<KT, VW, NV>(part, partials, blockIdx.x);
+  block_columns<KT, VW, NV>(part, p.partials + (size_t)tl * p.nparts * KT * NV, blockIdx.x);
 }
 
 // rows cut into chunks: crow[h] = (row, first slot), crow[n].y = total slots;
-// the chunks' sums are added in order
+// the chunks' sums are added in order, eight loads in flight
 template <typename T, int KT, bool AA>
-__global__ void __launch_bounds__(256) ppr_fixup_kernel(const int2 *__restrict__ crow, int n_crow,
-                                                       const T *__restrict__ chunk_partials,
-                                                       const T *__restrict__ xo, T *__restrict__ xn,
-                                                       const unsigned *__restrict__ seeds,
-                                                       const unsigned char *__restrict__ dmask,
-                                                       const ColCtl *__restrict__ col, const ColAa *__restrict__ aa,
-                                                       const double *__restrict__ inv_size, double beta,
-                                                       const T *__restrict__ rhs, PprRing<T> ring, double *partials,
-                                                       int part_base, const TileCtl *tile) {
-  if (*(volatile const int *)&tile->done) return;
+__global__ void __launch_bounds__(256) ppr_fixup_kernel(const int2 *__restrict__ crow, int n_crow, int part_base,
+                                                       const PprSweep<T> p) {
+  const int tl = blockIdx.y;
+  if (*(volatile const int *)&p.tile[tl].done) return;
   constexpr int VW = PprLanes<T, KT>::VW, G = PprLanes<T, KT>::G, NV = AA ? 5 : 2;
   const int c = (threadIdx.x & (G - 1)) * VW;
+  const size_t off = (size_t)tl * p.n * KT;
+  const T *xo = p.xo + off;
+  const T *rhs = p.rhs ? p.rhs + off : nullptr;
+  const PprRing<T> ring{AA ? p.ring.r0 + off : nullptr, AA ? p.ring.r1 + off : nullptr,
+                        AA ? p.ring.r2 + off : nullptr};
+  const T *chunks = p.chunks + (size_t)tl * p.slots * KT;
   PprCols<VW> pc;
-  ppr_cols<VW, AA>(pc, c, col, inv_size, aa);
+  ppr_cols<VW, AA>(pc, c, p.col + tl * KT, p.inv_size + tl * KT, p.aa + tl * KT);
   const int64_t ng = ((int64_t)gridDim.x * blockDim.x) / G;
   T res[VW];
   double dm[VW];
@@ -368,50 +424,64 @@ __global__ void __launch_bounds__(256) ppr_fixup_kernel(const int2 *__restrict__
     for (int j = 0; j < 3 * VW; ++j) dots[j * 256 + threadIdx.x] = 0;
   for (int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G; g < n_crow; g += ng) {
     const int2 h = crow[g];
+    const int end = crow[g + 1].y;
+    PprRowIn<T, VW, AA> in;
+    ppr_row_in<T, VW, AA>(in, h.x, KT, c, pc, xo, p.seeds + (size_t)tl * p.n, p.dmask, rhs, ring);
     T acc[VW];
     #pragma unroll
     for (int q = 0; q < VW; ++q) acc[q] = 0;
-    for (int s = h.y; s < crow[g + 1].y; ++s) {
-      T p[VW];
-      ppr_ld<T, VW>(chunk_partials + (size_t)s * KT + c, p);
+    for (int s = h.y; s < end; s += 8) {
+      T v[8][VW];
       #pragma unroll
-      for (int q = 0; q < VW; ++q) acc[q] += p[q];
+      for (int u = 0; u < 8; ++u)
+        if (s + u < end) ppr_ld<T, VW>(chunks + (size_t)(s + u) * KT + c, v[u]);
+      #pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (s + u < end)
+          #pragma unroll
+          for (int q = 0; q < VW; ++q) acc[q] += v[u][q];
     }
-    PprRowIn<T, VW, AA> in;
-    ppr_row_in<T, VW, AA>(in, h.x, KT, c, pc, xo, seeds, dmask, rhs, ring);
-    ppr_emit<T, VW, AA>(h.x, KT, c, acc, pc, in, xn, beta, rhs != nullptr, ring, res, dm, dots);
+    ppr_emit<T, VW, AA>(h.x, KT, c, acc, pc, in, p.xn + off, p.beta, rhs != nullptr, ring, res, dm, dots);
   }
   double part[NV][VW];
   ppr_gather_parts<T, VW, NV, AA>(res, dm, dots, part);
-  block_columns<KT, VW, NV>(part, partials, part_base + blockIdx.x);
+  block_columns<KT, VW, NV>(part, p.partials + (size_t)tl * p.nparts * KT * NV, part_base + blockIdx.x);
 }
 
 // per column: sum the parts in order, advance the column, then the tile.
 // Accelerated: the new output's term and residual dots enter the column's
 // history and the weights of the next input are solved (aa_coefficients); a
 // column that stops takes its last output as it is.
-// 1024 threads: warp w sums the parts w, w + 32, ... in order, its lanes
-// reading each part's KT * NV values together; then the warps' sums are added
-// in order, and one thread per column advances it.
+// kPprFin blocks a tile (blockIdx.y): block b takes the parts b, b + kPprFin,
+// ... (its warps every 32nd of them in order, the lanes a part's KT * NV values
+// together, then the warps in order), and the block that arrives last adds the
+// blocks' sums in order and, one thread per column, advances the columns.  One
+// block for all parts took 55 us for the 1824 parts of a 32-vector tile.
+constexpr int kPprFin = 16;
 template <int KT, bool AA>
-__global__ void __launch_bounds__(1024) ppr_finalize_kernel(const double *__restrict__ partials, int nparts,
-                                                           ColCtl *col, ColAa *aa, TileCtl *tile, double beta,
-                                                           double cst, int max_iter, int k_in_tile, int first) {
+__global__ void __launch_bounds__(1024) ppr_finalize_kernel(const double *__restrict__ all_partials, size_t tile_parts,
+                                                           int nparts, double *fin, unsigned *arrived, ColCtl *cols,
+                                                           ColAa *aas, TileCtl *tiles, double beta, double cst,
+                                                           int max_iter, int k, int first) {
   constexpr int NV = AA ? 5 : 2, W = KT * NV, PER = (W + 31) / 32;
   __shared__ double sh[32][W];
-  __shared__ int active;
-  if (threadIdx.x == 0) active = 0;
-  __syncthreads();
+  __shared__ int active, last;
+  const int tl = blockIdx.y;
+  TileCtl *tile = tiles + tl;
+  ColCtl *col = cols + tl * KT;
+  ColAa *aa = aas + tl * KT;
   if (*(volatile int *)&tile->done) {
-    if (threadIdx.x == 0) tile->ran = 0;
+    if (threadIdx.x == 0 && blockIdx.x == 0) tile->ran = 0;
     return;
   }
+  if (threadIdx.x == 0) active = 0;
+  const double *partials = all_partials + (size_t)tl * tile_parts * W;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double a[PER];
   #pragma unroll
   for (int i = 0; i < PER; ++i) a[i] = 0;
   #pragma unroll 4
-  for (int p = warp; p < nparts; p += 32)
+  for (int p = blockIdx.x + kPprFin * warp; p < nparts; p += 32 * kPprFin)
     #pragma unroll
     for (int i = 0; i < PER; ++i)
       if (lane + 32 * i < W) a[i] += partials[(size_t)p * W + lane + 32 * i];
@@ -419,10 +489,27 @@ __global__ void __launch_bounds__(1024) ppr_finalize_kernel(const double *__rest
   for (int i = 0; i < PER; ++i)
     if (lane + 32 * i < W) sh[warp][lane + 32 * i] = a[i];
   __syncthreads();
+  double *mine = fin + (size_t)tl * kPprFin * W;
   if (threadIdx.x < W) {
     double t = 0;
     for (int w = 0; w < 32; ++w) t += sh[w][threadIdx.x];
-    sh[0][threadIdx.x] = t;  // read only by this thread above
+    __stcg(mine + (size_t)blockIdx.x * W + threadIdx.x, t);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicInc(arrived + tl, kPprFin - 1) == kPprFin - 1;  // back to 0 with the last
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return;
+  if (threadIdx.x < W) {
+    double b[kPprFin], t = 0;
+    #pragma unroll
+    for (int w = 0; w < kPprFin; ++w) b[w] = __ldcg(mine + (size_t)w * W + threadIdx.x);
+    #pragma unroll
+    for (int w = 0; w < kPprFin; ++w) t += b[w];
+    sh[0][threadIdx.x] = t;
   }
   __syncthreads();
   const int c = threadIdx.x;
@@ -462,7 +549,7 @@ __global__ void __launch_bounds__(1024) ppr_finalize_kernel(const double *__rest
     } else {
       cc.add = beta * d + cst;
     }
-    if (c < k_in_tile && !cc.done) atomicOr(&active, 1);
+    if (tl * KT + c < k && !cc.done) atomicOr(&active, 1);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -478,9 +565,12 @@ __global__ void __launch_bounds__(1024) ppr_finalize_kernel(const double *__rest
 template <typename T, int KT>
 __global__ void __launch_bounds__(256) ppr_combine_kernel(int n, const T *__restrict__ g0,
                                                          const T *__restrict__ g1, const T *__restrict__ g2,
-                                                         T *__restrict__ x, const ColAa *__restrict__ aa,
-                                                         const TileCtl *tile) {
-  if (!*(volatile const int *)&tile->ran) return;
+                                                         T *__restrict__ x, const ColAa *__restrict__ aas,
+                                                         const TileCtl *tiles) {
+  const int tl = blockIdx.y;
+  if (!*(volatile const int *)&tiles[tl].ran) return;
+  const ColAa *aa = aas + tl * KT;
+  const size_t off = (size_t)tl * n * KT;
   constexpr int VW = PprLanes<T, KT>::VW, G = PprLanes<T, KT>::G;
   const int c = (threadIdx.x & (G - 1)) * VW;
   T c0[VW], c1[VW], c2[VW];
@@ -496,7 +586,7 @@ __global__ void __launch_bounds__(256) ppr_combine_kernel(int n, const T *__rest
   }
   const int64_t ng = ((int64_t)gridDim.x * blockDim.x) / G;
   for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G; i < n; i += ng) {
-    const size_t at = (size_t)i * KT + c;
+    const size_t at = off + (size_t)i * KT + c;
     T a[VW], b[VW], e[VW], v[VW];
     ppr_ld<T, VW>(g0 + at, a);
     if (mm >= 1) ppr_ld<T, VW>(g1 + at, b);
@@ -591,9 +681,12 @@ __global__ void ppr_seed_bits_kernel(unsigned *seeds, int n, const int2 *__restr
   }
 }
 
-// The work list of a handle's batched sweeps: rows, and rows longer than
-// kPprChunk entries cut into chunks; built once (it depends on the row
-// structure only) and kept on the handle.
+// The work list of a handle's batched sweeps in decreasing length: rows, and
+// rows longer than a chunk cut into chunks; built once (it depends on the row
+// structure only) and kept on the handle.  A chunk is walked by one row group,
+// so it is a 16384th of the entries, 64 to 512: on small graphs a long chunk
+// outlasts the sweep (R-MAT 2^17, 32 FP32 vectors: 179 us a sweep with chunks
+// of 512 entries), on large ones short chunks only cost partial sums.
 struct PprPlan {
   int4 *items = nullptr;  // (row, begin, end, chunk slot or -1)
   int2 *crow = nullptr;   // chunked rows: (row, first slot); crow[n_crow].y = slots
@@ -614,18 +707,29 @@ tbsla_status_t ppr_plan(const tbsla_matrix *Mc, const PprPlan **out) {
   const int n = M->n_row;
   std::vector<int> rp((size_t)n + 1);
   TB_CUDA(cudaMemcpy(rp.data(), M->idx0, ((size_t)n + 1) * sizeof(int), cudaMemcpyDeviceToHost));
+  int chunk = kPprChunkMin;
+  while (chunk < kPprChunkMax && (int64_t)chunk * 2 * 16384 <= M->stored) chunk *= 2;
   std::vector<int4> items;
   std::vector<int2> crow;
   int slots = 0;
   items.reserve((size_t)n);
   for (int r = 0; r < n; ++r) {
     const int a = rp[(size_t)r], b = rp[(size_t)r + 1];
-    if (b - a <= kPprChunk) {
+    if (b - a <= chunk) {
       items.push_back(make_int4(r, a, b, -1));
       continue;
     }
     crow.push_back(make_int2(r, slots));
-    for (int e = a; e < b; e += kPprChunk) items.push_back(make_int4(r, e, std::min(e + kPprChunk, b), slots++));
+    for (int e = a; e < b; e += chunk) items.push_back(make_int4(r, e, std::min(e + chunk, b), slots++));
+  }
+  // decreasing length, equal lengths in row order (a counting sort)
+  {
+    std::vector<size_t> at((size_t)chunk + 2, 0);
+    for (const int4 &q : items) ++at[(size_t)(chunk - (q.z - q.y)) + 1];
+    for (size_t l = 1; l < at.size(); ++l) at[l] += at[l - 1];
+    std::vector<int4> sorted(items.size());
+    for (const int4 &q : items) sorted[at[(size_t)(chunk - (q.z - q.y))]++] = q;
+    items.swap(sorted);
   }
   PprPlan *P = new PprPlan;
   P->n_items = (int)items.size();
@@ -728,14 +832,12 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
     for (int v : dist) pairs.push_back(make_int2(c, v));
     inv[(size_t)c] = 1.0 / (double)dist.size();
   }
-  // the sweep grid: two waves of the blocks that fit on the GPU at once (a
-  // grid-stride loop; one wave leaves SMs idle in its tail, more waves give
-  // the finalize more per-block partials to add: R-MAT 2^20, 64 vectors,
-  // 16 waves 1.47 ms per sweep + 0.75 ms finalize, 1 wave 1.58 + 0.05)
+  // the sweep grid of a tile: the blocks that fit on the GPU at once (the items
+  // are dealt in decreasing length, so one wave is even)
   int sms = 0, per_sm = 0;
   TB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, M->device));
   TB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ppr_spmm_kernel<T, KT, AA>, 256, 0));
-  const int grid_mm = std::max(1, 2 * sms * std::max(per_sm, 1));
+  const int grid_mm = std::max(1, sms * std::max(per_sm, 1));
   const int grid_fx = std::max(1, std::min((n_crow * G + 255) / 256, sms * 4));
   const int grid_in = 152 * 4;
   const int grid_vec = 152 * 8;  // streaming passes over a tile (combine, compaction)
@@ -749,7 +851,8 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
   int2 *d_pairs = nullptr;
   unsigned char *dmask = nullptr;
   int *d_zeros = nullptr;
-  double *d_inv = nullptr, *partials = nullptr;
+  double *d_inv = nullptr, *partials = nullptr, *fin = nullptr;
+  unsigned *arrived = nullptr;
   ColCtl *d_col = nullptr;
   ColAa *d_aa = nullptr;
   TileCtl *d_tile = nullptr;
@@ -775,7 +878,9 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
   } else {
     alloc((void **)&x[1], (size_t)tiles * xbytes);
   }
-  alloc((void **)&chunk, (size_t)std::max(slots, 1) * KT * sizeof(T));
+  alloc((void **)&chunk, (size_t)tiles * std::max(slots, 1) * KT * sizeof(T));
+  alloc((void **)&fin, (size_t)tiles * kPprFin * KT * NV * sizeof(double));
+  alloc((void **)&arrived, (size_t)tiles * sizeof(unsigned));
   alloc((void **)&d_seeds, (size_t)tiles * n * sizeof(unsigned));
   alloc((void **)&d_pairs, pairs.size() * sizeof(int2));
   alloc((void **)&dmask, (size_t)n);
@@ -817,6 +922,7 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
     if (e == cudaSuccess && b) e = cudaMemcpyAsync(d, h, b, cudaMemcpyHostToDevice, s);
   };
   up(d_pairs, pairs.data(), pairs.size() * sizeof(int2));
+  if (e == cudaSuccess) e = cudaMemsetAsync(arrived, 0, (size_t)tiles * sizeof(unsigned), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(d_seeds, 0, (size_t)tiles * n * sizeof(unsigned), s);
   if (e == cudaSuccess)
     ppr_seed_bits_kernel<KT><<<152, 256, 0, s>>>(d_seeds, n, d_pairs, (int)pairs.size());
@@ -840,9 +946,17 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
     if (opt.rhs)
       ppr_load_kernel<T, KT, NV><<<grid_in, 256, 0, s>>>(n, opt.rhs, d_vec + (size_t)t * KT, newid_dev, dmask,
                                                          rhs_t[0] + (size_t)t * n * KT, nullptr);
-    ppr_finalize_kernel<KT, AA><<<1, 1024, 0, s>>>(pt, grid_in, d_col + (size_t)t * KT, d_aa + (size_t)t * KT,
-                                                 d_tile + t, beta, cst, p->max_iter, std::min(KT, k - t * KT), 1);
   }
+  // launches over the tiles of a layout (blockIdx.y, at most kTilesPerLaunch)
+  constexpr int kTilesPerLaunch = 65535;
+  auto finalize = [&](int count, int parts, int first) {
+    for (int t = 0; t < count; t += kTilesPerLaunch)
+      ppr_finalize_kernel<KT, AA><<<dim3(kPprFin, std::min(kTilesPerLaunch, count - t)), 1024, 0, s>>>(
+          partials + (size_t)t * nparts * KT * NV, (size_t)nparts, parts, fin + (size_t)t * kPprFin * KT * NV,
+          arrived + t, d_col + (size_t)t * KT, d_aa + (size_t)t * KT, d_tile + t, beta, cst, p->max_iter,
+          first ? k - t * KT : count * KT, first);
+  };
+  finalize(tiles, grid_in, 1);
   int rbase = 0;  // rhs_t[rbase] holds the current layout's right-hand side
   if (cudaGetLastError() != cudaSuccess) { cleanup(); return fail(TBSLA_ERR_CUDA, "batched PageRank init"); }
   // Sweeps in sets of K on every tile of the current layout (stopped tiles
@@ -864,39 +978,43 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
   int *d_map = nullptr;
   alloc((void **)&d_map, (size_t)tiles * KT * sizeof(int));
   if (st != TBSLA_OK) { cleanup(); return st; }
-  std::vector<char> tile_live((size_t)tiles, 1);
   int phase = 0;
   const size_t tstride = (size_t)n * KT;
   while (true) {
     for (int k2 = 0; k2 < K; ++k2, ++phase, ++gk) {
       const int w = (int)(gk % 3), w1 = (int)((gk + 2) % 3), w2 = (int)((gk + 1) % 3);
-      for (int t = 0; t < cur_tiles; ++t) {
-        if (!tile_live[(size_t)t]) continue;  // stopped before this set of K sweeps
+      for (int t = 0; t < cur_tiles; t += kTilesPerLaunch) {
+        const unsigned count = (unsigned)std::min(kTilesPerLaunch, cur_tiles - t);
         const size_t off = (size_t)t * tstride;
-        const T *xo = AA ? x[0] + off : x[(base + phase) & 1] + off;
-        T *xn = AA ? g_ring[w] + off : x[(base + phase + 1) & 1] + off;
-        PprRing<T> ring{AA ? r_ring[w] + off : nullptr, AA ? r_ring[w1] + off : nullptr,
-                        AA ? r_ring[w2] + off : nullptr};
-        double *pt = partials + (size_t)t * nparts * KT * NV;
-        const unsigned *sd = d_seeds + (size_t)t * n;
-        const ColCtl *cl = d_col + (size_t)t * KT;
-        const ColAa *ca = d_aa + (size_t)t * KT;
-        const double *iv = d_inv + (size_t)t * KT;
-        const T *rh = opt.rhs ? rhs_t[rbase] + off : nullptr;
-        ppr_spmm_kernel<T, KT, AA><<<grid_mm, 256, 0, s>>>(plan->items, plan->n_items, M->idx1, values, xo, xn,
-                                                           sd, dmask, cl, ca, iv, beta, rh, ring, chunk, pt,
-                                                           d_tile + t);
+        PprSweep<T> sw;
+        sw.xo = AA ? x[0] + off : x[(base + phase) & 1] + off;
+        sw.xn = AA ? g_ring[w] + off : x[(base + phase + 1) & 1] + off;
+        sw.ring = PprRing<T>{AA ? r_ring[w] + off : nullptr, AA ? r_ring[w1] + off : nullptr,
+                             AA ? r_ring[w2] + off : nullptr};
+        sw.rhs = opt.rhs ? rhs_t[rbase] + off : nullptr;
+        sw.seeds = d_seeds + (size_t)t * n;
+        sw.dmask = dmask;
+        sw.col = d_col + (size_t)t * KT;
+        sw.aa = d_aa + (size_t)t * KT;
+        sw.inv_size = d_inv + (size_t)t * KT;
+        sw.chunks = chunk + (size_t)t * slots * KT;
+        sw.partials = partials + (size_t)t * nparts * KT * NV;
+        sw.tile = d_tile + t;
+        sw.beta = beta;
+        sw.n = n;
+        sw.slots = slots;
+        sw.nparts = nparts;
+        ppr_spmm_kernel<T, KT, AA><<<dim3(grid_mm, count), 256, 0, s>>>(plan->items, plan->n_items, M->idx1, values, sw);
         if (n_crow)
-          ppr_fixup_kernel<T, KT, AA><<<grid_fx, 256, 0, s>>>(plan->crow, n_crow, chunk, xo, xn, sd, dmask, cl, ca,
-                                                              iv, beta, rh, ring, pt, grid_mm, d_tile + t);
-        ppr_finalize_kernel<KT, AA><<<1, 1024, 0, s>>>(pt, n_crow ? grid_mm + grid_fx : grid_mm,
-                                                     d_col + (size_t)t * KT, d_aa + (size_t)t * KT, d_tile + t,
-                                                     beta, cst, p->max_iter, KT, 0);
-        if (AA)
-          ppr_combine_kernel<T, KT><<<grid_vec, 256, 0, s>>>(n, g_ring[w] + off, g_ring[w1] + off,
-                                                            g_ring[w2] + off, x[0] + off, d_aa + (size_t)t * KT,
-                                                            d_tile + t);
+          ppr_fixup_kernel<T, KT, AA><<<dim3(grid_fx, count), 256, 0, s>>>(plan->crow, n_crow, grid_mm, sw);
       }
+      finalize(cur_tiles, n_crow ? grid_mm + grid_fx : grid_mm, 0);
+      if (AA)
+        for (int t = 0; t < cur_tiles; t += kTilesPerLaunch) {
+          const size_t off = (size_t)t * tstride;
+          ppr_combine_kernel<T, KT><<<dim3(grid_vec, std::min(kTilesPerLaunch, cur_tiles - t)), 256, 0, s>>>(
+              n, g_ring[w] + off, g_ring[w1] + off, g_ring[w2] + off, x[0] + off, d_aa + (size_t)t * KT, d_tile + t);
+        }
     }
     if (cudaMemcpyAsync(htc.data(), d_tile, (size_t)cur_tiles * sizeof(TileCtl), cudaMemcpyDeviceToHost, s) !=
             cudaSuccess ||
@@ -934,7 +1052,6 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
         const T *xf = (AA ? x[0] : x[(base + htc[(size_t)t].iter) & 1]) + (size_t)t * tstride;
         ppr_pick_kernel<T, KT><<<152 * 8, 256, 0, s>>>(xf, n, newid_dev, pk, d_out);
       }
-      tile_live[(size_t)t] = !htc[(size_t)t].done;
       busy += !htc[(size_t)t].done;
     }
     if (cudaGetLastError() != cudaSuccess) { cleanup(); return fail(TBSLA_ERR_CUDA, "batched PageRank results"); }
@@ -995,7 +1112,6 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
       cur_tiles = need;
       slot_vec = nvec;
       inv = ninv;
-      std::fill(tile_live.begin(), tile_live.end(), 1);
     }
   }
   if (cudaStreamSynchronize(s) != cudaSuccess || cudaGetLastError() != cudaSuccess) {
