@@ -15,7 +15,7 @@ namespace tbsla {
 
 tbsla_status_t spmv_dispatch(const tbsla_matrix *A, tbsla_dtype_t store, tbsla_dtype_t xt, const void *x,
                              tbsla_dtype_t yt, void *y, int vect_incr, cudaStream_t s);
-tbsla_status_t rederive_stores(tbsla_matrix *A, cudaStream_t s);
+tbsla_status_t sell_refresh(tbsla_matrix *A, cudaStream_t s);
 
 namespace {
 
@@ -85,11 +85,27 @@ __global__ void grad_segments_kernel(int rows, const int *__restrict__ rowptr, i
   }
 }
 
-// dst[k'] = src[perm[k']]
-__global__ void permute_values_kernel(const double *__restrict__ src, const int *__restrict__ perm, int64_t n,
-                                      double *__restrict__ dst) {
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
-    dst[k] = src[perm[k]];
+// entry k' of the transposed copy's stores from new values at perm[k'], four
+// gathers of a thread in flight
+template <typename S>
+__global__ void __launch_bounds__(256) permute_values_kernel(const S *__restrict__ src, const int *__restrict__ perm,
+                                                            int64_t n, double *__restrict__ f64,
+                                                            float *__restrict__ f32,
+                                                            __nv_bfloat16 *__restrict__ bf16) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += 4 * stride) {
+    S v[4];
+    #pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = k + u * stride < n ? __ldg(src + ld_stream(perm + k + u * stride)) : S(0);
+    #pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int64_t at = k + u * stride;
+      if (at >= n) break;
+      if (f64) f64[at] = (double)v[u];
+      if (f32) f32[at] = sizeof(S) == 8 ? __double2float_rn((double)v[u]) : (float)v[u];
+      if (bf16) bf16[at] = __double2bfloat16((double)v[u]);
+    }
+  }
 }
 
 bool csr_direct(const tbsla_matrix *A) { return A && A->format == TBSLA_FMT_CSR && A->csr_variant == 0; }
@@ -163,15 +179,23 @@ tbsla_status_t ensure_transpose(tbsla_matrix *A, tbsla_matrix **T) {
   return TBSLA_OK;
 }
 
-// After A's F64 values changed: the copy's values follow
-tbsla_status_t transpose_refresh(tbsla_matrix *A, cudaStream_t s) {
-  if (!A->transpose) return TBSLA_OK;
+// After A's values changed to d_values: the copy's stores follow in one pass
+// (and, where it has one, its ELL-layout copy)
+tbsla_status_t transpose_refresh(tbsla_matrix *A, tbsla_dtype_t type, const void *d_values, cudaStream_t s) {
+  if (!A->transpose || !A->stored) return TBSLA_OK;
   tbsla_matrix *T = A->transpose;
-  if (A->stored)
-    permute_values_kernel<<<152 * 8, 256, 0, s>>>(static_cast<const double *>(A->values[0]), A->transpose_perm,
-                                                 A->stored, static_cast<double *>(T->values[0]));
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((A->stored + 1023) / 1024, 152 * 32));
+  double *f64 = static_cast<double *>(T->values[0]);
+  float *f32 = static_cast<float *>(T->values[1]);
+  __nv_bfloat16 *bf16 = static_cast<__nv_bfloat16 *>(T->values[2]);
+  if (type == TBSLA_F64)
+    permute_values_kernel<double><<<grid, 256, 0, s>>>(static_cast<const double *>(d_values), A->transpose_perm,
+                                                       A->stored, f64, f32, bf16);
+  else
+    permute_values_kernel<float><<<grid, 256, 0, s>>>(static_cast<const float *>(d_values), A->transpose_perm,
+                                                      A->stored, f64, f32, bf16);
   TB_CUDA(cudaGetLastError());
-  return rederive_stores(T, s);
+  return sell_refresh(T, s);
 }
 
 tbsla_status_t grad_values_f64(const tbsla_matrix *A, const double *a, const double *b, double scale, double *out,
