@@ -258,9 +258,21 @@ tbsla_status_t launch_product(const tbsla_matrix *A, const V *vals, const XT *x,
     break;
   case TBSLA_FMT_DENSE:
     if (A->rows > 0 && A->cols > 0) {
-      const int warps = (A->rows + 3) / 4;
+      // 16-byte loads when every row and x start on 16 bytes
+      constexpr int VW = 16 / (int)sizeof(V);
+      const bool vec = A->cols % VW == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+      // warps per row group: as many as leave each four steps of columns, so
+      // that blocks are short and many (8000 x 9001 FP64 in blocks of 35 steps,
+      // one wave and a tenth: 281 us, against 175 with few, long blocks)
+      const int64_t groups = ((int64_t)A->rows + kDenseRows - 1) / kDenseRows;
+      const int batch = 32 * (vec ? VW * (VW == 8 ? 2 : 4) : 8);  // columns of a warp's step
+      int splits = 1;
+      while (splits < 8 && A->cols / (2 * splits) >= 4 * batch) splits *= 2;
+      while (splits < 8 && groups * splits < 152 * 16 && A->cols / (2 * splits) >= 128) splits *= 2;
+      const int grid = (int)((groups * splits + 7) / 8);
       KernelTimer kt(A, s);
-      dense_kernel<V, XT, Epi><<<(warps + 7) / 8, 256, 0, s>>>(vals, x, A->rows, A->cols, epi);
+      if (vec) dense_kernel<VW, V, XT, Epi><<<grid, 256, 0, s>>>(vals, x, A->rows, A->cols, splits, epi);
+      else dense_kernel<1, V, XT, Epi><<<grid, 256, 0, s>>>(vals, x, A->rows, A->cols, splits, epi);
       kt.stop();
     }
     break;
