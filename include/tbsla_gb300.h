@@ -487,9 +487,10 @@ tbsla_status_t tbsla_pagerank_adjoint(const tbsla_matrix_t *A, const tbsla_pager
  * whose residual combination is smallest, as in tbsla_pagerank; same
  * stopping rule and fixed point, fewer sweeps).  d_out: n*k doubles, vector
  * c at d_out + c*n; iterations / residuals: k host entries each, or NULL.
- * Allocates its work buffers per call: 2 n k values of the precision, 7 n k
- * with acceleration (iterate, three outputs, three residuals).  No reference
- * counterpart. */
+ * Work buffers: 2 n k values of the precision, 7 n k with acceleration
+ * (iterate, three outputs, three residuals); up to 512 MiB of them stay with
+ * the handle for its next solve (concurrent solves allocate their own).  No
+ * reference counterpart. */
 tbsla_status_t tbsla_ppr_batched(const tbsla_matrix_t *A, const tbsla_pagerank_params_t *p, int k,
                                  const int *nodes, const int *offsets, int tile, double *d_out, int *iterations,
                                  double *residuals, void *stream);
@@ -503,8 +504,8 @@ tbsla_status_t tbsla_ppr_batched(const tbsla_matrix_t *A, const tbsla_pagerank_p
  * p->accel = 1, whose FP32 solves are accelerated) and x += e, at most
  * 8 rounds.  FP64 is used only for the residual sweeps, the L1 norms and the
  * update.  iterations: FP32 and FP64 sweeps together; residuals: the last
- * ||r_c||_1.  Allocates 2 n k doubles of work space per call (stream
- * ordered).  No reference counterpart. */
+ * ||r_c||_1.  2 n k doubles of work space beside the solves' (kept with the
+ * handle up to 512 MiB).  No reference counterpart. */
 tbsla_status_t tbsla_ppr_batched_refined(const tbsla_matrix_t *A, const tbsla_pagerank_params_t *p, int k,
                                          const int *nodes, const int *offsets, int tile, double *d_out,
                                          int *iterations, double *residuals, void *stream);

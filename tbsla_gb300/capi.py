@@ -322,14 +322,14 @@ class DeviceMatrix:
     # -- products on host vectors -------------------------------------
     def spmv_host(self, x: np.ndarray, vect_incr: int = 0) -> np.ndarray:
         x = np.ascontiguousarray(x, np.float64)
-        y = np.zeros(max(self.info().n_row, 1), np.float64)
+        y = np.empty(max(self.info().n_row, 1), np.float64)  # the call writes every entry
         check(lib().tbsla_spmv_host(self.h, _ptr(x), x.size, _ptr(y), y.size, vect_incr))
         return y[: self.info().n_row]
 
     def a_axpx_host(self, x: np.ndarray, vect_incr: int = 0) -> np.ndarray:
         x = np.ascontiguousarray(x, np.float64)
         n = self.info().n_row
-        y = np.zeros(max(n, 1), np.float64)
+        y = np.empty(max(n, 1), np.float64)  # the call writes every entry
         check(lib().tbsla_a_axpx_host(self.h, _ptr(x), x.size, _ptr(y), y.size, vect_incr))
         return y[:n]
 

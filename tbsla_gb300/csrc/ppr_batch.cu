@@ -36,6 +36,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "anderson.cuh"
@@ -687,21 +688,96 @@ __global__ void ppr_seed_bits_kernel(unsigned *seeds, int n, const int2 *__restr
 // so it is a 16384th of the entries, 64 to 512: on small graphs a long chunk
 // outlasts the sweep (R-MAT 2^17, 32 FP32 vectors: 179 us a sweep with chunks
 // of 512 entries), on large ones short chunks only cost partial sums.
+// Device memory kept with the handle between solves (allocating and freeing a
+// solve's two dozen buffers took a third of a 64-vector solve on R-MAT 2^17:
+// six FP32 and FP64 solves of a refined one).  One solve holds it at a time,
+// others allocate their own; more than kPprKeepBytes is given back at the end
+// of the solve, the rest with the handle.
+constexpr size_t kPprKeepBytes = (size_t)512 << 20;
+struct PprMemory {
+  std::mutex busy;
+  char *base = nullptr;
+  size_t bytes = 0;
+};
+// The buffers of one solve, cut from one allocation: add() the requests, then
+// get(); released (after the work that uses it) by the destructor.
+class PprBuffers {
+ public:
+  PprBuffers(PprMemory *kept, cudaStream_t s) : kept_(kept), s_(s) {}
+  ~PprBuffers() {
+    if (!base_) return;
+    cudaStreamSynchronize(s_);
+    if (!mine_) {
+      if (kept_->bytes > kPprKeepBytes) drop();
+      kept_->busy.unlock();
+    } else {
+      cudaFree(base_);
+    }
+  }
+  template <typename T> void add(T **p, size_t bytes) {
+    req_.push_back({reinterpret_cast<void **>(p), (bytes + 255) / 256 * 256 + 256});
+  }
+  tbsla_status_t get() {
+    size_t total = 0;
+    for (auto &r : req_) total += r.second;
+    mine_ = !kept_->busy.try_lock();
+    cudaError_t e = cudaSuccess;
+    if (mine_) {
+      e = cudaMalloc((void **)&base_, total);
+    } else {
+      if (kept_->bytes < total) {
+        drop();
+        e = cudaMalloc((void **)&kept_->base, total);
+        if (e == cudaSuccess) kept_->bytes = total;
+        else kept_->base = nullptr;
+      }
+      base_ = kept_->base;
+      if (e != cudaSuccess) kept_->busy.unlock();
+    }
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      base_ = nullptr;
+      return fail(TBSLA_ERR_OOM, "batched PageRank buffers (%zu bytes)", total);
+    }
+    char *p = base_;
+    for (auto &r : req_) {
+      *r.first = p;
+      p += r.second;
+    }
+    return TBSLA_OK;
+  }
+
+ private:
+  void drop() {
+    if (kept_->base) cudaFree(kept_->base);
+    kept_->base = nullptr;
+    kept_->bytes = 0;
+  }
+  PprMemory *kept_;
+  cudaStream_t s_;
+  char *base_ = nullptr;
+  bool mine_ = false;
+  std::vector<std::pair<void **, size_t>> req_;
+};
+
 struct PprPlan {
+  PprMemory solve, refine;  // buffers of a solve, and of the refinement around it
   int4 *items = nullptr;  // (row, begin, end, chunk slot or -1)
   int2 *crow = nullptr;   // chunked rows: (row, first slot); crow[n_crow].y = slots
   int n_items = 0, n_crow = 0, slots = 0;
 };
 void ppr_plan_free(void *q) {
   PprPlan *P = static_cast<PprPlan *>(q);
+  if (P->solve.base) cudaFree(P->solve.base);
+  if (P->refine.base) cudaFree(P->refine.base);
   if (P->items) cudaFree(P->items);
   if (P->crow) cudaFree(P->crow);
   delete P;
 }
-tbsla_status_t ppr_plan(const tbsla_matrix *Mc, const PprPlan **out) {
+tbsla_status_t ppr_plan(const tbsla_matrix *Mc, PprPlan **out) {
   tbsla_matrix *M = const_cast<tbsla_matrix *>(Mc);
   if (M->ppr_plan) {
-    *out = static_cast<const PprPlan *>(M->ppr_plan);
+    *out = static_cast<PprPlan *>(M->ppr_plan);
     return TBSLA_OK;
   }
   const int n = M->n_row;
@@ -809,7 +885,7 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
   const T *values = static_cast<const T *>(M->values[std::is_same<T, double>::value ? 0 : 1]);
   TB_CHECK(values, "the matrix lacks the %s value store", std::is_same<T, double>::value ? "F64" : "F32");
   const int tiles = (k + KT - 1) / KT;
-  const PprPlan *plan = nullptr;
+  PprPlan *plan = nullptr;
   TB_TRY(ppr_plan(M, &plan));
   const int n_crow = plan->n_crow, slots = plan->slots;
   // seeds: bit c of seeds[t*n + i] = row i is a seed of vector t*KT + c, set
@@ -858,17 +934,10 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
   TileCtl *d_tile = nullptr;
   T *rhs_t[2] = {nullptr, nullptr};  // the right-hand side in the tiles' layout (ping-pong for repacking)
   int *d_vec = nullptr;              // per slot: the column of x0 / rhs it holds, or -1
-  std::vector<void *> owned;
-  tbsla_status_t st = TBSLA_OK;
-  auto alloc = [&](void **ptr, size_t bytes) {
-    if (st != TBSLA_OK) return;
-    if (cudaMalloc(ptr, std::max<size_t>(bytes, 16)) != cudaSuccess) {
-      cudaGetLastError();
-      st = fail(TBSLA_ERR_OOM, "batched PageRank buffers (%zu bytes)", bytes);
-      return;
-    }
-    owned.push_back(*ptr);
-  };
+  char *d_ctl = nullptr;  // tile, column and Anderson state, one after another: one copy reads them
+  int *d_map = nullptr;
+  PprBuffers buffers(&plan->solve, s);
+  auto alloc = [&](void **ptr, size_t bytes) { buffers.add(ptr, bytes); };
   alloc((void **)&x[0], (size_t)tiles * xbytes);
   if (AA) {
     for (int j = 0; j < 3; ++j) {
@@ -887,19 +956,20 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
   alloc((void **)&d_zeros, sizeof(int));
   alloc((void **)&d_inv, inv.size() * sizeof(double));
   alloc((void **)&partials, (size_t)tiles * nparts * KT * NV * sizeof(double));
-  alloc((void **)&d_col, (size_t)tiles * KT * sizeof(ColCtl));
-  alloc((void **)&d_aa, (size_t)tiles * KT * sizeof(ColAa));
-  alloc((void **)&d_tile, (size_t)tiles * sizeof(TileCtl));
+  const size_t col_at = (size_t)tiles * sizeof(TileCtl), aa_at = col_at + (size_t)tiles * KT * sizeof(ColCtl);
+  const size_t ctl_bytes = aa_at + (AA ? (size_t)tiles * KT * sizeof(ColAa) : 0);
+  static_assert(sizeof(TileCtl) % 8 == 0 && sizeof(ColCtl) % 8 == 0, "the control arrays follow one another");
+  alloc((void **)&d_ctl, aa_at + (size_t)tiles * KT * sizeof(ColAa));
   alloc((void **)&d_vec, (size_t)tiles * KT * sizeof(int));
+  alloc((void **)&d_map, (size_t)tiles * KT * sizeof(int));
   if (opt.rhs) {
     alloc((void **)&rhs_t[0], (size_t)tiles * xbytes);
     if (!AA) alloc((void **)&rhs_t[1], (size_t)tiles * xbytes);
   }
-  auto cleanup = [&]() {
-    cudaStreamSynchronize(s);
-    for (void *q : owned) cudaFree(q);
-  };
-  if (st != TBSLA_OK) { cleanup(); return st; }
+  TB_TRY(buffers.get());
+  d_tile = reinterpret_cast<TileCtl *>(d_ctl);
+  d_col = reinterpret_cast<ColCtl *>(d_ctl + col_at);
+  d_aa = reinterpret_cast<ColAa *>(d_ctl + aa_at);
   const double cst = opt.cst < 0 ? 1.0 - p->beta : opt.cst;
   auto src_col = [&](int v) { return v < 0 ? -1 : opt.src ? opt.src[v] : v; };
   std::vector<ColCtl> hcol((size_t)tiles * KT);
@@ -931,9 +1001,8 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
   up(d_aa, haa.data(), haa.size() * sizeof(ColAa));
   up(d_tile, htile.data(), htile.size() * sizeof(TileCtl));
   up(d_vec, hvec.data(), hvec.size() * sizeof(int));
-  if (e != cudaSuccess) { cleanup(); return fail(TBSLA_ERR_CUDA, "batched PageRank upload: %s", cudaGetErrorString(e)); }
-  st = column_mask(const_cast<tbsla_matrix *>(M), values, dmask, d_zeros, s);
-  if (st != TBSLA_OK) { cleanup(); return st; }
+  if (e != cudaSuccess) return fail(TBSLA_ERR_CUDA, "batched PageRank upload: %s", cudaGetErrorString(e));
+  TB_TRY(column_mask(const_cast<tbsla_matrix *>(M), values, dmask, d_zeros, s));
   const double beta = p->beta;
   for (int t = 0; t < tiles; ++t) {
     double *pt = partials + (size_t)t * nparts * KT * NV;
@@ -958,7 +1027,7 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
   };
   finalize(tiles, grid_in, 1);
   int rbase = 0;  // rhs_t[rbase] holds the current layout's right-hand side
-  if (cudaGetLastError() != cudaSuccess) { cleanup(); return fail(TBSLA_ERR_CUDA, "batched PageRank init"); }
+  if (cudaGetLastError() != cudaSuccess) return fail(TBSLA_ERR_CUDA, "batched PageRank init");
   // Sweeps in sets of K on every tile of the current layout (stopped tiles
   // return at once).  After each set the vectors that stopped are written
   // out and dropped; when the live vectors fit in fewer tiles they are
@@ -967,7 +1036,8 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
   // plain, the layout's iterates start in x[base] and sweep j reads
   // x[(base+j)&1]; accelerated, sweep number gk of the solve writes ring slot
   // gk % 3.
-  const int K = p->check_every > 0 ? p->check_every : 4;  // 4: R-MAT 2^22, 256 vectors, 3-9 % faster than 8
+  // sweeps per look of the host (4: R-MAT 2^22, 256 vectors, 3-9 % faster than 8)
+  const int K = std::min(p->check_every > 0 ? p->check_every : 4, std::max(p->max_iter, 1));
   int cur_tiles = tiles, base = 0;
   int64_t gk = 0;
   std::vector<int> slot_vec((size_t)tiles * KT, -1);  // vector in each slot, -1 for none
@@ -975,9 +1045,7 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
   std::vector<TileCtl> htc((size_t)tiles);
   std::vector<ColCtl> hcc((size_t)tiles * KT);
   std::vector<ColAa> hca((size_t)tiles * KT);
-  int *d_map = nullptr;
-  alloc((void **)&d_map, (size_t)tiles * KT * sizeof(int));
-  if (st != TBSLA_OK) { cleanup(); return st; }
+  std::vector<char> hctl(ctl_bytes);
   int phase = 0;
   const size_t tstride = (size_t)n * KT;
   while (true) {
@@ -1016,16 +1084,12 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
               n, g_ring[w] + off, g_ring[w1] + off, g_ring[w2] + off, x[0] + off, d_aa + (size_t)t * KT, d_tile + t);
         }
     }
-    if (cudaMemcpyAsync(htc.data(), d_tile, (size_t)cur_tiles * sizeof(TileCtl), cudaMemcpyDeviceToHost, s) !=
-            cudaSuccess ||
-        cudaMemcpyAsync(hcc.data(), d_col, (size_t)cur_tiles * KT * sizeof(ColCtl), cudaMemcpyDeviceToHost, s) !=
-            cudaSuccess ||
-        (AA && cudaMemcpyAsync(hca.data(), d_aa, (size_t)cur_tiles * KT * sizeof(ColAa), cudaMemcpyDeviceToHost,
-                               s) != cudaSuccess) ||
-        cudaStreamSynchronize(s) != cudaSuccess) {
-      cleanup();
+    if (cudaMemcpyAsync(hctl.data(), d_ctl, ctl_bytes, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess)
       return fail(TBSLA_ERR_CUDA, "batched PageRank sweeps failed");
-    }
+    std::memcpy(htc.data(), hctl.data(), (size_t)cur_tiles * sizeof(TileCtl));
+    std::memcpy(hcc.data(), hctl.data() + col_at, (size_t)cur_tiles * KT * sizeof(ColCtl));
+    if (AA) std::memcpy(hca.data(), hctl.data() + aa_at, (size_t)cur_tiles * KT * sizeof(ColAa));
     // write out and drop the vectors that stopped (a stopped vector is
     // frozen: plain, its tile's last iterate, x[(base + tile iter) & 1],
     // holds it; accelerated, x; a stopped tile's vectors have all stopped,
@@ -1054,7 +1118,7 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
       }
       busy += !htc[(size_t)t].done;
     }
-    if (cudaGetLastError() != cudaSuccess) { cleanup(); return fail(TBSLA_ERR_CUDA, "batched PageRank results"); }
+    if (cudaGetLastError() != cudaSuccess) return fail(TBSLA_ERR_CUDA, "batched PageRank results");
     if (live == 0) break;
     const int need = (live + KT - 1) / KT;
     if (need < busy) {
@@ -1092,7 +1156,7 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
       up(d_col, ncol.data(), ncol.size() * sizeof(ColCtl));
       if (AA) up(d_aa, naa.data(), naa.size() * sizeof(ColAa));
       up(d_tile, ntile.data(), ntile.size() * sizeof(TileCtl));
-      if (e != cudaSuccess) { cleanup(); return fail(TBSLA_ERR_CUDA, "batched PageRank repack: %s", cudaGetErrorString(e)); }
+      if (e != cudaSuccess) return fail(TBSLA_ERR_CUDA, "batched PageRank repack: %s", cudaGetErrorString(e));
       if (AA) {
         T *bufs[8] = {x[0], g_ring[0], g_ring[1], g_ring[2], r_ring[0], r_ring[1], r_ring[2], rhs_t[0]};
         for (int t = 0; t < need; ++t)
@@ -1107,18 +1171,15 @@ tbsla_status_t run_tiles_impl(const tbsla_matrix *M, const int *newid_dev, const
         }
         base = src ^ 1;
       }
-      if (cudaGetLastError() != cudaSuccess) { cleanup(); return fail(TBSLA_ERR_CUDA, "batched PageRank repack"); }
+      if (cudaGetLastError() != cudaSuccess) return fail(TBSLA_ERR_CUDA, "batched PageRank repack");
       phase = 0;
       cur_tiles = need;
       slot_vec = nvec;
       inv = ninv;
     }
   }
-  if (cudaStreamSynchronize(s) != cudaSuccess || cudaGetLastError() != cudaSuccess) {
-    cleanup();
+  if (cudaStreamSynchronize(s) != cudaSuccess || cudaGetLastError() != cudaSuccess)
     return fail(TBSLA_ERR_CUDA, "batched PageRank results");
-  }
-  cleanup();
   return TBSLA_OK;
 }
 
@@ -1165,21 +1226,12 @@ tbsla_status_t run_refined(const tbsla_matrix *M, const int *nd, const std::vect
   q.tol = std::max(p->tol, kF32SolveFloor);
   TB_TRY((run_tiles<float, KT>(M, nd, nh, &q, k, nodes, offsets, d_out, itot.data(), nullptr, s)));
   double *g = nullptr, *e = nullptr;
-  TB_CUDA(cudaMallocAsync((void **)&g, (size_t)total * sizeof(double), s));
-  if (cudaMallocAsync((void **)&e, (size_t)total * sizeof(double), s) != cudaSuccess) {
-    cudaGetLastError();
-    cudaFreeAsync(g, s);
-    return fail(TBSLA_ERR_OOM, "refinement buffers (2 x %lld doubles)", (long long)total);
-  }
-  struct Free {
-    cudaStream_t s;
-    double *a, *b;
-    ~Free() {
-      cudaFreeAsync(a, s);
-      cudaFreeAsync(b, s);
-      cudaStreamSynchronize(s);
-    }
-  } release{s, g, e};
+  PprPlan *plan = nullptr;
+  TB_TRY(ppr_plan(M, &plan));
+  PprBuffers buffers(&plan->refine, s);
+  buffers.add(&g, (size_t)total * sizeof(double));
+  buffers.add(&e, (size_t)total * sizeof(double));
+  TB_TRY(buffers.get());
   const int grid = 152 * 8;
   for (int round = 0;; ++round) {
     // r = G(x) - x: one FP64 sweep from x (the sweep's L1 change is ||r_c||_1)
