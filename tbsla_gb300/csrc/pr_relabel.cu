@@ -21,13 +21,14 @@
 // length) descending, so that neighbouring rows have similar lengths and
 // the thread-per-row kernel's warps run similar trip counts.
 //
-// The copy is built once per handle on the host (download, counting sort by
-// degree, row copy) and uploaded as an ordinary CSR handle with the same
-// value stores.
+// The copy is built once per handle on the device (a stable sort of the
+// vertices by degree, then of the entries by new row and column), an ordinary
+// CSR handle with the same value stores.
 #include <algorithm>
 #include <vector>
 
 #include "common.cuh"
+#include "device_sort.cuh"
 
 namespace tbsla {
 
@@ -65,6 +66,41 @@ __global__ void column_count_kernel(const int *__restrict__ colidx, int64_t nnz,
     atomicAdd(deg + (colidx[k] - f_col), 1);  // columns are in [f_col, f_col + n) (candidate())
 }
 
+// key: out-degree class descending, then in-degree (row length) descending;
+// class = floor(log2(out-degree + 1))
+__global__ void vertex_keys_kernel(const int *__restrict__ deg, const int *__restrict__ rowptr, int n, int top_cls,
+                                   uint64_t *__restrict__ keys, int *__restrict__ verts) {
+  for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
+    const int cls = 31 - __clz(deg[v] + 1);
+    keys[v] = (uint64_t)(top_cls - cls) << 32 | (uint32_t)(0x7fffffff - (rowptr[v + 1] - rowptr[v]));
+    verts[v] = (int)v;
+  }
+}
+
+// newid[order[i]] = i
+__global__ void new_labels_kernel(const int *__restrict__ order, int n, int *__restrict__ newid) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    newid[order[i]] = (int)i;
+}
+
+__global__ void relabelled_keys_kernel(const int *__restrict__ row, const int *__restrict__ col, int f_col,
+                                       const int *__restrict__ newid, int64_t nnz, int n,
+                                       uint64_t *__restrict__ keys, int *__restrict__ entries) {
+  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nnz; k += (int64_t)gridDim.x * blockDim.x) {
+    keys[k] = (uint64_t)newid[row[k]] * (uint64_t)n + (uint64_t)newid[col[k] - f_col];
+    entries[k] = (int)k;
+  }
+}
+
+__global__ void split_keys_kernel(const uint64_t *__restrict__ keys, int64_t nnz, int n, int *__restrict__ row,
+                                  int *__restrict__ col) {
+  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nnz; k += (int64_t)gridDim.x * blockDim.x) {
+    const uint64_t r = keys[k] / (uint64_t)n;
+    row[k] = (int)r;
+    col[k] = (int)(keys[k] - r * (uint64_t)n);
+  }
+}
+
 int cls_max(int maxdeg) { return 31 - __builtin_clz((unsigned)maxdeg + 1u); }
 
 bool candidate(const tbsla_matrix *A) {
@@ -89,15 +125,15 @@ tbsla_status_t build(tbsla_matrix *A, bool check_skew, bool *built) {
   *built = false;
   const int n = A->n_row;
   const int64_t nnz = A->stored;
-  // out-degrees on the device
+  // out-degrees
+  SortScratch degrees;
   int *d_deg = nullptr;
-  TB_CUDA(cudaMalloc(&d_deg, (size_t)n * sizeof(int)));
-  cudaMemset(d_deg, 0, (size_t)n * sizeof(int));
+  TB_TRY(degrees.get(&d_deg, n));
+  TB_CUDA(cudaDeviceSynchronize());  // A's values and arrays are in place, whichever stream wrote them
+  TB_CUDA(cudaMemset(d_deg, 0, (size_t)n * sizeof(int)));
   column_count_kernel<<<152 * 8, 256>>>(A->idx1, nnz, A->f_col, d_deg);
   std::vector<int> deg((size_t)n);
-  const cudaError_t e = cudaMemcpy(deg.data(), d_deg, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost);
-  cudaFree(d_deg);
-  TB_CUDA(e);
+  TB_CUDA(cudaMemcpy(deg.data(), d_deg, (size_t)n * sizeof(int), cudaMemcpyDeviceToHost));
   const int maxdeg = *std::max_element(deg.begin(), deg.end());
   if (check_skew) {
     // entries in the columns of the n/10 vertices of highest out-degree
@@ -111,104 +147,64 @@ tbsla_status_t build(tbsla_matrix *A, bool check_skew, bool *built) {
     }
     if (2 * top < nnz) return TBSLA_OK;  // no hot set worth packing
   }
-  std::vector<int> rp((size_t)n + 1), ci((size_t)nnz);
-  std::vector<double> va((size_t)nnz);
-  TB_TRY(tbsla_csr_download(A, rp.data(), ci.data(), va.data()));
-  // two stable counting sorts: by in-degree (descending), then by out-degree
-  // class (descending)
-  int maxin = 0;
-  for (int v = 0; v < n; ++v) maxin = std::max(maxin, rp[(size_t)v + 1] - rp[(size_t)v]);
-  std::vector<int> by_in((size_t)n), order((size_t)n);
-  {
-    std::vector<int64_t> start((size_t)maxin + 2, 0);
-    for (int v = 0; v < n; ++v) ++start[(size_t)(maxin - (rp[(size_t)v + 1] - rp[(size_t)v])) + 1];
-    for (size_t k = 1; k < start.size(); ++k) start[k] += start[k - 1];
-    for (int v = 0; v < n; ++v) by_in[(size_t)start[(size_t)(maxin - (rp[(size_t)v + 1] - rp[(size_t)v]))]++] = v;
-  }
-  {
-    auto cls = [&](int v) { return 31 - __builtin_clz((unsigned)deg[(size_t)v] + 1u); };  // floor(log2(d + 1))
-    const int top_cls = cls_max(maxdeg);
-    std::vector<int64_t> start((size_t)top_cls + 2, 0);
-    for (int v = 0; v < n; ++v) ++start[(size_t)(top_cls - cls(v)) + 1];
-    for (size_t k = 1; k < start.size(); ++k) start[k] += start[k - 1];
-    for (int i = 0; i < n; ++i) {
-      const int v = by_in[(size_t)i];
-      order[(size_t)start[(size_t)(top_cls - cls(v))]++] = v;
+  // vertices by out-degree class, then in-degree, both descending: one stable
+  // sort of (class, in-degree) keys
+  const int grid = entry_grid(n), egrid = entry_grid(nnz);
+  SortScratch sc;
+  uint64_t *vkeys = nullptr, *vsorted = nullptr, *ekeys = nullptr, *esorted = nullptr;
+  int *verts = nullptr, *order = nullptr, *entries = nullptr, *eorder = nullptr, *row = nullptr;
+  double *vals = nullptr;
+  TB_TRY(sc.get(&vkeys, n));
+  TB_TRY(sc.get(&verts, n));
+  const int top_cls = cls_max(maxdeg);
+  vertex_keys_kernel<<<grid, 256>>>(d_deg, A->idx0, n, top_cls, vkeys, verts);
+  TB_TRY(sort_entries(sc, vkeys, verts, n, 32 + key_bits((uint64_t)top_cls), &vsorted, &order));
+  tbsla_matrix *B = new_matrix(TBSLA_FMT_CSR);
+  if (!B) return fail(TBSLA_ERR_OOM, "host allocation failed");
+  struct Guard {
+    tbsla_matrix *B;
+    int *newid = nullptr;
+    ~Guard() {
+      if (newid) cudaFree(newid);
+      if (B) free_matrix(B);
     }
+  } guard{B};
+  B->device = A->device;
+  TB_CUDA(cudaSetDevice(A->device));
+  if (cudaMalloc(&guard.newid, (size_t)n * sizeof(int)) != cudaSuccess) {
+    cudaGetLastError();
+    return fail(TBSLA_ERR_OOM, "relabel map (%d ints)", n);
   }
-  std::vector<int> newid((size_t)n);
-  for (int i = 0; i < n; ++i) newid[(size_t)order[(size_t)i]] = i;
-  // the copy: row i is old row order[i] with columns relabelled
-  std::vector<int> nrp((size_t)n + 1);
-  nrp[0] = 0;
-  for (int i = 0; i < n; ++i) {
-    const int old = order[(size_t)i];
-    nrp[(size_t)i + 1] = nrp[(size_t)i] + (rp[(size_t)old + 1] - rp[(size_t)old]);
-  }
-  std::vector<int> nci((size_t)nnz);
-  std::vector<double> nva((size_t)nnz);
-  const int f_col = A->f_col;
-#pragma omp parallel
-  {
-    std::vector<int> idx;
-    std::vector<int> tc;
-    std::vector<double> tv;
-#pragma omp for schedule(dynamic, 4096)
-    for (int i = 0; i < n; ++i) {
-      const int old = order[(size_t)i];
-      const int o0 = nrp[(size_t)i], len = nrp[(size_t)i + 1] - o0;
-      int *c = nci.data() + o0;
-      double *v = nva.data() + o0;
-      for (int k = 0; k < len; ++k) {
-        c[k] = newid[(size_t)(ci[(size_t)rp[(size_t)old] + k] - f_col)];
-        v[k] = va[(size_t)rp[(size_t)old] + k];
-      }
-      // entries in increasing new column (stable: repeated columns keep their order)
-      if (len <= 64) {
-        for (int k = 1; k < len; ++k) {
-          const int ck = c[k];
-          const double vk = v[k];
-          int j = k - 1;
-          for (; j >= 0 && c[j] > ck; --j) {
-            c[j + 1] = c[j];
-            v[j + 1] = v[j];
-          }
-          c[j + 1] = ck;
-          v[j + 1] = vk;
-        }
-      } else {
-        idx.resize((size_t)len);
-        for (int k = 0; k < len; ++k) idx[(size_t)k] = k;
-        std::stable_sort(idx.begin(), idx.end(), [c](int p, int q) { return c[p] < c[q]; });
-        tc.assign(c, c + len);
-        tv.assign(v, v + len);
-        for (int k = 0; k < len; ++k) {
-          c[k] = tc[(size_t)idx[(size_t)k]];
-          v[k] = tv[(size_t)idx[(size_t)k]];
-        }
-      }
-    }
-  }
-  rp.clear(); rp.shrink_to_fit();
-  ci.clear(); ci.shrink_to_fit();
-  va.clear(); va.shrink_to_fit();
-  tbsla_matrix_t *B = nullptr;
-  TB_TRY(tbsla_csr_create(n, n, 0, n, nrp.data(), nci.data(), nva.data(), A->stores, &B));
+  new_labels_kernel<<<grid, 256>>>(order, n, guard.newid);
+  // the entries by (new row, new column), repeated columns in their order
+  TB_TRY(sc.get(&ekeys, nnz));
+  TB_TRY(sc.get(&entries, nnz));
+  TB_TRY(sc.get(&row, nnz));
+  TB_TRY(sc.get(&vals, nnz));
+  entry_rows_kernel<<<152 * 16, 256>>>(n, A->idx0, row);
+  relabelled_keys_kernel<<<egrid, 256>>>(row, A->idx1, A->f_col, guard.newid, nnz, n, ekeys, entries);
+  TB_TRY(sort_entries(sc, ekeys, entries, nnz, key_bits((uint64_t)n * (uint64_t)n - 1), &esorted, &eorder));
+  B->n_row = B->n_col = B->rows = n;
+  B->stored = nnz;
+  // columns with entries come first (their class is above that of degree 0)
+  B->x_extent = n - std::count(deg.begin(), deg.end(), 0);
+  TB_TRY(alloc_ints(B, &B->idx0, (int64_t)n + 1));
+  TB_TRY(alloc_ints(B, &B->idx1, nnz));
+  split_keys_kernel<<<egrid, 256>>>(esorted, nnz, n, row, B->idx1);  // row: of the sorted entries now
+  key_starts_kernel<<<entry_grid((int64_t)n + 1), 256>>>(row, nnz, (int64_t)n, B->idx0);
+  take_kernel<<<egrid, 256>>>(static_cast<const double *>(A->values[0]), eorder, nnz, vals);
+  TB_CUDA(cudaGetLastError());
+  TB_TRY(store_values_device(B, vals, nnz, A->stores, 0));
+  std::vector<int> nrp((size_t)n + 1), newid((size_t)n);
+  TB_CUDA(cudaMemcpy(nrp.data(), B->idx0, nrp.size() * sizeof(int), cudaMemcpyDeviceToHost));
+  TB_CUDA(cudaMemcpy(newid.data(), guard.newid, newid.size() * sizeof(int), cudaMemcpyDeviceToHost));
+  TB_TRY(csr_bins(B, nrp));
+  int *d_newid = guard.newid;
+  guard.newid = nullptr;
+  guard.B = nullptr;
   B->x_keep = A->x_keep;
   B->x_keep_range = A->x_keep_range;
   B->short_mode = A->short_mode;
-  int *d_newid = nullptr;
-  if (cudaMalloc(&d_newid, (size_t)n * sizeof(int)) != cudaSuccess) {
-    cudaGetLastError();
-    tbsla_matrix_destroy(B);
-    return fail(TBSLA_ERR_OOM, "relabel map (%d ints)", n);
-  }
-  const cudaError_t e2 = cudaMemcpy(d_newid, newid.data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice);
-  if (e2 != cudaSuccess) {
-    cudaFree(d_newid);
-    tbsla_matrix_destroy(B);
-    TB_CUDA(e2);
-  }
   A->pr_relabel = B;
   A->pr_newid = d_newid;
   A->pr_newid_host = std::move(newid);

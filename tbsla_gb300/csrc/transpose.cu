@@ -3,12 +3,13 @@
 // product a b^T sampled on the sparsity pattern), and value replacement.
 //
 // The transposed copy is an ordinary CSR handle (so A^T x runs the same
-// kernels as A x).  It is built once on the host: entries sorted by column,
+// kernels as A x).  It is built once, on the device: entries sorted by column,
 // stably, so that row j of the copy lists column j's entries in increasing
 // row order.  transpose_perm maps its entries back to A's, so new values of A
 // reach the copy by a gather on the device.
 #include <vector>
 
+#include "device_sort.cuh"
 #include "product.cuh"
 
 namespace tbsla {
@@ -108,6 +109,15 @@ __global__ void __launch_bounds__(256) permute_values_kernel(const S *__restrict
   }
 }
 
+// key = column of the block, entry = position
+__global__ void __launch_bounds__(256) column_keys_kernel(const int *__restrict__ col, int f_col, int64_t n,
+                                                         uint32_t *__restrict__ keys, int *__restrict__ entries) {
+  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
+    keys[k] = (uint32_t)(col[k] - f_col);
+    entries[k] = (int)k;
+  }
+}
+
 bool csr_direct(const tbsla_matrix *A) { return A && A->format == TBSLA_FMT_CSR && A->csr_variant == 0; }
 
 template <typename T>
@@ -142,37 +152,63 @@ tbsla_status_t ensure_transpose(tbsla_matrix *A, tbsla_matrix **T) {
   TB_CHECK(A->format == TBSLA_FMT_CSR, "the transpose needs a CSR handle");
   TB_CHECK(A->values[0], "the transpose needs the F64 value store");
   TB_CUDA(cudaSetDevice(A->device));
-  const int rows = A->rows, ncol = A->n_col;
+  const int ncol = A->n_col;
   const int64_t nnz = A->stored;
-  std::vector<int> rp((size_t)rows + 1), ci((size_t)std::max<int64_t>(nnz, 1));
-  std::vector<double> va((size_t)std::max<int64_t>(nnz, 1));
-  TB_TRY(tbsla_csr_download(A, rp.data(), ci.data(), va.data()));
-  std::vector<int> tp((size_t)ncol + 1, 0);
-  for (int64_t k = 0; k < nnz; ++k) ++tp[(size_t)(ci[(size_t)k] - A->f_col) + 1];
-  for (int j = 0; j < ncol; ++j) tp[(size_t)j + 1] += tp[(size_t)j];
-  std::vector<int> next(tp.begin(), tp.end() - 1), tci((size_t)std::max<int64_t>(nnz, 1)),
-      perm((size_t)std::max<int64_t>(nnz, 1));
-  std::vector<double> tva((size_t)std::max<int64_t>(nnz, 1));
-  for (int i = 0; i < rows; ++i)
-    for (int k = rp[(size_t)i]; k < rp[(size_t)i + 1]; ++k) {
-      const int d = next[(size_t)(ci[(size_t)k] - A->f_col)]++;
-      tci[(size_t)d] = i;
-      tva[(size_t)d] = va[(size_t)k];
-      perm[(size_t)d] = k;
+  const int grid = entry_grid(nnz);
+  SortScratch sc;
+  uint32_t *keys = nullptr, *sorted = nullptr;
+  int *entries = nullptr, *order = nullptr, *row = nullptr;
+  double *vals = nullptr;
+  TB_TRY(sc.get(&keys, nnz));
+  TB_TRY(sc.get(&entries, nnz));
+  TB_TRY(sc.get(&row, nnz));
+  TB_TRY(sc.get(&vals, nnz));
+  tbsla_matrix *B = new_matrix(TBSLA_FMT_CSR);
+  if (!B) return fail(TBSLA_ERR_OOM, "host allocation failed");
+  struct Guard {
+    tbsla_matrix *B;
+    int *perm = nullptr;
+    ~Guard() {
+      if (perm) cudaFree(perm);
+      if (B) free_matrix(B);
     }
-  tbsla_matrix_t *B = nullptr;
-  TB_TRY(tbsla_csr_create(ncol, A->n_row, 0, ncol, tp.data(), tci.data(), tva.data(), A->stores, &B));
+  } guard{B};
+  B->device = A->device;
+  TB_CUDA(cudaSetDevice(A->device));
+  B->n_row = ncol;
+  B->n_col = A->n_row;
+  B->rows = ncol;
+  B->stored = nnz;
+  TB_TRY(alloc_ints(B, &B->idx0, (int64_t)ncol + 1));
+  TB_TRY(alloc_ints(B, &B->idx1, nnz));
+  if (cudaMalloc(&guard.perm, (size_t)std::max<int64_t>(nnz, 1) * sizeof(int)) != cudaSuccess) {
+    cudaGetLastError();
+    return fail(TBSLA_ERR_OOM, "transpose map (%lld ints)", (long long)nnz);
+  }
+  TB_CUDA(cudaDeviceSynchronize());  // A's values and arrays are in place, whichever stream wrote them
+  if (nnz) {
+    column_keys_kernel<<<grid, 256>>>(A->idx1, A->f_col, nnz, keys, entries);
+    TB_TRY(sort_entries(sc, keys, entries, nnz, key_bits((uint64_t)std::max(ncol - 1, 0)), &sorted, &order));
+    entry_rows_kernel<<<152 * 16, 256>>>(A->rows, A->idx0, row);
+    take_kernel<<<grid, 256>>>(row, order, nnz, B->idx1);
+    take_kernel<<<grid, 256>>>(static_cast<const double *>(A->values[0]), order, nnz, vals);
+    TB_CUDA(cudaMemcpyAsync(guard.perm, order, (size_t)nnz * sizeof(int), cudaMemcpyDeviceToDevice, 0));
+    int last = 0;  // the entries come in row order: the last one's row is the largest
+    TB_CUDA(cudaMemcpy(&last, row + nnz - 1, sizeof last, cudaMemcpyDeviceToHost));
+    B->x_extent = (int64_t)last + 1;
+  }
+  key_starts_kernel<<<entry_grid((int64_t)ncol + 1), 256>>>(sorted, nnz, (int64_t)ncol, B->idx0);
+  TB_CUDA(cudaGetLastError());
+  TB_TRY(store_values_device(B, vals, nnz, A->stores, 0));
+  std::vector<int> tp((size_t)ncol + 1);
+  TB_CUDA(cudaMemcpy(tp.data(), B->idx0, tp.size() * sizeof(int), cudaMemcpyDeviceToHost));
+  TB_TRY(csr_bins(B, tp));
   B->x_keep = A->x_keep;
   B->x_keep_range = A->x_keep_range;
   B->short_mode = A->short_mode;
-  int *d_perm = nullptr;
-  if (cudaMalloc(&d_perm, (size_t)std::max<int64_t>(nnz, 1) * sizeof(int)) != cudaSuccess ||
-      (nnz && cudaMemcpy(d_perm, perm.data(), (size_t)nnz * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)) {
-    cudaGetLastError();
-    if (d_perm) cudaFree(d_perm);
-    tbsla_matrix_destroy(B);
-    return fail(TBSLA_ERR_OOM, "transpose map (%lld ints)", (long long)nnz);
-  }
+  int *d_perm = guard.perm;
+  guard.perm = nullptr;
+  guard.B = nullptr;
   A->transpose = B;
   A->transpose_perm = d_perm;
   *T = B;

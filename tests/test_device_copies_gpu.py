@@ -1,0 +1,51 @@
+"""The copies a handle builds on the device on first use: the transposed copy
+of blocks (column offset, rows the block does not store, empty rows and
+columns, repeated columns, no entries at all) and the degree-relabelled copy
+of small forced cases.  The transposed product adds a column's entries in row
+order: with integer values the sums are exact."""
+import math
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.mark.parametrize("n_row,n_col,f_col,rows,nnz", [(1, 1, 0, 1, 1), (5, 9, 0, 5, 0), (40, 30, 100, 33, 200),
+                                                        (3000, 5, 7, 3000, 20000), (7, 70001, 0, 7, 40000),
+                                                        (1025, 1024, 1, 1024, 5000)])
+def test_transposed_copy_of_blocks(gpu, n_row, n_col, f_col, rows, nnz):
+    rng = np.random.default_rng(nnz + n_col)
+    row = np.sort(rng.integers(0, rows, nnz))
+    rp = np.searchsorted(row, np.arange(rows + 1)).astype(np.int32)
+    ci = rng.integers(0, n_col, nnz).astype(np.int32)
+    va = rng.integers(-9, 10, nnz).astype(np.float64)
+    A = gpu.DeviceMatrix.csr(n_row, n_col, rp, ci + f_col, va, f_col=f_col, stores=gpu.STORE_F64 | gpu.STORE_F32,
+                             rows=rows)
+    x = rng.integers(-9, 10, n_row).astype(np.float64)
+    want = np.bincount(ci, va * x[row], n_col) if nnz else np.zeros(n_col)
+    for store, vt, tdt in ((gpu.F64, gpu.F64, torch.float64), (gpu.F32, gpu.F32, torch.float32)):
+        tx = torch.from_numpy(x).cuda().to(tdt)
+        y = torch.full((n_col,), 5.0, dtype=tdt, device="cuda")
+        for _ in range(2):
+            A.spmv_transpose_ex(store, vt, tx.data_ptr(), vt, y.data_ptr())
+            assert np.array_equal(y.double().cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("n,nnz", [(1, 1), (2, 5), (1000, 40000), (4097, 9000)])
+def test_relabelled_copy(gpu, orc, n, nnz):
+    rng = np.random.default_rng(n)
+    row = np.sort((n * rng.random(nnz) ** 3).astype(np.int64))
+    rp = np.searchsorted(row, np.arange(n + 1)).astype(np.int32)
+    ci = (n * rng.random(nnz) ** 2).astype(np.int32)  # repeated columns among them
+    va = 1.0 / np.bincount(ci, minlength=n)[ci]
+    dang = (np.bincount(ci, minlength=n) == 0).astype(np.uint8)
+    A = gpu.DeviceMatrix.csr(n, n, rp, ci, va, stores=gpu.STORE_F64 | gpu.STORE_F32)
+    A.tune(gpu.TUNE_PR_RELABEL, 1)
+    xo, _, _ = orc.page_rank_dangling(rp, ci, va, dang, 0.85, 1e-14, 5000)
+    xo = xo / math.fsum(xo)
+    for prec, accel in ((gpu.F64, 0), (gpu.F64, 1), (gpu.F32, 1)):
+        x, r = A.pagerank_host(beta=0.85, tol=1e-11, max_iter=5000, mode=gpu.PR_DANGLING, precision=prec, accel=accel)
+        # ||x - G(x)||_1 < tol: within tol / (1 - beta) of the fixed point
+        assert r.converged and np.abs(x - xo).sum() <= 1e-11 / 0.15 + 1e-12
