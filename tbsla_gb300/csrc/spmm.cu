@@ -31,28 +31,16 @@ __device__ __forceinline__ void unpack(float v, float (&o)[1]) { o[0] = v; }
 __device__ __forceinline__ void unpack(double2 v, double (&o)[2]) { o[0] = v.x; o[1] = v.y; }
 __device__ __forceinline__ void unpack(float4 v, float (&o)[4]) { o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w; }
 
-// A row's entries are read four at a time, from a multiple of four on, with
-// one 16-byte load of columns and one of values (entries outside the row are
-// masked; the arrays carry 64 spare bytes): read one by one, an entry's index
-// and value cost a warp of several rows as many L1 passes as a narrow panel's
-// gathered X rows (cqmat 2^20 c = 16 FP32, k = 16: 114 us, so 88; k = 7, one
-// vector a lane: 103, so 90; k = 32, where the gathers' bytes bound it: 155, so
-// 152).  Measured worse at k = 32: entries read one lane each and shared by
-// shuffles (315 us), the next four read ahead (170), the ELL-layout copy with
-// eight lanes a row (195 to 460, the more slots in flight the slower), more
-// registers (48: 213).  wide_y: 16-byte stores of Y (its rows and width allow them).
 template <typename V, typename T, int KT, int VW>
-__global__ void __launch_bounds__(256, VW > 1 ? 6 : 8) csr_spmm_kernel(int rows, const int *__restrict__ rowptr,
+__global__ void __launch_bounds__(256) csr_spmm_kernel(int rows, const int *__restrict__ rowptr,
                                                       const int *__restrict__ colidx, const V *__restrict__ values,
                                                       const T *__restrict__ X, int64_t ldx, int f_col,
                                                       T *__restrict__ Y, int64_t ldy, int width, int row_shift,
-                                                      int n_out, bool wide_y) {
+                                                      int n_out) {
   using Acc = typename AccOf<T>::type;
   using Vec = typename VecOf<T, VW>::type;
   const int lane = threadIdx.x & (KT - 1);
   const int c = lane * VW;  // first vector of this lane
-  const char *xb = reinterpret_cast<const char *>(X + c) - (int64_t)f_col * ldx * (int64_t)sizeof(T);
-  const uint64_t ldxb = (uint64_t)ldx * sizeof(T);
   const int64_t ng = ((int64_t)gridDim.x * blockDim.x) / KT;
   for (int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / KT; g < rows; g += ng) {
     const int r = (int)g;
@@ -61,42 +49,19 @@ __global__ void __launch_bounds__(256, VW > 1 ? 6 : 8) csr_spmm_kernel(int rows,
       Acc acc[VW];
       #pragma unroll
       for (int q = 0; q < VW; ++q) acc[q] = 0;
-      for (int e = a & ~3; e < b; e += 4) {
-        const int4 k4 = __ldg(reinterpret_cast<const int4 *>(colidx + e));
-        const Vec4<V> w4 = ld4<V, false>(values + e);
-        const int cj[4] = {k4.x, k4.y, k4.z, k4.w};
-        T xv[4][VW];
-        if (e >= a && e + 4 <= b) {
-          #pragma unroll
-          for (int u = 0; u < 4; ++u) unpack(__ldg(reinterpret_cast<const Vec *>(xb + (uint64_t)(unsigned)cj[u] * ldxb)), xv[u]);
-          #pragma unroll
-          for (int u = 0; u < 4; ++u)
-            #pragma unroll
-            for (int q = 0; q < VW; ++q) acc[q] = fma_acc(to_acc(w4.v[u], Acc()), to_acc(xv[u][q], Acc()), acc[q]);
-        } else {
-          #pragma unroll
-          for (int u = 0; u < 4; ++u)
-            if (e + u >= a && e + u < b) {
-              unpack(__ldg(reinterpret_cast<const Vec *>(xb + (uint64_t)(unsigned)cj[u] * ldxb)), xv[u]);
-              #pragma unroll
-              for (int q = 0; q < VW; ++q) acc[q] = fma_acc(to_acc(w4.v[u], Acc()), to_acc(xv[u][q], Acc()), acc[q]);
-            }
-        }
+      #pragma unroll 4
+      for (int e = a; e < b; ++e) {
+        const Acc v = to_acc(ld_stream(values + e), Acc());
+        T xv[VW];
+        unpack(__ldg(reinterpret_cast<const Vec *>(X + (int64_t)(__ldg(colidx + e) - f_col) * ldx + c)), xv);
+        #pragma unroll
+        for (int q = 0; q < VW; ++q) acc[q] = fma_acc(v, to_acc(xv[q], Acc()), acc[q]);
       }
       const int out = r + row_shift;
       if (out >= 0 && out < n_out) {
-        T *yp = Y + (int64_t)out * ldy + c;
-        if (VW > 1 && wide_y) {
-          Vec o;
-          T *oe = reinterpret_cast<T *>(&o);
-          #pragma unroll
-          for (int q = 0; q < VW; ++q) oe[q] = (T)acc[q];
-          __stcs(reinterpret_cast<Vec *>(yp), o);
-        } else {
-          #pragma unroll
-          for (int q = 0; q < VW; ++q)
-            if (c + q < width) yp[q] = (T)acc[q];
-        }
+        #pragma unroll
+        for (int q = 0; q < VW; ++q)
+          if (c + q < width) Y[(int64_t)out * ldy + c + q] = (T)acc[q];
       }
     }
   }
@@ -183,13 +148,12 @@ tbsla_status_t spmm_panel(const tbsla_matrix *A, const int *rowptr, const V *val
   constexpr int VW16 = 16 / (int)sizeof(T);
   const bool vec = width % VW16 == 0 && (ldx * (int64_t)sizeof(T)) % 16 == 0 &&
                    (reinterpret_cast<uintptr_t>(X) & 15) == 0;
-  const bool wide_y = vec && (ldy * (int64_t)sizeof(T)) % 16 == 0 && (reinterpret_cast<uintptr_t>(Y) & 15) == 0;
   const int lanes = vec ? width / VW16 : width;
   const int kt = lanes <= 1 ? 1 : lanes <= 2 ? 2 : lanes <= 4 ? 4 : lanes <= 8 ? 8 : lanes <= 16 ? 16 : 32;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)rows * kt + 255) / 256, 152 * 64));
 #define TB_SPMM(KT_, VW_)                                                                                          \
   csr_spmm_kernel<V, T, KT_, VW_><<<grid, 256, 0, s>>>(rows, rowptr, A->idx1, vals, X, ldx, A->f_col, Y, ldy, width, \
-                                                      row_shift, A->n_row, wide_y)
+                                                      row_shift, A->n_row)
   if (vec) {
     switch (kt) {
     case 1: TB_SPMM(1, VW16); break;
