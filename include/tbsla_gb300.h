@@ -348,9 +348,10 @@ tbsla_status_t tbsla_coo_spmv_noalloc_status(int *bad, void *stream);
 /* -------------------------------------------------------------- batches */
 /* Many CSR handles multiplied together: y_m = A_m x_m for every member in
  * ONE kernel launch (a persistent grid walking row items of every member
- * with a fixed stride, so sums are deterministic; members that keep the
- * ELL-layout copy, TBSLA_TUNE_SHORT_ROWS 3, are read from it for the F64 and
- * F32 stores).  No reference counterpart (the reference multiplies one
+ * with a fixed stride, so sums are deterministic; members with an
+ * ELL-layout copy, TBSLA_TUNE_SHORT_ROWS 3 or one tbsla_batch_create adds to a
+ * smaller member of short, even rows (its entries' memory again), are read
+ * from it for the F64 and F32 stores).  No reference counterpart (the reference multiplies one
  * matrix per call). */
 typedef struct tbsla_batch tbsla_batch_t;
 /* members: count CSR handles on one device, kept alive by the caller */
@@ -362,7 +363,7 @@ tbsla_status_t tbsla_batch_bind(tbsla_batch_t *B, tbsla_dtype_t store, const voi
  * left as it is); NULL: every member.  For iterative callers that stop
  * members independently. */
 tbsla_status_t tbsla_batch_set_mask(tbsla_batch_t *B, const int *d_mask);
-/* persistent grid of 152 x blocks_per_sm blocks (default 6) */
+/* persistent grid of 152 x blocks_per_sm blocks (default 12) */
 tbsla_status_t tbsla_batch_tune(tbsla_batch_t *B, int blocks_per_sm);
 /* Enqueues the one launch on `stream`: no allocation, no synchronisation. */
 tbsla_status_t tbsla_batch_spmv(tbsla_batch_t *B, void *stream);

@@ -7,10 +7,13 @@
 // sum is fixed and the launch needs no counter to reset: it can be replayed
 // from a CUDA graph as is.  A row is summed by one thread in its stored
 // order (the thread-per-row loads of csr_direct.cuh: the single products'
-// arithmetic with TBSLA_TUNE_SHORT_ROWS = 0).  Members that keep the
-// ELL-layout copy (csr_sell_kernel's arrays) for the bound store are read
-// from it, two rows per thread (items of 2 * kBatchRows rows): the same sums,
-// coalesced loads.  An optional device mask skips members (per-instance
+// arithmetic with TBSLA_TUNE_SHORT_ROWS = 0).  Members with an ELL-layout copy
+// for the bound store (csr_sell_kernel's, or one the batch had built for a
+// member too small to keep that: batch_copy) are read from it, two rows per
+// thread (items of 2 * kBatchRows rows): the same sums, coalesced loads.  64
+// cqmat matrices of 1e3 to 1e5 rows, FP32: 81 us reading the CSR arrays of the
+// members below 2^16 rows (a 16-byte load of 32 rows touches 20 lines or more),
+// 66 with their copies.  An optional device mask skips members (per-instance
 // convergence masking for iterative callers).
 #include <algorithm>
 #include <vector>
@@ -18,6 +21,8 @@
 #include "product.cuh"
 
 namespace tbsla {
+
+tbsla_status_t batch_copy(tbsla_matrix *A);
 
 struct BatchMember {
   const int *rowptr;
@@ -110,7 +115,10 @@ struct tbsla_batch {
   int4 *d_items = nullptr;
   int n_items = 0;
   const int *d_mask = nullptr;       // caller's mask or NULL
-  int blocks_per_sm = 6;             // persistent grid: 152 x blocks_per_sm (tbsla_batch_tune)
+  // persistent grid: 152 x blocks_per_sm (tbsla_batch_tune).  64 cqmat
+  // matrices of up to 1e5 rows, FP32 / FP64: 4: 87 / 111 us, 6: 73 / 94, 12: 66 /
+  // 87, 16: 70 / 91, one block per item: 68 / 88
+  int blocks_per_sm = 12;
   tbsla_dtype_t store = TBSLA_F64;   // value store chosen by tbsla_batch_bind
   bool bound = false;
   cudaGraphExec_t graph = nullptr;   // tbsla_batch_spmv_graph
@@ -150,18 +158,23 @@ tbsla_status_t tbsla_batch_create(int count, const tbsla_matrix_t *const *member
       return fail(TBSLA_ERR_INVALID_ARG, "batch member %d is not a CSR handle on device %d", m, B->device);
     }
     B->members.push_back(A);
+    const tbsla_status_t cs = batch_copy(const_cast<tbsla_matrix *>(A));
+    if (cs != TBSLA_OK) {
+      delete B;
+      return cs;
+    }
     BatchMember d{};
     d.rowptr = A->idx0;
     d.colidx = A->idx1;
     d.f_col = A->f_col;
     d.rows = A->rows;
     d.n_row = A->n_row;
-    d.sell_width = A->sell_width;
-    d.sell_cols = A->sell_cols;
-    d.sell_stride = A->sell_stride;
+    d.sell_width = A->sell_width ? A->sell_width : A->bsell_width;
+    d.sell_cols = A->sell_width ? A->sell_cols : A->bsell_cols;
+    d.sell_stride = A->sell_width ? A->sell_stride : A->bsell_stride;
     B->table.push_back(d);
     // members with the ELL-layout copy: items of two rows per thread
-    const int span = A->sell_width ? 2 * kBatchRows : kBatchRows;
+    const int span = d.sell_width ? 2 * kBatchRows : kBatchRows;
     for (int r = 0; r < A->n_row; r += span) items.push_back(make_int4(m, r, std::min(r + span, A->n_row), 0));
   }
   B->n_items = (int)items.size();
@@ -188,7 +201,7 @@ tbsla_status_t tbsla_batch_bind(tbsla_batch_t *B, tbsla_dtype_t store, const voi
     TB_CHECK(d_y[m] || A->n_row == 0, "y of member %zu is NULL", m);
     TB_CHECK(d_x[m] || A->stored == 0, "x of member %zu is NULL", m);
     B->table[m].values = A->values[si];
-    B->table[m].sell_vals = A->sell_width && si < 2 ? A->sell_vals[si] : nullptr;
+    B->table[m].sell_vals = si >= 2 ? nullptr : A->sell_width ? A->sell_vals[si] : A->bsell_vals[si];
     B->table[m].x = d_x[m];
     B->table[m].y = d_y[m];
   }

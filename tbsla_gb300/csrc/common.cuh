@@ -115,6 +115,12 @@ struct tbsla_matrix {
   void *sell_vals[3] = {nullptr, nullptr, nullptr};
   int64_t sell_stride = 0;  // rows rounded up to a multiple of 128
   int sell_width = 0;       // slots per row (the longest row); 0: no copy
+  // the same copy for members of a batch below the rows where plain products
+  // gain from one (batch.cu builds it; F64 and F32 stores)
+  int *bsell_cols = nullptr;
+  void *bsell_vals[2] = {nullptr, nullptr};
+  int64_t bsell_stride = 0;
+  int bsell_width = 0;
   int sell_rows = 0;        // rows per thread of csr_sell_kernel (1, 2, 4; 0: by size)
   int4 *warp_items = nullptr;
   int n_warp_items = 0;

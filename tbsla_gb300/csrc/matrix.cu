@@ -201,6 +201,57 @@ static tbsla_status_t upload_values(tbsla_matrix *A, const double *host, int64_t
   return TBSLA_OK;
 }
 
+// The values of a batch member's ELL-layout copy from its stores
+static tbsla_status_t batch_copy_refresh(tbsla_matrix *A, cudaStream_t s) {
+  if (!A->bsell_width) return TBSLA_OK;
+  const int grid = grid_for(A->rows, 256);
+  if (A->bsell_vals[0])
+    sell_scatter_kernel<double><<<grid, 256, 0, s>>>(A->idx0, A->bsell_stride, A->rows,
+                                                     static_cast<const double *>(A->values[0]),
+                                                     static_cast<double *>(A->bsell_vals[0]));
+  if (A->bsell_vals[1])
+    sell_scatter_kernel<float><<<grid, 256, 0, s>>>(A->idx0, A->bsell_stride, A->rows,
+                                                    static_cast<const float *>(A->values[1]),
+                                                    static_cast<float *>(A->bsell_vals[1]));
+  TB_CUDA(cudaGetLastError());
+  return TBSLA_OK;
+}
+
+// Builds it for a member of a batch: a CSR handle without the copy of
+// csr_bins, every row short, at least 256 rows of four entries on average, at
+// most 1/32 more slots than entries.  Best effort, as in csr_bins.
+tbsla_status_t batch_copy(tbsla_matrix *A) {
+  if (A->bsell_width || A->sell_width || A->format != TBSLA_FMT_CSR || A->stage_cap == 0 || A->rows < 256 ||
+      !(A->values[0] || A->values[1]))
+    return TBSLA_OK;
+  const int64_t stride = ((int64_t)A->rows + 31) / 32 * 32, total = stride * A->short_max;
+  if (A->stored < 4ll * A->rows || total > A->stored + A->stored / 32) return TBSLA_OK;
+  const size_t esz[3] = {4, 8, 4};
+  void **bufs[3] = {(void **)&A->bsell_cols, &A->bsell_vals[0], &A->bsell_vals[1]};
+  bool ok = true;
+  for (int k = 0; k < 3 && ok; ++k)
+    if (k == 0 || A->values[k - 1]) ok = dev_alloc(A, bufs[k], (size_t)total * esz[k]) == TBSLA_OK;
+  if (!ok) {
+    for (int k = 0; k < 3; ++k)
+      if (*bufs[k]) {
+        cudaFree(*bufs[k]);
+        *bufs[k] = nullptr;
+        A->device_bytes -= total * (int64_t)esz[k] + 64;
+      }
+    g_err.clear();
+    return TBSLA_OK;
+  }
+  TB_CUDA(cudaMemset(A->bsell_cols, 0xff, (size_t)total * sizeof(int)));  // padding: column -1
+  for (int k = 0; k < 2; ++k)
+    if (A->bsell_vals[k]) TB_CUDA(cudaMemset(A->bsell_vals[k], 0, (size_t)total * esz[k + 1]));
+  sell_scatter_kernel<int><<<grid_for(A->rows, 256), 256>>>(A->idx0, stride, A->rows, A->idx1, A->bsell_cols);
+  A->bsell_stride = stride;
+  A->bsell_width = A->short_max;
+  TB_TRY(batch_copy_refresh(A, 0));
+  TB_CUDA(cudaDeviceSynchronize());
+  return TBSLA_OK;
+}
+
 // The sliced copies of A's value stores (csr_sell_kernel) from the stores
 tbsla_status_t sell_refresh(tbsla_matrix *A, cudaStream_t s) {
   if (!A->sell_width) return TBSLA_OK;
@@ -238,7 +289,7 @@ template <typename S> static tbsla_status_t store_new_values(tbsla_matrix *A, co
     store_values_kernel<S><<<grid_for(n, 256), 256, 0, s>>>(src, out, n);
   }
   TB_CUDA(cudaGetLastError());
-  return TBSLA_OK;
+  return batch_copy_refresh(A, s);
 }
 
 // The F32 / BF16 stores of A recomputed from its F64 store (and the sliced
@@ -326,7 +377,7 @@ static void free_handle(tbsla_matrix *A) {
                   A->short_rows, A->warp_items, A->chunk_rows, A->chunk_partials, A->chunk_partials32,
                   A->tile_start, A->tile_head_row, A->tile_head_val,
                   A->tile_tail_val, A->tile_emitted, A->tile_head_val32, A->tile_tail_val32,
-                  A->dangling, A->pr_scratch, A->col_pattern, A->seg_row, A->d_x, A->d_y, A->d_t, A->d_err, A->pr_newid, A->pr_out,
+                  A->dangling, A->pr_scratch, A->col_pattern, A->seg_row, A->bsell_cols, A->bsell_vals[0], A->bsell_vals[1], A->d_x, A->d_y, A->d_t, A->d_err, A->pr_newid, A->pr_out,
                   A->transpose_perm, A->coo_rowptr, A->sell_cols, A->sell_vals[0], A->sell_vals[1],
                   A->sell_vals[2]};
   for (void *p : ptrs) if (p) cudaFree(p);

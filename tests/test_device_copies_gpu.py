@@ -49,3 +49,34 @@ def test_relabelled_copy(gpu, orc, n, nnz):
         x, r = A.pagerank_host(beta=0.85, tol=1e-11, max_iter=5000, mode=gpu.PR_DANGLING, precision=prec, accel=accel)
         # ||x - G(x)||_1 < tol: within tol / (1 - beta) of the fixed point
         assert r.converged and np.abs(x - xo).sum() <= 1e-11 / 0.15 + 1e-12
+
+
+@pytest.mark.parametrize("rows", [255, 256, 257, 511, 513, 4000])
+def test_batch_members_with_a_copy_of_their_own(gpu, rows):
+    """Members around the size from which a batch builds their ELL-layout
+    copy: the one-thread-per-row product's bits, also after new values, and
+    the handle's own products are as before."""
+    rng = np.random.default_rng(rows)
+    n_col, c = rows + 3, 9
+    rp = (np.arange(rows + 1) * c).astype(np.int32)
+    ci = rng.integers(0, n_col, rows * c).astype(np.int32)
+    va = rng.uniform(-1, 1, rows * c)
+    A = gpu.DeviceMatrix.csr(rows + 2, n_col, rp, ci, va, stores=gpu.STORE_F64 | gpu.STORE_F32, rows=rows)
+    A.tune(gpu.TUNE_SHORT_ROWS, 0)
+    held = A.info().device_bytes
+    B = gpu.Batch([A])
+    slots = (rows + 31) // 32 * 32 * c  # rows are padded to a multiple of 32, by at most 1/32 of the entries
+    copied = rows >= 256 and slots <= rows * c + rows * c // 32
+    assert (A.info().device_bytes > held) == copied and A.info().slices == 0
+    for store, tdt in ((gpu.F64, torch.float64), (gpu.F32, torch.float32)):
+        x = torch.rand(n_col, dtype=tdt, device="cuda")
+        y, ref = (torch.full((rows + 2,), 7.0, dtype=tdt, device="cuda") for _ in range(2))
+        B.bind(store, [x.data_ptr()], [y.data_ptr()])
+        for new in (False, True):
+            if new:
+                A.set_values(gpu.F64, torch.from_numpy(rng.uniform(-1, 1, rows * c)).cuda().data_ptr())
+            y.fill_(7.0)
+            B.spmv()
+            A.spmv_ex(store, gpu.F64 if store == gpu.F64 else gpu.F32, x.data_ptr(),
+                      gpu.F64 if store == gpu.F64 else gpu.F32, ref.data_ptr())
+            assert torch.equal(y, ref)
