@@ -264,11 +264,11 @@ tbsla_status_t launch_product(const tbsla_matrix *A, const V *vals, const XT *x,
       // warps per row group: as many as leave each four steps of columns, so
       // that blocks are short and many (8000 x 9001 FP64 in blocks of 35 steps,
       // one wave and a tenth: 281 us, against 175 with few, long blocks)
-      const int64_t groups = ((int64_t)A->rows + kDenseRows - 1) / kDenseRows;
-      const int batch = 32 * (vec ? VW * (VW == 8 ? 2 : 4) : 8);  // columns of a warp's step
+      const int64_t groups = ((int64_t)A->rows + dense_rows<V>() - 1) / dense_rows<V>();
+      const int batch = 32 * (vec ? VW * dense_steps<V, VW>() : dense_steps<V, 1>());  // columns of a warp's step
       int splits = 1;
       while (splits < 8 && A->cols / (2 * splits) >= 4 * batch) splits *= 2;
-      while (splits < 8 && groups * splits < 152 * 16 && A->cols / (2 * splits) >= 128) splits *= 2;
+      while (splits < 8 && groups * splits < 152 * 6 && A->cols / (2 * splits) >= 128) splits *= 2;
       const int grid = (int)((groups * splits + 7) / 8);
       KernelTimer kt(A, s);
       if (vec) dense_kernel<VW, V, XT, Epi><<<grid, 256, 0, s>>>(vals, x, A->rows, A->cols, splits, epi);

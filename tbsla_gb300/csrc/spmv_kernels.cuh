@@ -11,7 +11,7 @@
 // ELL is stored column-major (slot-major) and read with 16-byte vector loads,
 // four rows per thread, each row summed in slot order exactly as
 // MatrixELL::Ax (src/cpp/matrix/MatrixELL.cpp:101-114) orders it.
-// DENSE is a row-major GEMV, two rows per warp.
+// DENSE is a row-major GEMV, two or four rows per warp.
 //
 // The products are written through an epilogue functor `Epi` that receives
 // each finished row once:  epi.emit(row, value).
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(256) ell_warp_kernel(const int *__restrict__ c
 }
 
 // --------------------------------------------------------------- DENSE
-// Row-major GEMV: a warp takes kDenseRows rows, so that every x chunk loaded
+// Row-major GEMV: a warp takes two rows (FP64: four), so that every x chunk loaded
 // serves them all, and `splits` warps of a block share the columns of a row
 // group (few rows would leave the GPU empty); lanes stride over the columns VW
 // at a time: 16-byte loads when the rows start on 16 bytes (VW elements),
@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(256) ell_warp_kernel(const int *__restrict__ c
 // order.  What bounds it is the loads in flight: four rows a warp and one
 // element a lane held 13 warps per SM and ran an FP32 matrix of 8000 x 9001 at
 // 2660 GB/s (108 us).
-constexpr int kDenseRows = 2;
+template <typename V> constexpr int dense_rows() { return sizeof(V) == 8 ? 4 : 2; }
 
 // VW consecutive elements at p, aligned to their size together
 template <int VW> __device__ __forceinline__ void ld_dense(const double *p, double (&v)[VW]) {
@@ -451,12 +451,20 @@ template <int VW, typename XT, typename Acc> __device__ __forceinline__ void ld_
   }
 }
 
+// steps of a warp in flight.  FP64, whose pipe is the bound, takes more rows
+// and fewer steps, which fits more warps: 9000 x 400 in 24.5 us with two rows
+// and two steps, 21.1 with four and two, 17.7 with four and one (as with the
+// few long warps of before), 8000 x 9001 in 153, 146 and 146 (175)
+template <typename V, int VW> constexpr int dense_steps() {
+  return sizeof(V) == 8 ? (VW == 1 ? 2 : 1) : VW == 1 ? 8 : VW == 8 ? 2 : 4;
+}
+
 template <int VW, typename V, typename XT, typename Epi>
 __global__ void __launch_bounds__(256) dense_kernel(const V *__restrict__ a, const XT *__restrict__ x, int rows,
                                                     int cols, int splits, Epi epi) {
   using Acc = typename Epi::Acc;
   using Ld = typename std::conditional<sizeof(V) == 8, double, float>::type;
-  constexpr int R = kDenseRows, U = VW == 1 ? 8 : VW == 8 ? 2 : 4;
+  constexpr int R = dense_rows<V>(), U = dense_steps<V, VW>();
   __shared__ Acc part[8][R][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t r0 = ((int64_t)blockIdx.x * (8 / splits) + warp / splits) * R;
