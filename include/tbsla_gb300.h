@@ -363,7 +363,8 @@ tbsla_status_t tbsla_batch_bind(tbsla_batch_t *B, tbsla_dtype_t store, const voi
  * left as it is); NULL: every member.  For iterative callers that stop
  * members independently. */
 tbsla_status_t tbsla_batch_set_mask(tbsla_batch_t *B, const int *d_mask);
-/* persistent grid of 152 x blocks_per_sm blocks (default 12) */
+/* persistent grid of 152 x blocks_per_sm blocks (default 12, 6 for batches of
+ * few rows) */
 tbsla_status_t tbsla_batch_tune(tbsla_batch_t *B, int blocks_per_sm);
 /* Enqueues the one launch on `stream`: no allocation, no synchronisation. */
 tbsla_status_t tbsla_batch_spmv(tbsla_batch_t *B, void *stream);

@@ -115,10 +115,12 @@ struct tbsla_batch {
   int4 *d_items = nullptr;
   int n_items = 0;
   const int *d_mask = nullptr;       // caller's mask or NULL
-  // persistent grid: 152 x blocks_per_sm (tbsla_batch_tune).  64 cqmat
-  // matrices of up to 1e5 rows, FP32 / FP64: 4: 87 / 111 us, 6: 73 / 94, 12: 66 /
-  // 87, 16: 70 / 91, one block per item: 68 / 88
-  int blocks_per_sm = 12;
+  // persistent grid: 152 x blocks_per_sm (tbsla_batch_tune; 0: 12, or 6 when
+  // there are fewer items than that holds).  64 cqmat matrices of up to 1e5
+  // rows, FP32 / FP64: 4: 87 / 111 us, 6: 73 / 94, 12: 66 / 87, 16: 70 / 91, one
+  // block per item: 68 / 88; 41 of up to 21954 rows (1100 items), BF16: 6 18 us,
+  // 12 20 us
+  int blocks_per_sm = 0;
   tbsla_dtype_t store = TBSLA_F64;   // value store chosen by tbsla_batch_bind
   bool bound = false;
   cudaGraphExec_t graph = nullptr;   // tbsla_batch_spmv_graph
@@ -131,7 +133,8 @@ struct tbsla_batch {
 
 static tbsla_status_t batch_launch(tbsla_batch *B, tbsla_dtype_t store, cudaStream_t s) {
   if (B->n_items == 0) return TBSLA_OK;
-  const int grid = std::max(1, std::min(B->n_items, 152 * B->blocks_per_sm));
+  const int per_sm = B->blocks_per_sm ? B->blocks_per_sm : B->n_items >= 152 * 12 ? 12 : 6;
+  const int grid = std::max(1, std::min(B->n_items, 152 * per_sm));
   if (store == TBSLA_F64)
     batch_spmv_kernel<double, double><<<grid, 256, 0, s>>>(B->d_table, B->d_items, B->n_items, B->d_mask);
   else if (store == TBSLA_F32)
@@ -173,9 +176,15 @@ tbsla_status_t tbsla_batch_create(int count, const tbsla_matrix_t *const *member
     d.sell_cols = A->sell_width ? A->sell_cols : A->bsell_cols;
     d.sell_stride = A->sell_width ? A->sell_stride : A->bsell_stride;
     B->table.push_back(d);
-    // members with the ELL-layout copy: items of two rows per thread
-    const int span = d.sell_width ? 2 * kBatchRows : kBatchRows;
-    for (int r = 0; r < A->n_row; r += span) items.push_back(make_int4(m, r, std::min(r + span, A->n_row), 0));
+  }
+  // members with an ELL-layout copy: items of two rows per thread, one when the
+  // batch would not give every SM a few items
+  int64_t pairs = 0;
+  for (const tbsla_matrix *A : B->members) pairs += (A->n_row + 2 * kBatchRows - 1) / (2 * kBatchRows);
+  for (int m = 0; m < count; ++m) {
+    const int n_row = B->members[(size_t)m]->n_row;
+    const int span = B->table[(size_t)m].sell_width && pairs >= 152 * 4 ? 2 * kBatchRows : kBatchRows;
+    for (int r = 0; r < n_row; r += span) items.push_back(make_int4(m, r, std::min(r + span, n_row), 0));
   }
   B->n_items = (int)items.size();
   cudaSetDevice(B->device);

@@ -80,3 +80,27 @@ def test_batch_members_with_a_copy_of_their_own(gpu, rows):
             A.spmv_ex(store, gpu.F64 if store == gpu.F64 else gpu.F32, x.data_ptr(),
                       gpu.F64 if store == gpu.F64 else gpu.F32, ref.data_ptr())
             assert torch.equal(y, ref)
+
+
+@pytest.mark.parametrize("count", [5, 6, 16])
+def test_batch_items_and_grid_by_row_count(gpu, count):
+    """Both item spans and both default grids: each member's rows carry the
+    bits of its own one-thread-per-row product."""
+    rng = np.random.default_rng(count)
+    rows, c = 60001, 5
+    rp = (np.arange(rows + 1) * c).astype(np.int32)
+    mats, xs, ys = [], [], []
+    for _ in range(count):
+        ci = rng.integers(0, rows, rows * c).astype(np.int32)
+        A = gpu.DeviceMatrix.csr(rows, rows, rp, ci, rng.uniform(-1, 1, rows * c), stores=gpu.STORE_F64, rows=rows)
+        A.tune(gpu.TUNE_SHORT_ROWS, 0)
+        mats.append(A)
+        xs.append(torch.rand(rows, dtype=torch.float64, device="cuda"))
+        ys.append(torch.full((rows,), 7.0, dtype=torch.float64, device="cuda"))
+    B = gpu.Batch(mats)
+    B.bind(gpu.F64, [x.data_ptr() for x in xs], [y.data_ptr() for y in ys])
+    B.spmv()
+    ref = torch.empty(rows, dtype=torch.float64, device="cuda")
+    for A, x, y in zip(mats, xs, ys):
+        A.spmv_ex(gpu.F64, gpu.F64, x.data_ptr(), gpu.F64, ref.data_ptr())
+        assert torch.equal(y, ref)
