@@ -257,7 +257,7 @@ tbsla_status_t tbsla_spmv_host(tbsla_matrix_t *A, const double *x, int64_t nx, d
 
 /* y = A^T x (CSR handles): the gradient of y = A x with respect to x.  x has
  * n_row entries, y n_col entries (indexed col - f_col).  The transpose is
- * built on the first call (host sort of the entries by column, stable) and
+ * built on the first call (stable sort of the entries by column, on the device) and
  * kept with the handle; store / types as tbsla_spmv_ex.  No reference
  * counterpart. */
 tbsla_status_t tbsla_spmv_transpose_ex(const tbsla_matrix_t *A, tbsla_dtype_t store, tbsla_dtype_t x_type,

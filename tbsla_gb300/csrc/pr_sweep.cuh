@@ -7,10 +7,9 @@
 // launch and a refill.  As one launch per row class, finalize, dot and
 // combination (4 to 11 launches a sweep), the reference mode on cqmat 1e5 took
 // 28 us a sweep and the accelerated adjoint on R-MAT 2^16 95 us; here a sweep
-// is one pass over the row items, one grid barrier whose last block reduces
-// the partial sums and advances the control block, and where the mode needs
-// one an elementwise pass (max-normalisation, Anderson combination) with its
-// own barrier.
+// is one pass over the row items, one grid barrier after which every block
+// reduces the partial sums and advances the control block, and where the mode
+// needs one an elementwise pass (Anderson combination) with its own barrier.
 //
 // Work split: one block of 1024 threads per SM (64 registers a thread), so that
 // a barrier has few arrivals and few partial sums.  Rows are cut into classes
@@ -45,7 +44,11 @@ struct PrCtl {
   double beta, tol, inv_n, tele_scale;  // tele_scale: (1-beta)/n or (1-beta)/|P|
   double add;       // term of the next FP64 sweep (reference: tele; dangling: (b d + (1-b) s)/n)
   double add_in;    // term of the next inner sweep
-  double maxv;      // reference mode: max of the unnormalised iterate
+  // reference mode: max of the new iterate; max of the iterate a sweep reads
+  // (1: normalised); what its product is multiplied with; max of it over that of
+  // the one before; the residual before `resid`
+  double maxv, scale, beta_s, rho, resid_prev;
+  int known, pass;  // resid is the read iterate's; the new iterate is normalised in place
   double resid, s;
   double inner_resid, inner_tol;
   double inner_eta; // inner tolerance relative to ||r||
@@ -166,6 +169,15 @@ __device__ __forceinline__ bool pr_barrier(unsigned *bar, unsigned &target) {
 // sh: kPrShared doubles of shared memory.
 constexpr int kPrShared = 3 * kPrThreads + 3 * 256;
 
+// The maximum is taken by the order of the bits: fmax is several instructions of
+// the FP64 pipe (reference mode on cqmat 1e5: this step 3.6 us, its reduction
+// over the blocks 1.9 us; by bits 2.1 and 1.1).  Neither argument is a NaN.
+__device__ __forceinline__ long long pr_key(double v) {
+  const long long b = __double_as_longlong(v);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+__device__ __forceinline__ double pr_max(double a, double b) { return pr_key(a) < pr_key(b) ? b : a; }
+
 template <int NV>
 __device__ __forceinline__ void pr_block_partials(const double (&v)[NV], bool take_max, double *sh, double *partials,
                                                   int stride, int slot) {
@@ -183,8 +195,8 @@ __device__ __forceinline__ void pr_block_partials(const double (&v)[NV], bool ta
       const int j = warp >> 3;
       const bool mx = take_max && h + j == 0;
       const double *p = sh + j * kPrThreads + (warp & 7) * 128 + lane;
-      const double a = mx ? fmax(p[0], p[32]) : p[0] + p[32], b = mx ? fmax(p[64], p[96]) : p[64] + p[96];
-      half[j * 256 + (warp & 7) * 32 + lane] = mx ? fmax(a, b) : a + b;
+      const double a = mx ? pr_max(p[0], p[32]) : p[0] + p[32], b = mx ? pr_max(p[64], p[96]) : p[64] + p[96];
+      half[j * 256 + (warp & 7) * 32 + lane] = mx ? pr_max(a, b) : a + b;
     }
     __syncthreads();
     if (warp < min(M, NV - h)) {
@@ -193,19 +205,19 @@ __device__ __forceinline__ void pr_block_partials(const double (&v)[NV], bool ta
       #pragma unroll
       for (int u = 1; u < 8; ++u) {
         const double b = half[warp * 256 + lane + 32 * u];
-        a = mx ? fmax(a, b) : a + b;
+        a = mx ? pr_max(a, b) : a + b;
       }
       #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         const double b = __shfl_down_sync(0xffffffffu, a, o);
-        a = mx ? fmax(a, b) : a + b;
+        a = mx ? pr_max(a, b) : a + b;
       }
       if (lane == 0) __stcg(partials + (size_t)(h + warp) * stride + slot, a);
     }
   }
 }
 
-// the partials [0, nparts) of every value, in a fixed order; valid in thread 0
+// the partials [0, nparts) of every value, in a fixed order; valid in warp 0
 template <int NV>
 __device__ __forceinline__ void pr_reduce_partials(const double *partials, int stride, int nparts, bool take_max,
                                                    double (&v)[NV]) {
@@ -220,17 +232,17 @@ __device__ __forceinline__ void pr_reduce_partials(const double *partials, int s
       #pragma unroll
       for (int u = 0; u < 8; ++u) b[u] = k + 32 * u < nparts ? __ldcg(p + k + 32 * u) : mx ? -INFINITY : 0.0;
       #pragma unroll
-      for (int u = 0; u < 8; ++u) a = mx ? fmax(a, b[u]) : a + b[u];
+      for (int u = 0; u < 8; ++u) a = mx ? pr_max(a, b[u]) : a + b[u];
     }
     #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const double b = __shfl_down_sync(0xffffffffu, a, o);
-      a = mx ? fmax(a, b) : a + b;
+      a = mx ? pr_max(a, b) : a + b;
     }
     if (lane == 0) sh[warp] = a;
   }
   __syncthreads();
-  if (threadIdx.x == 0)
+  if (warp == 0)
     #pragma unroll
     for (int j = 0; j < NV; ++j) v[j] = sh[j];
 }
@@ -250,18 +262,61 @@ __device__ __forceinline__ double pr_anderson(PrCtl::Aa &st, int k, double term,
   return add;
 }
 
+// Reference mode, after sweep k: b = u / max(u) is left undone.  The update is
+// linear in b up to its teleport term, itself a multiple of sum(b), so a sweep
+// reads the unnormalised u_k, scales its product and term by the power of two
+// that brings max(u_k) to [1, 2) (exact, where the division rounded every
+// entry), and finds on the way what the sweep before it changed, u_k / max(u_k)
+// - u_{k-1} / max(u_{k-1}): a sweep is one pass and one barrier.  With a pass
+// of its own that divides (4.4 of 17 us a sweep on cqmat 1e5, and a barrier)
+// 112 sweeps took 1888 us, now 1390 to 1440.  The convergence test comes one sweep
+// late, and that sweep is lost when it says stop; so the pass that divides and
+// tests at once runs where the test may hold (the last sweep allowed; the first
+// two; the residual, should it go on falling as it did, below 1.25 tol), where
+// the walk is not this kernel's (a lost sweep is a whole product), and where the
+// maximum is no ordinary number.  Runs in a warp, the two divisions in two
+// lanes (each is a chain of some twenty FP64 instructions; five of them in
+// one thread: 2.1 us a sweep).
+__device__ __forceinline__ void pr_ref_advance(PrCtl &c, int k, bool product, double mx, double sum, double change) {
+  const int lane = threadIdx.x & 31;
+  const double q = lane ? change / fabs(c.scale) : mx / c.scale;
+  const double resid = __shfl_sync(0xffffffffu, q, 1);
+  if (lane) return;
+  c.maxv = mx;
+  if (!c.known) {
+    c.resid_prev = c.resid;
+    c.resid = resid;
+    if (c.resid < c.tol) {  // iterate k is the result; the new one is dropped
+      c.converged = c.done = 1;
+      return;
+    }
+  }
+  c.iter = k + 1;
+  c.f64_sweeps += 1;
+  c.pass = product || k < 2 || c.iter >= c.max_iter || !(fabs(mx) > 1e-30 && fabs(mx) < 1e30) ||
+           c.resid * (c.resid < c.resid_prev ? c.resid : c.resid_prev) < 1.25 * c.tol * c.resid_prev;
+  if (!c.pass) {
+    c.known = 0;
+    c.scale = mx;
+    c.rho = q;
+    const double p = __longlong_as_double((2046ll << 52) - (__double_as_longlong(fabs(mx)) & (2047ll << 52)));
+    c.beta_s = c.beta * p;
+    c.add = c.tele_scale * (sum * p);
+  }
+}
+
 // ------------------------------------------------------------ epilogue
 // A finished row: new value, and the thread's sums, in FP64 (the FP32 inner
 // sweeps' change, which only stops the inner solve, in FP32; their mass and
 // sum in pairs of FP32 numbers, six FP32 operations instead of a conversion
-// and an FP64 addition): the maximum
+// and an FP64 addition): the maximum, the sum and the last sweep's change
 // (reference); the change, the dangling mass (adjoint: v . lambda) and, where
 // the next term needs it, the sum; accelerated, then the residual's dots with
 // the last three residuals.
 template <int MODE, typename T, bool AA> struct PrEmit {
   using Acc = T;
   static constexpr bool kSum = MODE == kSweepDang || MODE == kSweepInner;  // the sum is needed
-  static constexpr int kBase = MODE == kSweepRef ? 1 : kSum ? 3 : 2;
+  static constexpr int kBase = kSum || MODE == kSweepRef ? 3 : 2;
   static constexpr int NV = kBase + (AA ? 3 : 0);
   T *y;
   const T *xold;
@@ -270,8 +325,8 @@ template <int MODE, typename T, bool AA> struct PrEmit {
   const unsigned char *dmask, *tmask;
   const double *tvec, *w;
   const float *rvec;
-  double beta, add, inv_n;
-  int hist;  // accelerated: residuals stored before this sweep
+  double beta, add, inv_n, rho;
+  int hist;  // accelerated: residuals stored before this sweep; reference: the last change is wanted
   T s0, s1, s2;
   double d0, d1, d2;
   float e1, e2;  // inner: the rounding errors of s1 and s2 (Knuth's two-sum)
@@ -301,10 +356,14 @@ template <int MODE, typename T, bool AA> struct PrEmit {
       // lambda' = beta A^T lambda + w + dangling * (beta v . lambda)
       val = __fma_rn(beta, v, w[row] + (dmask[row] ? add : 0.0));
     }
-    __stcg(y + row, val);
     if constexpr (MODE == kSweepRef) {
-      s0 = fmax(s0, val);
-    } else {
+      // the change the last sweep made, up to its scale
+      if (hist) s2 += fabs(fma(-rho, __ldcg(y + row), __ldcg(xold + row)));
+      s0 = val > s0 ? val : s0;
+      s1 += val;
+    }
+    __stcg(y + row, val);
+    if constexpr (MODE != kSweepRef) {
       const T r = val - __ldcg(xold + row);
       s0 += MODE == kSweepInner ? (T)fabsf((float)r) : (T)fabs((double)r);
       if constexpr (MODE == kSweepAdj) {
@@ -573,15 +632,15 @@ __global__ void __launch_bounds__(kPrThreads, 1) pr_solve_kernel(const PrMat<V, 
   unsigned target = 0, phase = 0;
   const int st = a.part_stride;
   auto buffer = [&]() { return a.partials + (size_t)(phase & 1) * 6 * st; };
-  // the end of a phase: the blocks meet, and thread 0 advances the control
-  // block from the reduced sums
-  auto meet = [&](auto values, int nparts, bool take_max, auto advance) {
+  // the end of a phase: the blocks meet, and the first `lanes` threads advance
+  // the control block from the reduced sums
+  auto meet = [&](auto values, int nparts, bool take_max, auto advance, int lanes = 1) {
     constexpr int N = sizeof(values) / sizeof(double);
     if (!pr_barrier(a.bar, target)) return false;
     double u[N];
     pr_reduce_partials<N>(buffer(), st, nparts, take_max, u);
     ++phase;
-    if (threadIdx.x == 0) advance(u);
+    if (threadIdx.x < lanes) advance(u);
     __syncthreads();
     return true;
   };
@@ -591,7 +650,12 @@ __global__ void __launch_bounds__(kPrThreads, 1) pr_solve_kernel(const PrMat<V, 
   if (!kInner && a.init) {
     // first iterate: reference 1 (0.25 with nodes), dangling 1/n, teleport v,
     // adjoint w; its mass gives the first sweep's term
-    if (threadIdx.x == 0) c = a.ctl0;
+    if (threadIdx.x == 0) {
+      c = a.ctl0;
+      c.scale = 1.0;
+      c.beta_s = c.beta;
+      c.known = 1;
+    }
     double v[2] = {0, 0};  // dangling mass (adjoint: v . w), sum
     for (int i = t0; i < n; i += nt) {
       double x0;
@@ -638,16 +702,17 @@ __global__ void __launch_bounds__(kPrThreads, 1) pr_solve_kernel(const PrMat<V, 
     e.tvec = a.tvec;
     e.w = a.w;
     e.rvec = a.rvec;
-    e.beta = c.beta;
+    e.beta = MODE == kSweepRef ? c.beta_s : c.beta;
+    e.rho = c.rho;
     e.add = kInner ? c.add_in : c.add;
     e.inv_n = c.inv_n;
-    e.hist = k;
+    e.hist = MODE == kSweepRef ? !c.known : k;
     T *const yk = e.y;
     pr_sweep<MODE, V, T, AA>(m, x, e, sh, buffer(), st);
     const int nparts = nb + (m.layout == kPrItems ? m.plan.n_chunked : 0);
     if (!meet(VN{}, nparts, MODE == kSweepRef, [&](const double (&v)[NV]) {
           if constexpr (MODE == kSweepRef) {
-            c.maxv = v[0];
+            pr_ref_advance(c, k, m.layout == kPrProduct, v[0], v[1], v[2]);
           } else if constexpr (kInner) {
             const double term = (c.beta * v[1] + (1.0 - c.beta) * v[2]) * c.inv_n;
             c.inner_resid = v[0];
@@ -668,28 +733,33 @@ __global__ void __launch_bounds__(kPrThreads, 1) pr_solve_kernel(const PrMat<V, 
             if constexpr (AA) c.add = pr_anderson(c.aa, k, term, v[NB], v[NB + 1], v[NB + 2]);
             else c.add = term;
           }
-        }))
+        }, MODE == kSweepRef ? 32 : 1))
       return;
     if constexpr (MODE == kSweepRef) {
-      // b /= max; sums of |b - b_prev| and of b
-      double v[2] = {0, 0};
-      const double mx = c.maxv;
-      for (int i = t0; i < n; i += nt) {
-        const double q = __ldcg(yk + i) / mx;
-        __stcg(yk + i, (T)q);
-        v[0] += fabs(q - (double)__ldcg(x + i));
-        v[1] += q;
+      if (c.done) break;
+      if (c.pass) {
+        // b /= max; sums of |b - b_prev| and of b
+        double v[2] = {0, 0};
+        const double mx = c.maxv, sc = c.scale;
+        for (int i = t0; i < n; i += nt) {
+          const double q = __ldcg(yk + i) / mx, p = __ldcg(x + i);
+          __stcg(yk + i, (T)q);
+          v[0] += fabs(q - (sc == 1.0 ? p : p / sc));
+          v[1] += q;
+        }
+        pr_block_partials<2>(v, false, sh, buffer(), st, b);
+        if (!meet(V2{}, nb, false, [&](const double (&u)[2]) {
+              c.resid_prev = c.resid;
+              c.resid = u[0];
+              c.known = 1;
+              c.scale = 1.0;
+              c.beta_s = c.beta;
+              c.add = c.tele_scale * u[1];
+              c.converged = u[0] < c.tol;
+              c.done = c.converged || c.iter >= c.max_iter;
+            }))
+          return;
       }
-      pr_block_partials<2>(v, false, sh, buffer(), st, b);
-      if (!meet(V2{}, nb, false, [&](const double (&u)[2]) {
-            c.resid = u[0];
-            c.iter = k + 1;
-            c.f64_sweeps += 1;
-            c.add = c.tele_scale * u[1];
-            c.converged = u[0] < c.tol;
-            c.done = c.converged || c.iter >= c.max_iter;
-          }))
-        return;
     }
     if constexpr (AA) {
       if (!(kInner ? c.inner_done : c.done)) {

@@ -88,3 +88,29 @@ def test_ell_layout_and_new_values(gpu, orc, fmt):
         t = torch.from_numpy(va2.ravel()).cuda()
         A.set_values(gpu.F64, t.data_ptr())
         check(va2)
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e40, 1e-40])
+def test_reference_mode_stops_where_the_oracle_does(gpu, orc, scale):
+    """The reference mode's normalisation is left to the next sweep, which also
+    tests the convergence: every stopping rule (tolerances from one sweep on,
+    every small iteration limit) gives the oracle's iteration count, and so do
+    maxima far from 1.  With values scaled by 1e40 the teleport term vanishes:
+    a sweep then keeps at least 0.8 of the mass (columns without entries), so
+    errors grow by less than 0.8^-6 < 4 over six sweeps."""
+    n = 3001
+    rng = np.random.default_rng(8)
+    rp, ci, va, _ = graph(rng, n, [40, 300])
+    A, o = gpu.DeviceMatrix.csr(n, n, rp, ci, va * scale), orc.from_arrays("CSR", n, n, va * scale, rp, ci)
+    for limit in (1, 2, 3, 4, 6):
+        b, r = A.pagerank_host(beta=0.85, tol=0.0, max_iter=limit, mode=gpu.PR_REFERENCE)
+        bo, it = o.page_rank(0.0, 0.85, limit)
+        assert r.iterations == it == limit
+        assert np.abs(b - bo).sum() <= 4 * 2 * 6 * (300 + n) * 2.0 ** -53
+    if scale == 1e40:
+        return
+    for tol in (1e4, 300.0, 30.0, 3.0, 0.3, 1e-2, 1e-4, 1e-6):
+        b, r = A.pagerank_host(beta=0.85, tol=tol, max_iter=500, mode=gpu.PR_REFERENCE)
+        bo, it = o.page_rank(tol, 0.85, 500)
+        assert r.iterations == it and r.converged, tol
+        assert np.abs(b - bo).sum() <= 2 * it * (300 + n) * 2.0 ** -53
