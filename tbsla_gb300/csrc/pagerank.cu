@@ -272,6 +272,8 @@ int sweep_limit(const tbsla_matrix *A) {
   return (int)std::max(16.0, std::min(1e6, 2e11 / work));
 }
 
+constexpr int kRefProductRows = 1 << 22;
+
 template <int MODE, typename V, typename T, bool AA>
 tbsla_status_t launch_solver(const tbsla_matrix *A, const PrMat<V, T> &m, PrArgs<T> &a, const PrWork *W,
                              cudaStream_t s) {
@@ -439,9 +441,20 @@ tbsla_status_t run_f64(tbsla_matrix *A, PrWork *W, PrArgs<double> &a, int check_
       a.r[i] = W->ar[i];
     }
   }
-  if (!walks_items(A) && !walks_slots(A) && !W->prod) TB_TRY(pr_alloc((void **)&W->prod, (size_t)W->n * 8));
+  bool walked = walks_items(A) || walks_slots(A);
+  // The reference mode never runs on the relabelled copy: on large graphs in
+  // their own labels the gathers go to DRAM, and the plain product, with twice
+  // the warps per SM, is faster by more than its launch and the step cost.  R-MAT
+  // of 2^20 / 2^21 / 2^22 / 2^23 / 2^24 vertices, 16 sweeps: walked 1.8 / 4.0 /
+  // 9.0 / 22.2 / 48.0 ms, by products 2.2 / 4.1 / 7.7 / 15.4 / 29.8; the ELL layout
+  // (even rows) is better walked at every size (2^24 rows, 205 sweeps: 118, 130 ms)
+  if (MODE == kSweepRef && A->n_row >= kRefProductRows && !walks_slots(A) &&
+      !(A->sell_width && A->values[0] && (A->short_mode == -1 || A->short_mode == 3)))
+    walked = false;
+  if (!walked && !W->prod) TB_TRY(pr_alloc((void **)&W->prod, (size_t)W->n * 8));
   PrMat<double, double> m;
   TB_TRY((solver_matrix<double, double>(A, static_cast<const double *>(A->values[0]), W->prod, &m)));
+  if (!walked) m.layout = kPrProduct;
   TB_TRY(pr_partials(W, m.layout == kPrItems ? m.plan.n_chunked : 0));
   a.x[0] = W->x[0];
   a.x[1] = W->x[1];

@@ -272,12 +272,11 @@ __device__ __forceinline__ double pr_anderson(PrCtl::Aa &st, int k, double term,
 // 112 sweeps took 1888 us, now 1390 to 1440.  The convergence test comes one sweep
 // late, and that sweep is lost when it says stop; so the pass that divides and
 // tests at once runs where the test may hold (the last sweep allowed; the first
-// two; the residual, should it go on falling as it did, below 1.25 tol), where
-// the walk is not this kernel's (a lost sweep is a whole product), and where the
-// maximum is no ordinary number.  Runs in a warp, the two divisions in two
+// two; the residual, should it go on falling as it did, below 1.25 tol), and
+// where the maximum is no ordinary number.  Runs in a warp, the two divisions in two
 // lanes (each is a chain of some twenty FP64 instructions; five of them in
 // one thread: 2.1 us a sweep).
-__device__ __forceinline__ void pr_ref_advance(PrCtl &c, int k, bool product, double mx, double sum, double change) {
+__device__ __forceinline__ void pr_ref_advance(PrCtl &c, int k, double mx, double sum, double change) {
   const int lane = threadIdx.x & 31;
   const double q = lane ? change / fabs(c.scale) : mx / c.scale;
   const double resid = __shfl_sync(0xffffffffu, q, 1);
@@ -293,7 +292,7 @@ __device__ __forceinline__ void pr_ref_advance(PrCtl &c, int k, bool product, do
   }
   c.iter = k + 1;
   c.f64_sweeps += 1;
-  c.pass = product || k < 2 || c.iter >= c.max_iter || !(fabs(mx) > 1e-30 && fabs(mx) < 1e30) ||
+  c.pass = k < 2 || c.iter >= c.max_iter || !(fabs(mx) > 1e-30 && fabs(mx) < 1e30) ||
            c.resid * (c.resid < c.resid_prev ? c.resid : c.resid_prev) < 1.25 * c.tol * c.resid_prev;
   if (!c.pass) {
     c.known = 0;
@@ -712,7 +711,7 @@ __global__ void __launch_bounds__(kPrThreads, 1) pr_solve_kernel(const PrMat<V, 
     const int nparts = nb + (m.layout == kPrItems ? m.plan.n_chunked : 0);
     if (!meet(VN{}, nparts, MODE == kSweepRef, [&](const double (&v)[NV]) {
           if constexpr (MODE == kSweepRef) {
-            pr_ref_advance(c, k, m.layout == kPrProduct, v[0], v[1], v[2]);
+            pr_ref_advance(c, k, v[0], v[1], v[2]);
           } else if constexpr (kInner) {
             const double term = (c.beta * v[1] + (1.0 - c.beta) * v[2]) * c.inv_n;
             c.inner_resid = v[0];

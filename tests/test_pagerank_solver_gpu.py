@@ -114,3 +114,18 @@ def test_reference_mode_stops_where_the_oracle_does(gpu, orc, scale):
         bo, it = o.page_rank(tol, 0.85, 500)
         assert r.iterations == it and r.converged, tol
         assert np.abs(b - bo).sum() <= 2 * it * (300 + n) * 2.0 ** -53
+
+
+def test_reference_mode_by_products(gpu, orc):
+    """2^22 rows of ragged lengths: a product per sweep and a step of the solver,
+    against the oracle after six sweeps (the bound of the other tests)."""
+    n = 1 << 22
+    rng = np.random.default_rng(22)
+    rp, ci, va, _ = graph(rng, n, [40])
+    A, o = gpu.DeviceMatrix.csr(n, n, rp, ci, va), orc.from_arrays("CSR", n, n, va, rp, ci)
+    assert A.info().slices == 0
+    for _ in range(2):
+        b, r = A.pagerank_host(beta=0.85, tol=0.0, max_iter=6, mode=gpu.PR_REFERENCE)
+    bo, it = o.page_rank(0.0, 0.85, 6)
+    assert r.iterations == it == 6
+    assert np.abs(b - bo).sum() <= 4 * 2 * 6 * (40 + n) * 2.0 ** -53
