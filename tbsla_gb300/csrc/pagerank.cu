@@ -412,14 +412,17 @@ tbsla_status_t pr_wait(PrWork *W) {
   return TBSLA_OK;
 }
 
-// order after work the caller queued on its stream
+// The solve's stream waits for the work queued on the caller's stream (NULL: the
+// legacy stream, with which a non-blocking stream has no order of its own):
+// teleport vectors and incoming gradients may still be written there, and the
+// result's buffer still read.
 tbsla_status_t pr_order(PrWork *W, cudaStream_t user) {
-  if (!user) return TBSLA_OK;
   cudaEvent_t ev;
   TB_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-  cudaEventRecord(ev, user);
-  cudaStreamWaitEvent(W->stream, ev, 0);
+  cudaError_t e = cudaEventRecord(ev, user);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(W->stream, ev, 0);
   cudaEventDestroy(ev);
+  TB_CUDA(e);
   return TBSLA_OK;
 }
 
