@@ -272,6 +272,15 @@ int sweep_limit(const tbsla_matrix *A) {
   return (int)std::max(16.0, std::min(1e6, 2e11 / work));
 }
 
+// Polls of a grid barrier before a block gives up: more than a second's worth,
+// and more than the longest wait in the order of things, for a lane that walks
+// an ELL row (up to half a microsecond a slot where the row is nearly alone on
+// its SM, at least a tenth a poll)
+template <typename V, typename T> unsigned barrier_polls(const PrMat<V, T> &m) {
+  const int64_t slots = m.layout == kPrSlots ? m.ewidth : 0;
+  return (unsigned)std::min<int64_t>((1 << 22) + 16 * slots, 1u << 31);
+}
+
 constexpr int kRefProductRows = 1 << 22;
 
 template <int MODE, typename V, typename T, bool AA>
@@ -293,6 +302,7 @@ tbsla_status_t launch_solver(const tbsla_matrix *A, const PrMat<V, T> &m, PrArgs
   a.n = W->n;
   a.ctl = W->ctl;
   a.bar = W->bar;
+  a.polls = barrier_polls(m);
   TB_CHECK(grid + (m.layout == kPrItems ? m.plan.n_chunked : 0) <= W->part_stride, "PageRank partials too small");
   void *args[] = {const_cast<PrMat<V, T> *>(&m), &a};
   TB_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(pr_solve_kernel<MODE, V, T, AA>), dim3(grid),

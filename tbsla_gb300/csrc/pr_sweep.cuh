@@ -125,16 +125,18 @@ template <typename T> struct PrArgs {
   PrCtl *ctl;
   PrCtl ctl0;
   unsigned *bar;          // grid barrier: [0] arrivals of this launch, [kPrLeft] blocks that left, [kPrGaveUp]
+  unsigned polls;         // of a barrier before a block gives up
 };
 
 // ------------------------------------------------------------ barrier
 // All blocks of the (cooperative) grid meet: `target` is the arrival count
-// that completes this barrier.  The wait is bounded: after two seconds of the
-// global timer the block raises bar[kPrGaveUp] and the kernel returns.
-constexpr unsigned long long kPrWaitNs = 2000000000ull;
+// that completes this barrier.  The wait is bounded by a number of polls (reads of
+// L2, some tenths of a microsecond each), not by a clock: time while the context
+// is off the GPU, which other contexts may share, is not counted.  A block
+// that gives up raises bar[kPrGaveUp] and the kernel returns.
 constexpr int kPrLeft = 32, kPrGaveUp = 48, kPrBarWords = 64;  // words of the barrier, in lines of their own
 
-__device__ __forceinline__ bool pr_barrier(unsigned *bar, unsigned &target) {
+__device__ __forceinline__ bool pr_barrier(unsigned *bar, unsigned &target, unsigned polls) {
   __shared__ int lost;
   target += gridDim.x;
   __syncthreads();
@@ -142,20 +144,12 @@ __device__ __forceinline__ bool pr_barrier(unsigned *bar, unsigned &target) {
     lost = 0;
     __threadfence();
     atomicAdd(bar, 1u);
-    unsigned long long t0 = 0;
-    for (int spin = 1; (int)(*(volatile unsigned *)bar - target) < 0; ++spin) {
-      if ((spin & 255) == 0) {
-        unsigned long long t;
-        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-        if (t0 == 0) {
-          t0 = t;
-        } else if (t - t0 > kPrWaitNs) {
-          atomicExch(bar + kPrGaveUp, 1u);
-          lost = 1;
-          break;
-        }
+    for (unsigned k = 0; (int)(*(volatile unsigned *)bar - target) < 0; ++k)
+      if (k >= polls) {
+        atomicExch(bar + kPrGaveUp, 1u);
+        lost = 1;
+        break;
       }
-    }
     __threadfence();
   }
   __syncthreads();
@@ -635,7 +629,7 @@ __global__ void __launch_bounds__(kPrThreads, 1) pr_solve_kernel(const PrMat<V, 
   // the control block from the reduced sums
   auto meet = [&](auto values, int nparts, bool take_max, auto advance, int lanes = 1) {
     constexpr int N = sizeof(values) / sizeof(double);
-    if (!pr_barrier(a.bar, target)) return false;
+    if (!pr_barrier(a.bar, target, a.polls)) return false;
     double u[N];
     pr_reduce_partials<N>(buffer(), st, nparts, take_max, u);
     ++phase;
@@ -772,7 +766,7 @@ __global__ void __launch_bounds__(kPrThreads, 1) pr_solve_kernel(const PrMat<V, 
           if (mm >= 2) q = fma(c2, __ldcg(a.g[s2] + i), q);
           __stcg(a.x[0] + i, q);
         }
-        if (!pr_barrier(a.bar, target)) return;
+        if (!pr_barrier(a.bar, target, a.polls)) return;
       }
     }
   }
