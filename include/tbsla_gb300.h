@@ -216,7 +216,12 @@ tbsla_status_t tbsla_matrix_set_variant(tbsla_matrix_t *A, int variant);
  *   TBSLA_TUNE_TC_SPLIT   DENSE tensor-core product (tbsla_dense_spmm, F32 /
  *                         BF16 stores): the number of parts K is split into,
  *                         1, 2, 4, 8 or 16, or 0 (default) to choose per call
- *                         from the shape and the SM count. */
+ *                         from the shape and the SM count.
+ *   TBSLA_TUNE_SOLVER_POLLS  how often a block of the PageRank solver polls a
+ *                         grid barrier before the solve ends with
+ *                         TBSLA_ERR_TIMEOUT (the handle stays usable); 0
+ *                         (default): some seconds' worth, more for ELL
+ *                         matrices of very long rows. */
 typedef enum {
   TBSLA_TUNE_X_L2_KEEP = 0,
   TBSLA_TUNE_PR_RELABEL = 1,
@@ -224,7 +229,8 @@ typedef enum {
   TBSLA_TUNE_SHORT_ROWS = 3,
   TBSLA_TUNE_TC_SPLIT = 4,
   TBSLA_TUNE_SELL_ROWS = 5,
-  TBSLA_TUNE_DROP_SLICED_COPY = 6
+  TBSLA_TUNE_DROP_SLICED_COPY = 6,
+  TBSLA_TUNE_SOLVER_POLLS = 7
 } tbsla_tune_knob_t;
 tbsla_status_t tbsla_matrix_tune(tbsla_matrix_t *A, int knob, double value);
 tbsla_status_t tbsla_matrix_info(const tbsla_matrix_t *A, tbsla_matrix_info_t *info);

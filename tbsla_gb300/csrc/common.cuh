@@ -153,6 +153,7 @@ struct tbsla_matrix {
   // PageRank workspace built on first use (pagerank.cu)
   void *pr_work = nullptr;
   void (*pr_work_free)(void *) = nullptr;
+  unsigned pr_polls = 0;             // polls of a solver barrier (tbsla_matrix_tune; 0: the default)
   bool pr_dmask_stale = false;       // the values changed since pr_work's dangling mask
   unsigned char *col_pattern = nullptr;  // columns without a stored entry (column_mask.cuh)
   // row classes of the PageRank solver (pagerank.cu; the row structure only)

@@ -1003,6 +1003,13 @@ tbsla_status_t tbsla_matrix_tune(tbsla_matrix_t *A, int knob, double value) {
       A->sell_stride = 0;
     }
     return TBSLA_OK;
+  case TBSLA_TUNE_SOLVER_POLLS:
+    TB_CHECK(value >= 0.0 && value <= 2147483648.0 && value == (double)(unsigned)value,
+             "solver polls %g not a whole number in [0, 2^31]", value);
+    A->pr_polls = (unsigned)value;
+    if (A->pr_relabel) A->pr_relabel->pr_polls = (unsigned)value;
+    if (A->transpose) A->transpose->pr_polls = (unsigned)value;
+    return TBSLA_OK;
   case TBSLA_TUNE_X_L2_RANGE:
     TB_CHECK(value == 0.0 || value == 1.0, "x L2 range mode %g not 0 or 1", value);
     A->x_keep_range = (int)value;

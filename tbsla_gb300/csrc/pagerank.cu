@@ -276,7 +276,8 @@ int sweep_limit(const tbsla_matrix *A) {
 // and more than the longest wait in the order of things, for a lane that walks
 // an ELL row (up to half a microsecond a slot where the row is nearly alone on
 // its SM, at least a tenth a poll)
-template <typename V, typename T> unsigned barrier_polls(const PrMat<V, T> &m) {
+template <typename V, typename T> unsigned barrier_polls(const tbsla_matrix *A, const PrMat<V, T> &m) {
+  if (A->pr_polls) return A->pr_polls;
   const int64_t slots = m.layout == kPrSlots ? m.ewidth : 0;
   return (unsigned)std::min<int64_t>((1 << 22) + 16 * slots, 1u << 31);
 }
@@ -302,7 +303,7 @@ tbsla_status_t launch_solver(const tbsla_matrix *A, const PrMat<V, T> &m, PrArgs
   a.n = W->n;
   a.ctl = W->ctl;
   a.bar = W->bar;
-  a.polls = barrier_polls(m);
+  a.polls = barrier_polls(A, m);
   TB_CHECK(grid + (m.layout == kPrItems ? m.plan.n_chunked : 0) <= W->part_stride, "PageRank partials too small");
   void *args[] = {const_cast<PrMat<V, T> *>(&m), &a};
   TB_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(pr_solve_kernel<MODE, V, T, AA>), dim3(grid),
@@ -408,16 +409,23 @@ tbsla_status_t pr_aa_buffers(PrWork *W) {
   return TBSLA_OK;
 }
 
-// Waits for the solve's stream; an abandoned barrier is reset and reported.
-tbsla_status_t pr_wait(PrWork *W) {
+// Waits for the solve's stream.  A barrier that was given up leaves the blocks
+// in different sweeps: the barrier and the chunk counts of the swept matrix's
+// plan (blocks that went on have counted chunks the others never did) are reset
+// for the next solve, and the error is returned.
+tbsla_status_t pr_wait(const tbsla_matrix *A, PrWork *W) {
   TB_CUDA(cudaGetLastError());
   TB_CUDA(cudaMemcpyAsync(W->ctl_host, W->ctl, kCtlBytes + kBarBytes, cudaMemcpyDeviceToHost, W->stream));
   TB_CUDA(cudaStreamSynchronize(W->stream));
   const unsigned *bar = reinterpret_cast<const unsigned *>(reinterpret_cast<const char *>(W->ctl_host) + kCtlBytes);
   if (bar[kPrGaveUp]) {
     TB_CUDA(cudaMemsetAsync(W->bar, 0, kBarBytes, W->stream));
+    if (A->pr_plan) {
+      const PrPlan &p = static_cast<const PlanHolder *>(A->pr_plan)->p;
+      TB_CUDA(cudaMemsetAsync(p.arrived, 0, (size_t)p.n_chunked * sizeof(int), W->stream));
+    }
     TB_CUDA(cudaStreamSynchronize(W->stream));
-    return fail(TBSLA_ERR_TIMEOUT, "a grid barrier of the PageRank solver ran out of time");
+    return fail(TBSLA_ERR_TIMEOUT, "a grid barrier of the PageRank solver ran out of polls");
   }
   return TBSLA_OK;
 }
@@ -476,7 +484,7 @@ tbsla_status_t run_f64(tbsla_matrix *A, PrWork *W, PrArgs<double> &a, int check_
     a.limit = sweep_limit(A);
     do {
       TB_TRY((launch_solver<MODE, double, double, AA>(A, m, a, W, W->stream)));
-      TB_TRY(pr_wait(W));
+      TB_TRY(pr_wait(A, W));
       a.init = 0;
     } while (!W->ctl_host->done);
     return TBSLA_OK;
@@ -491,7 +499,7 @@ tbsla_status_t run_f64(tbsla_matrix *A, PrWork *W, PrArgs<double> &a, int check_
       TB_TRY(spmv_dispatch(A, TBSLA_F64, TBSLA_F64, AA ? W->x[0] : W->x[k & 1], TBSLA_F64, W->prod, 0, W->stream));
       TB_TRY((launch_solver<MODE, double, double, AA>(A, m, a, W, W->stream)));
     }
-    TB_TRY(pr_wait(W));
+    TB_TRY(pr_wait(A, W));
   } while (!W->ctl_host->done);
   return TBSLA_OK;
 }
@@ -543,7 +551,7 @@ tbsla_status_t run_mixed(tbsla_matrix *A, PrWork *W, PrArgs<double> &a, tbsla_dt
     // three corrections bring an FP32 store to 1e-12: the host looks after
     // the fourth FP64 sweep, then after each
     if (!walked || round >= 3) {
-      TB_TRY(pr_wait(W));
+      TB_TRY(pr_wait(A, W));
       if (W->ctl_host->done) return TBSLA_OK;
     }
     if (walked) {
@@ -555,7 +563,7 @@ tbsla_status_t run_mixed(tbsla_matrix *A, PrWork *W, PrArgs<double> &a, tbsla_dt
         TB_TRY(spmv_dispatch(A, store, TBSLA_F32, AA ? W->e[0] : W->e[k & 1], TBSLA_F32, W->prod32, 0, W->stream));
         TB_TRY((launch_solver<kSweepInner, V, float, AA>(A, mi, in, W, W->stream)));
       }
-      TB_TRY(pr_wait(W));
+      TB_TRY(pr_wait(A, W));
       if (W->ctl_host->inner_done) break;
     }
   }

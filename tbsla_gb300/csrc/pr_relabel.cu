@@ -205,6 +205,7 @@ tbsla_status_t build(tbsla_matrix *A, bool check_skew, bool *built) {
   B->x_keep = A->x_keep;
   B->x_keep_range = A->x_keep_range;
   B->short_mode = A->short_mode;
+  B->pr_polls = A->pr_polls;
   A->pr_relabel = B;
   A->pr_newid = d_newid;
   A->pr_newid_host = std::move(newid);

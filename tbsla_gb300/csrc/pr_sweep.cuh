@@ -133,23 +133,31 @@ template <typename T> struct PrArgs {
 // that completes this barrier.  The wait is bounded by a number of polls (reads of
 // L2, some tenths of a microsecond each), not by a clock: time while the context
 // is off the GPU, which other contexts may share, is not counted.  A block
-// that gives up raises bar[kPrGaveUp] and the kernel returns.
+// that gives up raises bar[kPrGaveUp] for the host and kPrLost in the arrival
+// count, and returns; every other block, whether it waits or arrives later and
+// completes the count, sees the bit in the word it polls and returns too.
+// (A launch has at most 10^6 sweeps of two barriers each on one block per SM: its
+// arrivals stay far below that bit.)
 constexpr int kPrLeft = 32, kPrGaveUp = 48, kPrBarWords = 64;  // words of the barrier, in lines of their own
+constexpr unsigned kPrLost = 1u << 31;
 
 __device__ __forceinline__ bool pr_barrier(unsigned *bar, unsigned &target, unsigned polls) {
   __shared__ int lost;
   target += gridDim.x;
   __syncthreads();
   if (threadIdx.x == 0) {
-    lost = 0;
     __threadfence();
     atomicAdd(bar, 1u);
-    for (unsigned k = 0; (int)(*(volatile unsigned *)bar - target) < 0; ++k)
+    unsigned seen = *(volatile unsigned *)bar;
+    for (unsigned k = 0; seen < target; ++k) {  // kPrLost is above every target
       if (k >= polls) {
         atomicExch(bar + kPrGaveUp, 1u);
-        lost = 1;
+        seen = atomicOr(bar, kPrLost) | kPrLost;
         break;
       }
+      seen = *(volatile unsigned *)bar;
+    }
+    lost = (seen & kPrLost) != 0;
     __threadfence();
   }
   __syncthreads();

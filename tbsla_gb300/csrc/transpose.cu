@@ -264,6 +264,7 @@ tbsla_status_t ensure_transpose(tbsla_matrix *A, tbsla_matrix **T) {
   B->x_keep = A->x_keep;
   B->x_keep_range = A->x_keep_range;
   B->short_mode = A->short_mode;
+  B->pr_polls = A->pr_polls;
   int *d_perm = guard.perm;
   guard.perm = nullptr;
   guard.B = nullptr;
