@@ -8,6 +8,7 @@
 
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
+#include <algorithm>
 #include <vector>
 
 #include "common.cuh"
@@ -17,10 +18,11 @@ namespace tbsla {
 tbsla_matrix *new_matrix(int format);
 void free_matrix(tbsla_matrix *A);
 tbsla_status_t alloc_ints(tbsla_matrix *A, int **p, int64_t n);
-tbsla_status_t store_values_device(tbsla_matrix *A, const double *d_src, int64_t n, int stores, cudaStream_t s);
+tbsla_status_t rederive_stores(tbsla_matrix *A, cudaStream_t s);
 tbsla_status_t csr_bins(tbsla_matrix *A, const std::vector<int> &rp);
 
-// Device scratch, freed together (cudaFree waits for the device)
+// Device scratch: freed together at the end, or one by one as soon as it is not
+// needed (cudaFree waits for the device)
 struct SortScratch {
   std::vector<void *> owned;
   ~SortScratch() {
@@ -36,6 +38,12 @@ struct SortScratch {
     *p = static_cast<T *>(q);
     return TBSLA_OK;
   }
+  // p belongs to the caller from here on
+  void give(void *p) { owned.erase(std::find(owned.begin(), owned.end(), p)); }
+  void drop(void *p) {
+    give(p);
+    cudaFree(p);
+  }
 };
 
 inline int key_bits(uint64_t largest) {
@@ -44,26 +52,37 @@ inline int key_bits(uint64_t largest) {
   return b;
 }
 
-// keys and entries into increasing key order, equal keys in entry order;
-// sorted / order point into the scratch
-template <typename K>
-inline tbsla_status_t sort_entries(SortScratch &sc, K *keys, int *entries, int64_t n, int bits, K **sorted,
-                                   int **order) {
-  K *k2 = nullptr;
-  int *e2 = nullptr;
-  TB_TRY(sc.get(&k2, n));
-  TB_TRY(sc.get(&e2, n));
-  cub::DoubleBuffer<K> kb(keys, k2);
-  cub::DoubleBuffer<int> eb(entries, e2);
-  size_t bytes = 0;
-  TB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, bytes, kb, eb, n, 0, bits));
-  char *tmp = nullptr;
-  TB_TRY(sc.get(&tmp, (int64_t)bytes));
-  TB_CUDA(cub::DeviceRadixSort::SortPairs(tmp, bytes, kb, eb, n, 0, bits));
-  *sorted = kb.Current();
-  *order = eb.Current();
-  return TBSLA_OK;
-}
+// The keys and entries of a sort and the second pair of arrays it needs: 16 bytes
+// an entry with 32-bit keys, as much as a plain FP64 copy and its map take
+// afterwards, so that a copy which fits can also be built
+template <typename K> struct SortPairs {
+  K *keys = nullptr, *other_keys = nullptr;
+  int *entries = nullptr, *other_entries = nullptr;
+  int64_t n = 0;
+  tbsla_status_t get(SortScratch &sc, int64_t n_) {
+    n = n_;
+    TB_TRY(sc.get(&keys, n));
+    TB_TRY(sc.get(&other_keys, n));
+    TB_TRY(sc.get(&entries, n));
+    return sc.get(&other_entries, n);
+  }
+  // into increasing key order, equal keys as they were
+  tbsla_status_t sort(SortScratch &sc, int bits) {
+    cub::DoubleBuffer<K> kb(keys, other_keys);
+    cub::DoubleBuffer<int> eb(entries, other_entries);
+    size_t bytes = 0;
+    TB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, bytes, kb, eb, n, 0, bits));
+    char *tmp = nullptr;
+    TB_TRY(sc.get(&tmp, (int64_t)bytes));
+    TB_CUDA(cub::DeviceRadixSort::SortPairs(tmp, bytes, kb, eb, n, 0, bits));
+    sc.drop(tmp);
+    keys = kb.Current();
+    other_keys = kb.Alternate();
+    entries = eb.Current();
+    other_entries = eb.Alternate();
+    return TBSLA_OK;
+  }
+};
 
 namespace {
 
@@ -99,6 +118,20 @@ __global__ void __launch_bounds__(256) take_kernel(const T *__restrict__ src, co
 }
 
 inline int entry_grid(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 152 * 32)); }
+
+// The stores of B, those that A has (F64 among them), from A's values in another order
+inline tbsla_status_t take_values(tbsla_matrix *B, const tbsla_matrix *A, const int *order) {
+  const int64_t n = A->stored;
+  const size_t size[3] = {8, 4, 2};
+  for (int k = 0; k < 3; ++k)
+    if (A->values[k]) TB_TRY(dev_alloc(B, &B->values[k], (size_t)n * size[k]));
+  B->stores = A->stores;
+  if (n)
+    take_kernel<<<entry_grid(n), 256>>>(static_cast<const double *>(A->values[0]), order, n,
+                                        static_cast<double *>(B->values[0]));
+  TB_CUDA(cudaGetLastError());
+  return rederive_stores(B, 0);
+}
 
 }  // namespace
 }  // namespace tbsla

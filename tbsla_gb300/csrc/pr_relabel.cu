@@ -83,22 +83,26 @@ __global__ void new_labels_kernel(const int *__restrict__ order, int n, int *__r
     newid[order[i]] = (int)i;
 }
 
-__global__ void relabelled_keys_kernel(const int *__restrict__ row, const int *__restrict__ col, int f_col,
-                                       const int *__restrict__ newid, int64_t nnz, int n,
-                                       uint64_t *__restrict__ keys, int *__restrict__ entries) {
+// key = new column of the entry, entry = position
+__global__ void new_column_keys_kernel(const int *__restrict__ col, int f_col, const int *__restrict__ newid,
+                                       int64_t nnz, uint32_t *__restrict__ keys, int *__restrict__ entries) {
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nnz; k += (int64_t)gridDim.x * blockDim.x) {
-    keys[k] = (uint64_t)newid[row[k]] * (uint64_t)n + (uint64_t)newid[col[k] - f_col];
+    keys[k] = (uint32_t)newid[col[k] - f_col];
     entries[k] = (int)k;
   }
 }
 
-__global__ void split_keys_kernel(const uint64_t *__restrict__ keys, int64_t nnz, int n, int *__restrict__ row,
-                                  int *__restrict__ col) {
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nnz; k += (int64_t)gridDim.x * blockDim.x) {
-    const uint64_t r = keys[k] / (uint64_t)n;
-    row[k] = (int)r;
-    col[k] = (int)(keys[k] - r * (uint64_t)n);
-  }
+// rows[k] = newid[rows[k]]
+__global__ void new_rows_kernel(const int *__restrict__ newid, int64_t nnz, uint32_t *__restrict__ rows) {
+  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nnz; k += (int64_t)gridDim.x * blockDim.x)
+    rows[k] = (uint32_t)newid[rows[k]];
+}
+
+// out[k] = the new column of entry order[k]
+__global__ void take_columns_kernel(const int *__restrict__ col, int f_col, const int *__restrict__ newid,
+                                    const int *__restrict__ order, int64_t nnz, int *__restrict__ out) {
+  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nnz; k += (int64_t)gridDim.x * blockDim.x)
+    out[k] = newid[col[order[k]] - f_col];
 }
 
 int cls_max(int maxdeg) { return 31 - __builtin_clz((unsigned)maxdeg + 1u); }
@@ -150,15 +154,6 @@ tbsla_status_t build(tbsla_matrix *A, bool check_skew, bool *built) {
   // vertices by out-degree class, then in-degree, both descending: one stable
   // sort of (class, in-degree) keys
   const int grid = entry_grid(n), egrid = entry_grid(nnz);
-  SortScratch sc;
-  uint64_t *vkeys = nullptr, *vsorted = nullptr, *ekeys = nullptr, *esorted = nullptr;
-  int *verts = nullptr, *order = nullptr, *entries = nullptr, *eorder = nullptr, *row = nullptr;
-  double *vals = nullptr;
-  TB_TRY(sc.get(&vkeys, n));
-  TB_TRY(sc.get(&verts, n));
-  const int top_cls = cls_max(maxdeg);
-  vertex_keys_kernel<<<grid, 256>>>(d_deg, A->idx0, n, top_cls, vkeys, verts);
-  TB_TRY(sort_entries(sc, vkeys, verts, n, 32 + key_bits((uint64_t)top_cls), &vsorted, &order));
   tbsla_matrix *B = new_matrix(TBSLA_FMT_CSR);
   if (!B) return fail(TBSLA_ERR_OOM, "host allocation failed");
   struct Guard {
@@ -175,26 +170,47 @@ tbsla_status_t build(tbsla_matrix *A, bool check_skew, bool *built) {
     cudaGetLastError();
     return fail(TBSLA_ERR_OOM, "relabel map (%d ints)", n);
   }
-  new_labels_kernel<<<grid, 256>>>(order, n, guard.newid);
-  // the entries by (new row, new column), repeated columns in their order
-  TB_TRY(sc.get(&ekeys, nnz));
-  TB_TRY(sc.get(&entries, nnz));
-  TB_TRY(sc.get(&row, nnz));
-  TB_TRY(sc.get(&vals, nnz));
-  entry_rows_kernel<<<152 * 16, 256>>>(n, A->idx0, row);
-  relabelled_keys_kernel<<<egrid, 256>>>(row, A->idx1, A->f_col, guard.newid, nnz, n, ekeys, entries);
-  TB_TRY(sort_entries(sc, ekeys, entries, nnz, key_bits((uint64_t)n * (uint64_t)n - 1), &esorted, &eorder));
+  {
+    SortScratch sc;
+    SortPairs<uint64_t> p;
+    TB_TRY(p.get(sc, n));
+    const int top_cls = cls_max(maxdeg);
+    vertex_keys_kernel<<<grid, 256>>>(d_deg, A->idx0, n, top_cls, p.keys, p.entries);
+    TB_TRY(p.sort(sc, 32 + key_bits((uint64_t)top_cls)));
+    new_labels_kernel<<<grid, 256>>>(p.entries, n, guard.newid);
+    TB_CUDA(cudaGetLastError());
+  }
   B->n_row = B->n_col = B->rows = n;
   B->stored = nnz;
   // columns with entries come first (their class is above that of degree 0)
   B->x_extent = n - std::count(deg.begin(), deg.end(), 0);
   TB_TRY(alloc_ints(B, &B->idx0, (int64_t)n + 1));
+  // the entries by (new row, new column), repeated columns in their order: a
+  // stable sort by column, then one by row
+  SortScratch kept;
+  int *order = nullptr;
+  {
+    SortScratch sc;
+    SortPairs<uint32_t> p;
+    TB_TRY(p.get(sc, nnz));
+    const int bits = key_bits((uint64_t)std::max(n - 1, 0));
+    new_column_keys_kernel<<<egrid, 256>>>(A->idx1, A->f_col, guard.newid, nnz, p.keys, p.entries);
+    TB_TRY(p.sort(sc, bits));
+    entry_rows_kernel<<<152 * 16, 256>>>(n, A->idx0, reinterpret_cast<int *>(p.other_keys));
+    new_rows_kernel<<<egrid, 256>>>(guard.newid, nnz, p.other_keys);
+    take_kernel<<<egrid, 256>>>(p.other_keys, p.entries, nnz, p.keys);
+    TB_TRY(p.sort(sc, bits));
+    key_starts_kernel<<<entry_grid((int64_t)n + 1), 256>>>(p.keys, nnz, (int64_t)n, B->idx0);
+    TB_CUDA(cudaGetLastError());
+    order = p.entries;
+    sc.give(order);
+    kept.owned.push_back(order);
+  }
   TB_TRY(alloc_ints(B, &B->idx1, nnz));
-  split_keys_kernel<<<egrid, 256>>>(esorted, nnz, n, row, B->idx1);  // row: of the sorted entries now
-  key_starts_kernel<<<entry_grid((int64_t)n + 1), 256>>>(row, nnz, (int64_t)n, B->idx0);
-  take_kernel<<<egrid, 256>>>(static_cast<const double *>(A->values[0]), eorder, nnz, vals);
-  TB_CUDA(cudaGetLastError());
-  TB_TRY(store_values_device(B, vals, nnz, A->stores, 0));
+  take_columns_kernel<<<egrid, 256>>>(A->idx1, A->f_col, guard.newid, order, nnz, B->idx1);
+  TB_TRY(take_values(B, A, order));
+  TB_CUDA(cudaStreamSynchronize(0));
+  kept.drop(order);
   std::vector<int> nrp((size_t)n + 1), newid((size_t)n);
   TB_CUDA(cudaMemcpy(nrp.data(), B->idx0, nrp.size() * sizeof(int), cudaMemcpyDeviceToHost));
   TB_CUDA(cudaMemcpy(newid.data(), guard.newid, newid.size() * sizeof(int), cudaMemcpyDeviceToHost));

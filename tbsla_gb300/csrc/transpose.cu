@@ -213,14 +213,6 @@ tbsla_status_t ensure_transpose(tbsla_matrix *A, tbsla_matrix **T) {
   const int ncol = A->n_col;
   const int64_t nnz = A->stored;
   const int grid = entry_grid(nnz);
-  SortScratch sc;
-  uint32_t *keys = nullptr, *sorted = nullptr;
-  int *entries = nullptr, *order = nullptr, *row = nullptr;
-  double *vals = nullptr;
-  TB_TRY(sc.get(&keys, nnz));
-  TB_TRY(sc.get(&entries, nnz));
-  TB_TRY(sc.get(&row, nnz));
-  TB_TRY(sc.get(&vals, nnz));
   tbsla_matrix *B = new_matrix(TBSLA_FMT_CSR);
   if (!B) return fail(TBSLA_ERR_OOM, "host allocation failed");
   struct Guard {
@@ -238,26 +230,32 @@ tbsla_status_t ensure_transpose(tbsla_matrix *A, tbsla_matrix **T) {
   B->rows = ncol;
   B->stored = nnz;
   TB_TRY(alloc_ints(B, &B->idx0, (int64_t)ncol + 1));
-  TB_TRY(alloc_ints(B, &B->idx1, nnz));
-  if (cudaMalloc(&guard.perm, (size_t)std::max<int64_t>(nnz, 1) * sizeof(int)) != cudaSuccess) {
-    cudaGetLastError();
-    return fail(TBSLA_ERR_OOM, "transpose map (%lld ints)", (long long)nnz);
-  }
   TB_CUDA(cudaDeviceSynchronize());  // A's values and arrays are in place, whichever stream wrote them
+  {
+    SortScratch sc;
+    SortPairs<uint32_t> p;
+    TB_TRY(p.get(sc, nnz));
+    if (nnz) {
+      column_keys_kernel<<<grid, 256>>>(A->idx1, A->f_col, nnz, p.keys, p.entries);
+      TB_TRY(p.sort(sc, key_bits((uint64_t)std::max(ncol - 1, 0))));
+    }
+    key_starts_kernel<<<entry_grid((int64_t)ncol + 1), 256>>>(p.keys, nnz, (int64_t)ncol, B->idx0);
+    TB_CUDA(cudaGetLastError());
+    sc.give(p.entries);
+    guard.perm = p.entries;
+  }
+  TB_TRY(alloc_ints(B, &B->idx1, nnz));
   if (nnz) {
-    column_keys_kernel<<<grid, 256>>>(A->idx1, A->f_col, nnz, keys, entries);
-    TB_TRY(sort_entries(sc, keys, entries, nnz, key_bits((uint64_t)std::max(ncol - 1, 0)), &sorted, &order));
+    SortScratch sc;
+    int *row = nullptr;
+    TB_TRY(sc.get(&row, nnz));
     entry_rows_kernel<<<152 * 16, 256>>>(A->rows, A->idx0, row);
-    take_kernel<<<grid, 256>>>(row, order, nnz, B->idx1);
-    take_kernel<<<grid, 256>>>(static_cast<const double *>(A->values[0]), order, nnz, vals);
-    TB_CUDA(cudaMemcpyAsync(guard.perm, order, (size_t)nnz * sizeof(int), cudaMemcpyDeviceToDevice, 0));
+    take_kernel<<<grid, 256>>>(row, guard.perm, nnz, B->idx1);
     int last = 0;  // the entries come in row order: the last one's row is the largest
     TB_CUDA(cudaMemcpy(&last, row + nnz - 1, sizeof last, cudaMemcpyDeviceToHost));
     B->x_extent = (int64_t)last + 1;
   }
-  key_starts_kernel<<<entry_grid((int64_t)ncol + 1), 256>>>(sorted, nnz, (int64_t)ncol, B->idx0);
-  TB_CUDA(cudaGetLastError());
-  TB_TRY(store_values_device(B, vals, nnz, A->stores, 0));
+  TB_TRY(take_values(B, A, guard.perm));
   std::vector<int> tp((size_t)ncol + 1);
   TB_CUDA(cudaMemcpy(tp.data(), B->idx0, tp.size() * sizeof(int), cudaMemcpyDeviceToHost));
   TB_TRY(csr_bins(B, tp));
