@@ -18,6 +18,7 @@ namespace tbsla {
 
 // ---------------------------------------------------------------- errors
 tbsla_status_t fail(tbsla_status_t s, const char *fmt, ...);
+void forget_error();  // of a best-effort step that failed
 tbsla_status_t cuda_fail(cudaError_t e, const char *what, const char *file, int line);
 
 #define TB_CUDA(call)                                                           \

@@ -32,6 +32,8 @@ tbsla_status_t cuda_fail(cudaError_t e, const char *what, const char *file, int 
   return fail(s, "%s: %s (%s:%d)", what, cudaGetErrorString(e), file, line);
 }
 
+void forget_error() { g_err.clear(); }
+
 int current_device() {
   int d = 0;
   if (g_device >= 0) return g_device;

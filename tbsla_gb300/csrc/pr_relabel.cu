@@ -253,8 +253,13 @@ tbsla_status_t pr_relabelled(tbsla_matrix *A, tbsla_matrix **B) {
       return TBSLA_OK;
     }
   }
+  // the copy only makes the solve faster: without the device memory for it
+  // (16 bytes an entry to sort, then the copy) A itself is swept, and unless the copy
+  // was asked for the build is not tried again until the values change
   bool built = false;
-  TB_TRY(build(A, !forced, &built));
+  const tbsla_status_t st = build(A, !forced, &built);
+  if (st == TBSLA_ERR_OOM) forget_error();
+  else TB_TRY(st);
   A->pr_relabel_state = built ? 1 : 2;
   *B = built ? A->pr_relabel : nullptr;
   return TBSLA_OK;

@@ -70,3 +70,27 @@ def test_relabelled_copy_where_its_entries_fit(gpu):
     with Ballast(24 * A.info().stored + (64 << 20)):
         A.pagerank(out.data_ptr(), tol=0.0, max_iter=5, mode=gpu.PR_DANGLING)
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("scale,relabel", [(20, -1), (18, 1)])
+def test_solves_without_room_for_the_relabelled_copy(gpu, scale, relabel):
+    """The copy only makes a solve faster: with less memory than its build needs
+    (10 bytes an entry are left, it sorts 16) the handle itself is swept.  Both
+    orders of summation are within s (L + n) u of exact after s sweeps (L entries
+    in the longest row, u = 2^-53)."""
+    from tbsla_gb300 import capi
+    n, nnz, sweeps = 1 << scale, 1 << 24, 5
+    A = gpu.DeviceMatrix.rmat_pagerank(scale, nnz)
+    longest = int(np.diff(A.csr_download()[0]).max())
+    out, want, ppr = (torch.empty(n, dtype=torch.float64, device="cuda") for _ in range(3))
+    A.tune(gpu.TUNE_PR_RELABEL, 0)
+    A.pagerank(want.data_ptr(), tol=0.0, max_iter=sweeps, mode=gpu.PR_DANGLING)
+    capi.ppr_batched(A, [[5]], ppr.data_ptr(), tol=0.0, max_iter=sweeps)
+    want_ppr, bound = ppr.clone(), 2 * sweeps * (longest + n) * 2.0 ** -53
+    A.tune(gpu.TUNE_PR_RELABEL, relabel)
+    for _ in range(2):
+        with Ballast(10 * A.info().stored):
+            A.pagerank(out.data_ptr(), tol=0.0, max_iter=sweeps, mode=gpu.PR_DANGLING)
+            capi.ppr_batched(A, [[5]], ppr.data_ptr(), tol=0.0, max_iter=sweeps)
+            torch.cuda.synchronize()
+        assert float((out - want).abs().sum()) <= bound and float((ppr - want_ppr).abs().sum()) <= bound
