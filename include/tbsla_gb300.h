@@ -201,7 +201,9 @@ tbsla_status_t tbsla_matrix_set_variant(tbsla_matrix_t *A, int variant);
  *   TBSLA_TUNE_DROP_SLICED_COPY  1: frees the handle's ELL-layout copy (the
  *                         copy doubles the device memory of the entries);
  *                         products then read the CSR arrays.  Waits for the
- *                         device; the copy is not rebuilt.
+ *                         device; the copy is not rebuilt, by batches neither.
+ *                         Batches the handle is a member of are to be bound
+ *                         again before their next product.
  *   TBSLA_TUNE_PR_RELABEL PageRank on a copy of a CSR graph relabelled in
  *                         decreasing out-degree order (built on first use,
  *                         kept with the handle): 1 on, 0 off, -1 (default)
@@ -355,9 +357,10 @@ tbsla_status_t tbsla_coo_spmv_noalloc_status(int *bad, void *stream);
 /* Many CSR handles multiplied together: y_m = A_m x_m for every member in
  * ONE kernel launch (a persistent grid walking row items of every member
  * with a fixed stride, so sums are deterministic; members with an
- * ELL-layout copy, TBSLA_TUNE_SHORT_ROWS 3 or one tbsla_batch_create adds to a
- * smaller member of short, even rows (its entries' memory again), are read
- * from it for the F64 and F32 stores).  No reference counterpart (the reference multiplies one
+ * ELL-layout copy, TBSLA_TUNE_SHORT_ROWS 3 or one tbsla_batch_bind builds for a
+ * smaller member of short, even rows (columns and the bound store's values
+ * again; shared by the batches that bind that store and freed with the last of
+ * them), are read from it for the F64 and F32 stores).  No reference counterpart (the reference multiplies one
  * matrix per call). */
 typedef struct tbsla_batch tbsla_batch_t;
 /* members: count CSR handles on one device, kept alive by the caller */

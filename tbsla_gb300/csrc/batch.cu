@@ -8,8 +8,8 @@
 // from a CUDA graph as is.  A row is summed by one thread in its stored
 // order (the thread-per-row loads of csr_direct.cuh: the single products'
 // arithmetic with TBSLA_TUNE_SHORT_ROWS = 0).  Members with an ELL-layout copy
-// for the bound store (csr_sell_kernel's, or one the batch had built for a
-// member too small to keep that: batch_copy) are read from it, two rows per
+// for the bound store (csr_sell_kernel's, or one that the batches which bind
+// that store hold for a member too small for that: batch_copy) are read from it, two rows per
 // thread (items of 2 * kBatchRows rows): the same sums, coalesced loads.  64
 // cqmat matrices of 1e3 to 1e5 rows, FP32: 81 us reading the CSR arrays of the
 // members below 2^16 rows (a 16-byte load of 32 rows touches 20 lines or more),
@@ -22,7 +22,8 @@
 
 namespace tbsla {
 
-tbsla_status_t batch_copy(tbsla_matrix *A);
+bool batch_copy_wanted(const tbsla_matrix *A);
+tbsla_status_t batch_copy(tbsla_matrix *A, int k, std::shared_ptr<BatchCopy> *out);
 
 struct BatchMember {
   const int *rowptr;
@@ -111,6 +112,7 @@ struct tbsla_batch {
   int device = 0;
   std::vector<const tbsla_matrix *> members;
   std::vector<BatchMember> table;    // host copy of the member table
+  std::vector<std::shared_ptr<BatchCopy>> copies;  // of the members, for the bound store (NULL: none)
   BatchMember *d_table = nullptr;
   int4 *d_items = nullptr;
   int n_items = 0;
@@ -161,20 +163,12 @@ tbsla_status_t tbsla_batch_create(int count, const tbsla_matrix_t *const *member
       return fail(TBSLA_ERR_INVALID_ARG, "batch member %d is not a CSR handle on device %d", m, B->device);
     }
     B->members.push_back(A);
-    const tbsla_status_t cs = batch_copy(const_cast<tbsla_matrix *>(A));
-    if (cs != TBSLA_OK) {
-      delete B;
-      return cs;
-    }
     BatchMember d{};
     d.rowptr = A->idx0;
     d.colidx = A->idx1;
     d.f_col = A->f_col;
     d.rows = A->rows;
     d.n_row = A->n_row;
-    d.sell_width = A->sell_width ? A->sell_width : A->bsell_width;
-    d.sell_cols = A->sell_width ? A->sell_cols : A->bsell_cols;
-    d.sell_stride = A->sell_width ? A->sell_stride : A->bsell_stride;
     B->table.push_back(d);
   }
   // members with an ELL-layout copy: items of two rows per thread, one when the
@@ -182,8 +176,9 @@ tbsla_status_t tbsla_batch_create(int count, const tbsla_matrix_t *const *member
   int64_t pairs = 0;
   for (const tbsla_matrix *A : B->members) pairs += (A->n_row + 2 * kBatchRows - 1) / (2 * kBatchRows);
   for (int m = 0; m < count; ++m) {
-    const int n_row = B->members[(size_t)m]->n_row;
-    const int span = B->table[(size_t)m].sell_width && pairs >= 152 * 4 ? 2 * kBatchRows : kBatchRows;
+    const tbsla_matrix *A = B->members[(size_t)m];
+    const int n_row = A->n_row;
+    const int span = (A->sell_width || batch_copy_wanted(A)) && pairs >= 152 * 4 ? 2 * kBatchRows : kBatchRows;
     for (int r = 0; r < n_row; r += span) items.push_back(make_int4(m, r, std::min(r + span, n_row), 0));
   }
   B->n_items = (int)items.size();
@@ -204,18 +199,40 @@ tbsla_status_t tbsla_batch_bind(tbsla_batch_t *B, tbsla_dtype_t store, const voi
   TB_CHECK(B && d_x && d_y, "NULL argument");
   TB_CHECK(store == TBSLA_F64 || store == TBSLA_F32 || store == TBSLA_BF16, "bad store");
   const int si = store_index(store);
+  std::vector<std::shared_ptr<BatchCopy>> copies;
   for (size_t m = 0; m < B->members.size(); ++m) {
     const tbsla_matrix *A = B->members[m];
     TB_CHECK(A->values[si], "batch member %zu lacks the requested value store", m);
     TB_CHECK(d_y[m] || A->n_row == 0, "y of member %zu is NULL", m);
     TB_CHECK(d_x[m] || A->stored == 0, "x of member %zu is NULL", m);
-    B->table[m].values = A->values[si];
-    B->table[m].sell_vals = si >= 2 ? nullptr : A->sell_width ? A->sell_vals[si] : A->bsell_vals[si];
-    B->table[m].x = d_x[m];
-    B->table[m].y = d_y[m];
   }
   TB_CUDA(cudaSetDevice(B->device));
+  for (size_t m = 0; m < B->members.size(); ++m) {
+    const tbsla_matrix *A = B->members[m];
+    BatchMember &d = B->table[m];
+    d.values = A->values[si];
+    d.x = d_x[m];
+    d.y = d_y[m];
+    d.sell_vals = nullptr;  // BF16: none is read
+    std::shared_ptr<BatchCopy> c;
+    if (si < 2 && A->sell_width) {
+      d.sell_width = A->sell_width;
+      d.sell_cols = A->sell_cols;
+      d.sell_stride = A->sell_stride;
+      d.sell_vals = A->sell_vals[si];
+    } else if (si < 2 && batch_copy_wanted(A)) {
+      TB_TRY(batch_copy(const_cast<tbsla_matrix *>(A), si, &c));
+      if (c) {
+        d.sell_width = c->width;
+        d.sell_cols = c->cols;
+        d.sell_stride = c->stride;
+        d.sell_vals = c->vals[si];
+      }
+    }
+    copies.push_back(std::move(c));
+  }
   TB_CUDA(cudaMemcpy(B->d_table, B->table.data(), sizeof(BatchMember) * B->table.size(), cudaMemcpyHostToDevice));
+  B->copies.swap(copies);  // the former ones go; cudaFree waits for launches that read them
   B->bound = true;
   if (B->store != store && B->graph) {
     cudaGraphExecDestroy(B->graph);

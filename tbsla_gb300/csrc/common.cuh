@@ -7,6 +7,7 @@
 
 #include <cstdarg>
 #include <cstdint>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <utility>
@@ -58,6 +59,19 @@ namespace tbsla {
 // rows of at most this many entries, all in order: csr_tiny_kernel
 constexpr int kTinyRow = 4;
 }  // namespace tbsla
+
+// ELL-layout copy of a batch member, for the stores that batches have bound
+struct BatchCopy {
+  int *cols = nullptr;               // padding: column -1
+  void *vals[2] = {nullptr, nullptr};  // F64, F32
+  int64_t stride = 0, bytes = 0;
+  int width = 0;
+  ~BatchCopy() {
+    if (cols) cudaFree(cols);
+    for (void *p : vals)
+      if (p) cudaFree(p);
+  }
+};
 
 // The opaque matrix handle of the C ABI.
 struct tbsla_matrix {
@@ -116,12 +130,11 @@ struct tbsla_matrix {
   void *sell_vals[3] = {nullptr, nullptr, nullptr};
   int64_t sell_stride = 0;  // rows rounded up to a multiple of 128
   int sell_width = 0;       // slots per row (the longest row); 0: no copy
-  // the same copy for members of a batch below the rows where plain products
-  // gain from one (batch.cu builds it; F64 and F32 stores)
-  int *bsell_cols = nullptr;
-  void *bsell_vals[2] = {nullptr, nullptr};
-  int64_t bsell_stride = 0;
-  int bsell_width = 0;
+  bool sell_dropped = false;  // TBSLA_TUNE_DROP_SLICED_COPY: batches build none either
+  // the same copy for a member of batches with fewer rows than plain products
+  // gain from one at (batch_copy): it belongs to the batches that read it, and new
+  // values reach it here while there is one
+  std::weak_ptr<BatchCopy> batch_copy;
   int sell_rows = 0;        // rows per thread of csr_sell_kernel (1, 2, 4; 0: by size)
   int4 *warp_items = nullptr;
   int n_warp_items = 0;
@@ -189,6 +202,7 @@ struct tbsla_matrix {
   int64_t cap_x = 0, cap_y = 0, cap_t = 0;
 
   int64_t device_bytes = 0;
+  std::mutex first_use;  // guards what is built on first use by any of several threads
   std::mutex host_mu;
 
   // optional per-launch timing of the main product kernel

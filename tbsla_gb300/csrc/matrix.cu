@@ -203,54 +203,76 @@ static tbsla_status_t upload_values(tbsla_matrix *A, const double *host, int64_t
   return TBSLA_OK;
 }
 
-// The values of a batch member's ELL-layout copy from its stores
-static tbsla_status_t batch_copy_refresh(tbsla_matrix *A, cudaStream_t s) {
-  if (!A->bsell_width) return TBSLA_OK;
+// The values of store k of a batch member's ELL-layout copy
+static tbsla_status_t batch_copy_values(const tbsla_matrix *A, const BatchCopy &c, int k, cudaStream_t s) {
   const int grid = grid_for(A->rows, 256);
-  if (A->bsell_vals[0])
-    sell_scatter_kernel<double><<<grid, 256, 0, s>>>(A->idx0, A->bsell_stride, A->rows,
+  if (k == 0)
+    sell_scatter_kernel<double><<<grid, 256, 0, s>>>(A->idx0, c.stride, A->rows,
                                                      static_cast<const double *>(A->values[0]),
-                                                     static_cast<double *>(A->bsell_vals[0]));
-  if (A->bsell_vals[1])
-    sell_scatter_kernel<float><<<grid, 256, 0, s>>>(A->idx0, A->bsell_stride, A->rows,
+                                                     static_cast<double *>(c.vals[0]));
+  else
+    sell_scatter_kernel<float><<<grid, 256, 0, s>>>(A->idx0, c.stride, A->rows,
                                                     static_cast<const float *>(A->values[1]),
-                                                    static_cast<float *>(A->bsell_vals[1]));
+                                                    static_cast<float *>(c.vals[1]));
   TB_CUDA(cudaGetLastError());
   return TBSLA_OK;
 }
+static tbsla_status_t batch_copy_refresh(tbsla_matrix *A, cudaStream_t s) {
+  const std::shared_ptr<BatchCopy> c = A->batch_copy.lock();
+  for (int k = 0; c && k < 2; ++k)
+    if (c->vals[k]) TB_TRY(batch_copy_values(A, *c, k, s));
+  return TBSLA_OK;
+}
 
-// Builds it for a member of a batch: a CSR handle without the copy of
-// csr_bins, every row short, at least 256 rows of four entries on average, at
-// most 1/32 more slots than entries.  Best effort, as in csr_bins.
-tbsla_status_t batch_copy(tbsla_matrix *A) {
-  if (A->bsell_width || A->sell_width || A->format != TBSLA_FMT_CSR || A->stage_cap == 0 || A->rows < 256 ||
-      !(A->values[0] || A->values[1]))
-    return TBSLA_OK;
-  const int64_t stride = ((int64_t)A->rows + 31) / 32 * 32, total = stride * A->short_max;
-  if (A->stored < 4ll * A->rows || total > A->stored + A->stored / 32) return TBSLA_OK;
-  const size_t esz[3] = {4, 8, 4};
-  void **bufs[3] = {(void **)&A->bsell_cols, &A->bsell_vals[0], &A->bsell_vals[1]};
-  bool ok = true;
-  for (int k = 0; k < 3 && ok; ++k)
-    if (k == 0 || A->values[k - 1]) ok = dev_alloc(A, bufs[k], (size_t)total * esz[k]) == TBSLA_OK;
-  if (!ok) {
-    for (int k = 0; k < 3; ++k)
-      if (*bufs[k]) {
-        cudaFree(*bufs[k]);
-        *bufs[k] = nullptr;
-        A->device_bytes -= total * (int64_t)esz[k] + 64;
-      }
-    g_err.clear();
-    return TBSLA_OK;
+// Whether batches read A from a copy of their own: a CSR handle too small for the
+// copy of csr_bins, every row short, 256 to 2^16 rows of four entries on
+// average, at most 1/32 more slots than entries, and its caller did not drop
+// the ELL layout.
+bool batch_copy_wanted(const tbsla_matrix *A) {
+  if (A->sell_width || A->sell_dropped || A->format != TBSLA_FMT_CSR || A->stage_cap == 0 || A->rows < 256 ||
+      A->rows >= (1 << 16))
+    return false;
+  const int64_t total = ((int64_t)A->rows + 31) / 32 * 32 * A->short_max;
+  return A->stored >= 4ll * A->rows && total <= A->stored + A->stored / 32;
+}
+
+// A's copy with the values of store k (F64, F32), built or completed here, for
+// as long as the caller holds it; NULL without the memory for it (the batch then
+// reads the CSR arrays).
+tbsla_status_t batch_copy(tbsla_matrix *A, int k, std::shared_ptr<BatchCopy> *out) {
+  std::lock_guard<std::mutex> lk(A->first_use);
+  std::shared_ptr<BatchCopy> c = A->batch_copy.lock();
+  out->reset();
+  const bool fresh = !c;
+  if (fresh) {
+    c = std::make_shared<BatchCopy>();
+    c->width = A->short_max;
+    c->stride = ((int64_t)A->rows + 31) / 32 * 32;
   }
-  TB_CUDA(cudaMemset(A->bsell_cols, 0xff, (size_t)total * sizeof(int)));  // padding: column -1
-  for (int k = 0; k < 2; ++k)
-    if (A->bsell_vals[k]) TB_CUDA(cudaMemset(A->bsell_vals[k], 0, (size_t)total * esz[k + 1]));
-  sell_scatter_kernel<int><<<grid_for(A->rows, 256), 256>>>(A->idx0, stride, A->rows, A->idx1, A->bsell_cols);
-  A->bsell_stride = stride;
-  A->bsell_width = A->short_max;
-  TB_TRY(batch_copy_refresh(A, 0));
-  TB_CUDA(cudaDeviceSynchronize());
+  if (!c->vals[k]) {
+    const int64_t total = c->stride * c->width;
+    const size_t size = (size_t)total * (k == 0 ? 8 : 4);
+    void *cols = nullptr, *vals = nullptr;
+    if ((fresh && dev_alloc(nullptr, &cols, (size_t)total * sizeof(int)) != TBSLA_OK) ||
+        dev_alloc(nullptr, &vals, size) != TBSLA_OK) {
+      if (cols) cudaFree(cols);
+      g_err.clear();
+      return TBSLA_OK;
+    }
+    if (fresh) {
+      c->cols = static_cast<int *>(cols);
+      c->bytes += total * (int64_t)sizeof(int) + 64;
+      TB_CUDA(cudaMemset(cols, 0xff, (size_t)total * sizeof(int)));
+      sell_scatter_kernel<int><<<grid_for(A->rows, 256), 256>>>(A->idx0, c->stride, A->rows, A->idx1, c->cols);
+    }
+    c->vals[k] = vals;
+    c->bytes += (int64_t)size + 64;
+    TB_CUDA(cudaMemset(vals, 0, size));
+    TB_TRY(batch_copy_values(A, *c, k, 0));
+    TB_CUDA(cudaDeviceSynchronize());
+    A->batch_copy = c;
+  }
+  *out = c;
   return TBSLA_OK;
 }
 
@@ -379,7 +401,7 @@ static void free_handle(tbsla_matrix *A) {
                   A->short_rows, A->warp_items, A->chunk_rows, A->chunk_partials, A->chunk_partials32,
                   A->tile_start, A->tile_head_row, A->tile_head_val,
                   A->tile_tail_val, A->tile_emitted, A->tile_head_val32, A->tile_tail_val32,
-                  A->dangling, A->pr_scratch, A->col_pattern, A->seg_row, A->bsell_cols, A->bsell_vals[0], A->bsell_vals[1], A->d_x, A->d_y, A->d_t, A->d_err, A->pr_newid, A->pr_out,
+                  A->dangling, A->pr_scratch, A->col_pattern, A->seg_row, A->d_x, A->d_y, A->d_t, A->d_err, A->pr_newid, A->pr_out,
                   A->transpose_perm, A->coo_rowptr, A->sell_cols, A->sell_vals[0], A->sell_vals[1],
                   A->sell_vals[2]};
   for (void *p : ptrs) if (p) cudaFree(p);
@@ -988,6 +1010,7 @@ tbsla_status_t tbsla_matrix_tune(tbsla_matrix_t *A, int knob, double value) {
     return TBSLA_OK;
   case TBSLA_TUNE_DROP_SLICED_COPY:
     TB_CHECK(value == 1.0, "drop the sliced copy: value %g not 1", value);
+    A->sell_dropped = true;
     if (A->sell_width) {
       TB_CUDA(cudaSetDevice(A->device));
       TB_CUDA(cudaDeviceSynchronize());  // no product may still read it
@@ -1059,6 +1082,7 @@ tbsla_status_t tbsla_matrix_info(const tbsla_matrix_t *A, tbsla_matrix_info_t *i
   info->rows = A->rows; info->max_col = A->max_col;
   info->stored = A->stored; info->stores = A->stores;
   info->device_bytes = A->device_bytes;
+  if (const std::shared_ptr<BatchCopy> c = A->batch_copy.lock()) info->device_bytes += c->bytes;
   int k = 0;
   switch (A->format) {
   case TBSLA_FMT_CSR:
