@@ -275,12 +275,13 @@ __device__ __forceinline__ double pr_anderson(PrCtl::Aa &st, int k, double term,
 // late, and that sweep is lost when it says stop; so the pass that divides and
 // tests at once runs where the test may hold (the last sweep allowed; the first
 // two; the residual, should it go on falling as it did, below 1.25 tol), and
-// where the maximum is no ordinary number.  Runs in a warp, the two divisions in two
+// where the maximum is no ordinary positive number (a negative one turns the vector
+// round, which a power of two would not).  Runs in a warp, the two divisions in two
 // lanes (each is a chain of some twenty FP64 instructions; five of them in
 // one thread: 2.1 us a sweep).
 __device__ __forceinline__ void pr_ref_advance(PrCtl &c, int k, double mx, double sum, double change) {
   const int lane = threadIdx.x & 31;
-  const double q = lane ? change / fabs(c.scale) : mx / c.scale;
+  const double q = lane ? change / c.scale : mx / c.scale;
   const double resid = __shfl_sync(0xffffffffu, q, 1);
   if (lane) return;
   c.maxv = mx;
@@ -294,13 +295,13 @@ __device__ __forceinline__ void pr_ref_advance(PrCtl &c, int k, double mx, doubl
   }
   c.iter = k + 1;
   c.f64_sweeps += 1;
-  c.pass = k < 2 || c.iter >= c.max_iter || !(fabs(mx) > 1e-30 && fabs(mx) < 1e30) ||
+  c.pass = k < 2 || c.iter >= c.max_iter || !(mx > 1e-30 && mx < 1e30) ||
            c.resid * (c.resid < c.resid_prev ? c.resid : c.resid_prev) < 1.25 * c.tol * c.resid_prev;
   if (!c.pass) {
     c.known = 0;
     c.scale = mx;
     c.rho = q;
-    const double p = __longlong_as_double((2046ll << 52) - (__double_as_longlong(fabs(mx)) & (2047ll << 52)));
+    const double p = __longlong_as_double((2046ll << 52) - (__double_as_longlong(mx) & (2047ll << 52)));
     c.beta_s = c.beta * p;
     c.add = c.tele_scale * (sum * p);
   }
