@@ -227,23 +227,24 @@ tbsla_status_t solver_plan(tbsla_matrix *A, const PrPlan **out) {
   return TBSLA_OK;
 }
 
-// What the solver sweeps for the value store `vals` of A: the ELL layout (an
-// ELL handle, or the copy of a CSR / COO handle), the row items, or a product
-// launched before each step.
+// What the solver sweeps for the value store `vals` of A: where it walks A itself
+// the ELL layout (an ELL handle, or the copy of a CSR / COO handle) or the row
+// items, else a product launched before each step.
 template <typename V, typename T>
-tbsla_status_t solver_matrix(tbsla_matrix *A, const V *vals, T *prod, PrMat<V, T> *m) {
+tbsla_status_t solver_matrix(tbsla_matrix *A, const V *vals, bool walked, T *prod, PrMat<V, T> *m) {
   std::memset(m, 0, sizeof *m);
   m->rows = A->n_row;
   m->f_col = A->f_col;
   m->prod = prod;
   m->layout = kPrProduct;
+  if (!walked) return TBSLA_OK;
   if (walks_slots(A)) {
     m->layout = kPrSlots;
     m->ecols = A->idx0;
     m->evals = vals;
     m->estride = A->rows_pad;
     m->ewidth = A->max_col;
-  } else if (walks_items(A)) {
+  } else {
     const void *copy = nullptr;
     for (int k = 0; k < 2; ++k)
       if (A->sell_width && A->values[k] == static_cast<const void *>(vals)) copy = A->sell_vals[k];
@@ -474,8 +475,7 @@ tbsla_status_t run_f64(tbsla_matrix *A, PrWork *W, PrArgs<double> &a, int check_
     walked = false;
   if (!walked && !W->prod) TB_TRY(pr_alloc((void **)&W->prod, (size_t)W->n * 8));
   PrMat<double, double> m;
-  TB_TRY((solver_matrix<double, double>(A, static_cast<const double *>(A->values[0]), W->prod, &m)));
-  if (!walked) m.layout = kPrProduct;
+  TB_TRY((solver_matrix<double, double>(A, static_cast<const double *>(A->values[0]), walked, W->prod, &m)));
   TB_TRY(pr_partials(W, m.layout == kPrItems ? m.plan.n_chunked : 0));
   a.x[0] = W->x[0];
   a.x[1] = W->x[1];
@@ -516,9 +516,9 @@ tbsla_status_t run_mixed(tbsla_matrix *A, PrWork *W, PrArgs<double> &a, tbsla_dt
   if (!walked && !W->prod) TB_TRY(pr_alloc((void **)&W->prod, (size_t)W->n * 8));
   if (!walked && !W->prod32) TB_TRY(pr_alloc((void **)&W->prod32, (size_t)W->n * 4));
   PrMat<double, double> m;
-  TB_TRY((solver_matrix<double, double>(A, static_cast<const double *>(A->values[0]), W->prod, &m)));
+  TB_TRY((solver_matrix<double, double>(A, static_cast<const double *>(A->values[0]), walked, W->prod, &m)));
   PrMat<V, float> mi;
-  TB_TRY((solver_matrix<V, float>(A, static_cast<const V *>(A->values[store_index(store)]), W->prod32, &mi)));
+  TB_TRY((solver_matrix<V, float>(A, static_cast<const V *>(A->values[store_index(store)]), walked, W->prod32, &mi)));
   TB_TRY(pr_partials(W, m.layout == kPrItems ? m.plan.n_chunked : mi.layout == kPrItems ? mi.plan.n_chunked : 0));
   a.x[0] = W->x[0];
   a.x[1] = W->x[1];

@@ -129,3 +129,19 @@ def test_reference_mode_by_products(gpu, orc):
     bo, it = o.page_rank(0.0, 0.85, 6)
     assert r.iterations == it == 6
     assert np.abs(b - bo).sum() <= 4 * 2 * 6 * (40 + n) * 2.0 ** -53
+
+
+def test_reference_mode_by_products_keeps_no_work_list(gpu):
+    """Where the reference mode multiplies by products, the first solve takes its
+    vectors (26 bytes a row) and no list of the rows (16 bytes for each that has
+    entries, seven eighths here)."""
+    torch = pytest.importorskip("torch")
+    n = 1 << 22
+    rng = np.random.default_rng(22)
+    rp, ci, va, _ = graph(rng, n, [40])
+    A = gpu.DeviceMatrix.csr(n, n, rp, ci, va)
+    out = torch.empty(n, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    A.pagerank(out.data_ptr(), tol=0.0, max_iter=3, mode=gpu.PR_REFERENCE)
+    assert free - torch.cuda.mem_get_info()[0] <= 32 * n
