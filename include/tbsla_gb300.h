@@ -357,10 +357,10 @@ tbsla_status_t tbsla_coo_spmv_noalloc_status(int *bad, void *stream);
 /* Many CSR handles multiplied together: y_m = A_m x_m for every member in
  * ONE kernel launch (a persistent grid walking row items of every member
  * with a fixed stride, so sums are deterministic; members with an
- * ELL-layout copy, TBSLA_TUNE_SHORT_ROWS 3 or one tbsla_batch_bind builds for a
- * smaller member of short, even rows (columns and the bound store's values
- * again; shared by the batches that bind that store and freed with the last of
- * them), are read from it for the F64 and F32 stores).  No reference counterpart (the reference multiplies one
+ * ELL-layout copy, TBSLA_TUNE_SHORT_ROWS 3 or one that the batches of a
+ * smaller member of short, even rows hold (its columns, and the values of a
+ * store while that is bound; shared by them and freed with the last), are read
+ * from it for the F64 and F32 stores).  No reference counterpart (the reference multiplies one
  * matrix per call). */
 typedef struct tbsla_batch tbsla_batch_t;
 /* members: count CSR handles on one device, kept alive by the caller */

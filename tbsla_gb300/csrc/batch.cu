@@ -112,7 +112,7 @@ struct tbsla_batch {
   int device = 0;
   std::vector<const tbsla_matrix *> members;
   std::vector<BatchMember> table;    // host copy of the member table
-  std::vector<std::shared_ptr<BatchCopy>> copies;  // of the members, for the bound store (NULL: none)
+  std::vector<std::shared_ptr<BatchCopy>> copies;  // of the members (NULL: none, or BF16 is bound)
   BatchMember *d_table = nullptr;
   int4 *d_items = nullptr;
   int n_items = 0;
@@ -155,6 +155,7 @@ tbsla_status_t tbsla_batch_create(int count, const tbsla_matrix_t *const *member
   TB_CHECK(count > 0 && members, "empty batch");
   tbsla_batch *B = new tbsla_batch();
   B->device = members[0]->device;
+  cudaSetDevice(B->device);
   std::vector<int4> items;
   for (int m = 0; m < count; ++m) {
     const tbsla_matrix *A = members[m];
@@ -163,6 +164,14 @@ tbsla_status_t tbsla_batch_create(int count, const tbsla_matrix_t *const *member
       return fail(TBSLA_ERR_INVALID_ARG, "batch member %d is not a CSR handle on device %d", m, B->device);
     }
     B->members.push_back(A);
+    B->copies.emplace_back();
+    if (batch_copy_wanted(A)) {  // its columns; the values of the store that is bound follow
+      const tbsla_status_t st = batch_copy(const_cast<tbsla_matrix *>(A), -1, &B->copies.back());
+      if (st != TBSLA_OK) {
+        delete B;
+        return st;
+      }
+    }
     BatchMember d{};
     d.rowptr = A->idx0;
     d.colidx = A->idx1;
@@ -182,7 +191,6 @@ tbsla_status_t tbsla_batch_create(int count, const tbsla_matrix_t *const *member
     for (int r = 0; r < n_row; r += span) items.push_back(make_int4(m, r, std::min(r + span, n_row), 0));
   }
   B->n_items = (int)items.size();
-  cudaSetDevice(B->device);
   if (cudaMalloc(&B->d_table, sizeof(BatchMember) * count) != cudaSuccess ||
       cudaMalloc(&B->d_items, sizeof(int4) * std::max<size_t>(items.size(), 1)) != cudaSuccess ||
       (!items.empty() &&

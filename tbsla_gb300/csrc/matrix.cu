@@ -230,49 +230,51 @@ static tbsla_status_t batch_copy_refresh(tbsla_matrix *A, cudaStream_t s) {
 // the ELL layout.
 bool batch_copy_wanted(const tbsla_matrix *A) {
   if (A->sell_width || A->sell_dropped || A->format != TBSLA_FMT_CSR || A->stage_cap == 0 || A->rows < 256 ||
-      A->rows >= (1 << 16))
+      A->rows >= (1 << 16) || !(A->values[0] || A->values[1]))
     return false;
   const int64_t total = ((int64_t)A->rows + 31) / 32 * 32 * A->short_max;
   return A->stored >= 4ll * A->rows && total <= A->stored + A->stored / 32;
 }
 
-// A's copy with the values of store k (F64, F32), built or completed here, for
-// as long as the caller holds it; NULL without the memory for it (the batch then
-// reads the CSR arrays).
+// A's copy, its columns and with k >= 0 the values of store k (F64, F32), built or
+// completed here, for as long as the caller holds it; NULL without the memory for
+// it (the batch then reads the CSR arrays).
 tbsla_status_t batch_copy(tbsla_matrix *A, int k, std::shared_ptr<BatchCopy> *out) {
   std::lock_guard<std::mutex> lk(A->first_use);
-  std::shared_ptr<BatchCopy> c = A->batch_copy.lock();
   out->reset();
-  const bool fresh = !c;
-  if (fresh) {
+  std::shared_ptr<BatchCopy> c = A->batch_copy.lock();
+  const int64_t stride = ((int64_t)A->rows + 31) / 32 * 32, total = stride * A->short_max;
+  bool built = false;
+  if (!c) {
     c = std::make_shared<BatchCopy>();
     c->width = A->short_max;
-    c->stride = ((int64_t)A->rows + 31) / 32 * 32;
-  }
-  if (!c->vals[k]) {
-    const int64_t total = c->stride * c->width;
-    const size_t size = (size_t)total * (k == 0 ? 8 : 4);
-    void *cols = nullptr, *vals = nullptr;
-    if ((fresh && dev_alloc(nullptr, &cols, (size_t)total * sizeof(int)) != TBSLA_OK) ||
-        dev_alloc(nullptr, &vals, size) != TBSLA_OK) {
-      if (cols) cudaFree(cols);
-      g_err.clear();
+    c->stride = stride;
+    if (dev_alloc(nullptr, (void **)&c->cols, (size_t)total * sizeof(int)) != TBSLA_OK) {
+      forget_error();
       return TBSLA_OK;
     }
-    if (fresh) {
-      c->cols = static_cast<int *>(cols);
-      c->bytes += total * (int64_t)sizeof(int) + 64;
-      TB_CUDA(cudaMemset(cols, 0xff, (size_t)total * sizeof(int)));
-      sell_scatter_kernel<int><<<grid_for(A->rows, 256), 256>>>(A->idx0, c->stride, A->rows, A->idx1, c->cols);
+    c->bytes = total * (int64_t)sizeof(int) + 64;
+    TB_CUDA(cudaMemset(c->cols, 0xff, (size_t)total * sizeof(int)));
+    sell_scatter_kernel<int><<<grid_for(A->rows, 256), 256>>>(A->idx0, stride, A->rows, A->idx1, c->cols);
+    TB_CUDA(cudaGetLastError());
+    built = true;
+  }
+  if (k >= 0 && !c->vals[k]) {
+    const size_t size = (size_t)total * (k == 0 ? 8 : 4);
+    void *vals = nullptr;
+    if (dev_alloc(nullptr, &vals, size) != TBSLA_OK) {
+      forget_error();
+      return TBSLA_OK;
     }
     c->vals[k] = vals;
     c->bytes += (int64_t)size + 64;
     TB_CUDA(cudaMemset(vals, 0, size));
     TB_TRY(batch_copy_values(A, *c, k, 0));
-    TB_CUDA(cudaDeviceSynchronize());
-    A->batch_copy = c;
+    built = true;
   }
-  *out = c;
+  if (built) TB_CUDA(cudaDeviceSynchronize());
+  A->batch_copy = c;
+  *out = std::move(c);
   return TBSLA_OK;
 }
 

@@ -62,14 +62,14 @@ def test_copies_live_and_die_with_their_batches(gpu):
     Ms = [even(gpu, n, c, rng) for n, c in ((256, 4), (257, 32), (3000, 9), (60001, 5))]
     before = held(Ms)
     B = gpu.Batch(Ms)
-    assert held(Ms) == before                       # none before a store is bound
+    slots = [(n + 31) // 32 * 32 * c for n, c in ((256, 4), (257, 32), (3000, 9), (60001, 5))]
+    # the columns, where rounding the rows up to 32 adds at most 1/32 (257 rows: none)
+    assert [b - a for a, b in zip(before, held(Ms))] == [64 + 4 * s if i != 1 else 0 for i, s in enumerate(slots)]
     products(gpu, B, Ms, "BF16")
     assert held(Ms) == before                       # BF16 reads the CSR arrays
     products(gpu, B, Ms, "F32")
     one = held(Ms)
-    # columns and FP32 values: 8 bytes for each slot (rows rounded up to 32), where the
-    # rounding adds at most 1/32 (257 rows: none)
-    slots = [(n + 31) // 32 * 32 * c for n, c in ((256, 4), (257, 32), (3000, 9), (60001, 5))]
+    # and the FP32 values
     assert [b - a for a, b in zip(before, one)] == [2 * 64 + 8 * s if i != 1 else 0 for i, s in enumerate(slots)]
     C = gpu.Batch(Ms[1:])
     products(gpu, C, Ms[1:], "F32")
