@@ -16,8 +16,9 @@
  * failure.  On TBSLA_ERR_CUDA the handle stays valid only if the CUDA context
  * does.
  *
- * Threading: a handle may be used from several threads for reads (spmv on
- * device pointers); the *_host entry points use the handle's own stream and
+ * Threading: a handle may be used from several threads for reads (spmv and
+ * transposed products on device pointers, batched PageRank solves; the copies
+ * and plans they build on first use are built once); the *_host entry points use the handle's own stream and
  * staging buffers and must not run concurrently on one handle.
  */
 #ifndef TBSLA_GB300_H

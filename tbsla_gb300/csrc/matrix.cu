@@ -526,6 +526,7 @@ __global__ void __launch_bounds__(256) mask_start_kernel(const unsigned char *__
 }
 
 tbsla_status_t column_pattern(tbsla_matrix *A, const unsigned char **pattern) {
+  std::lock_guard<std::mutex> lk(A->first_use);
   if (!A->col_pattern) {
     unsigned char *p = nullptr;
     const size_t n = (size_t)std::max(A->n_col, 1);

@@ -776,6 +776,7 @@ void ppr_plan_free(void *q) {
 }
 tbsla_status_t ppr_plan(const tbsla_matrix *Mc, PprPlan **out) {
   tbsla_matrix *M = const_cast<tbsla_matrix *>(Mc);
+  std::lock_guard<std::mutex> lk(M->first_use);
   if (M->ppr_plan) {
     *out = static_cast<PprPlan *>(M->ppr_plan);
     return TBSLA_OK;

@@ -235,6 +235,7 @@ tbsla_status_t build(tbsla_matrix *A, bool check_skew, bool *built) {
 tbsla_status_t pr_relabelled(tbsla_matrix *A, tbsla_matrix **B) {
   *B = nullptr;
   if (A->pr_relabel_mode == 0 || !candidate(A)) return TBSLA_OK;
+  std::lock_guard<std::mutex> lk(A->first_use);
   if (A->pr_relabel_state == 1) {
     *B = A->pr_relabel;
     return TBSLA_OK;

@@ -226,6 +226,7 @@ tbsla_status_t grad_segments(tbsla_matrix *A) {
 
 // The transposed copy of a CSR handle, built on first use.
 tbsla_status_t ensure_transpose(tbsla_matrix *A, tbsla_matrix **T) {
+  std::lock_guard<std::mutex> lk(A->first_use);
   if (A->transpose) {
     *T = A->transpose;
     return TBSLA_OK;
