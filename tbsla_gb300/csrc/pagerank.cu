@@ -5,8 +5,8 @@
 // partial sums (residual, dangling mass, total mass, or the maximum; with
 // acceleration the residual dots); all sweeps of a solve run in one
 // cooperative launch (pr_sweep.cuh) for the layouts it walks: CSR and
-// row-sorted COO row items, the ELL layout.  Others (DENSE, row blocks, merge
-// path, rows the format never visits) launch their product and one step of
+// row-sorted COO row items, the ELL layout.  Others (DENSE, rows the format
+// never visits) launch their product and one step of
 // the same kernel per sweep.  No atomics on values: every result is
 // independent of scheduling.
 //
@@ -119,14 +119,19 @@ tbsla_status_t pr_alloc(void **p, size_t bytes) {
 }
 
 // ------------------------------------------------------------ plan
-// The layouts the solver kernel walks itself, every row visited exactly once
+// The layouts the solver kernel walks itself, every row visited exactly once.  The
+// kernel variant of the handle's products makes no difference: the row pointer
+// and the slots are there for all of them, and a product and a step per sweep
+// cost more launches than the graph of sweeps that such handles had (row-sorted
+// COO with the merge path, 65536 rows, 17 sweeps: 757 us, 626 as a graph, 246
+// walked; ELL with four rows a thread, 16 sweeps: 410, 343, 243).
 bool walks_items(const tbsla_matrix *A) {
   const bool csr = A->format == TBSLA_FMT_CSR;
   const bool coo = (A->format == TBSLA_FMT_COO || A->format == TBSLA_FMT_SCOO) && A->coo_rowptr;
-  return (csr || coo) && A->csr_variant == 0 && A->rows == A->n_row && A->stored > 0 && A->stored <= INT_MAX - 4096;
+  return (csr || coo) && A->rows == A->n_row && A->stored > 0 && A->stored <= INT_MAX - 4096;
 }
 bool walks_slots(const tbsla_matrix *A) {
-  return A->format == TBSLA_FMT_ELL && A->csr_variant == 0 && A->rows == A->n_row && A->rows > 0 && A->max_col > 0;
+  return A->format == TBSLA_FMT_ELL && A->rows == A->n_row && A->rows > 0 && A->max_col > 0;
 }
 
 struct PlanHolder {
