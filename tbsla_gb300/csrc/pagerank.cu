@@ -671,7 +671,7 @@ static tbsla_status_t adjoint_impl(tbsla_matrix *A, const tbsla_pagerank_params_
   TB_TRY(pr_setup(A, &W));
   tbsla_matrix *T = nullptr;
   TB_TRY(ensure_transpose(A, &T));
-  TB_CHECK(walks_items(T), "the transposed copy does not take the fused sweep");
+  TB_CHECK(T->stored > 0, "the adjoint needs a matrix with entries");
   const int n = W->n;
   if (!W->lam) TB_TRY(pr_alloc((void **)&W->lam, (size_t)n * 8));
   TB_TRY(pr_order(W, user));
