@@ -170,7 +170,8 @@ struct tbsla_matrix {
   unsigned pr_polls = 0;             // polls of a solver barrier (tbsla_matrix_tune; 0: the default)
   bool pr_dmask_stale = false;       // the values changed since pr_work's dangling mask
   unsigned char *col_pattern = nullptr;  // columns without a stored entry (column_mask.cuh)
-  // row classes of the PageRank solver (pagerank.cu; the row structure only)
+  int pr_near = 0;  // neighbouring rows gather neighbouring entries: 0 not looked at, 1 yes, 2 no
+  // row classes of the PageRank solver (pagerank.cu; the pattern only)
   void *pr_plan = nullptr;
   void (*pr_plan_free)(void *) = nullptr;
   unsigned char *dangling = nullptr;

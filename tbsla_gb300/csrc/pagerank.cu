@@ -134,6 +134,44 @@ bool walks_slots(const tbsla_matrix *A) {
   return A->format == TBSLA_FMT_ELL && A->rows == A->n_row && A->rows > 0 && A->max_col > 0;
 }
 
+// cnt[0] of cnt[1] entries of sampled rows have the entry at their place in the next
+// row within kNearCols columns of it (a warp per sampled row)
+constexpr int kNearSamples = 4096, kNearCols = 1024;
+__global__ void __launch_bounds__(256) near_columns_kernel(const int *__restrict__ rowptr, const int *__restrict__ colidx,
+                                                          int rows, unsigned long long *cnt) {
+  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  const int r = (int)((int64_t)w * (rows - 1) / kNearSamples);
+  const int a = rowptr[r], b = rowptr[r + 1], len = min(b - a, rowptr[r + 2] - b);
+  unsigned near = 0;
+  for (int k = lane; k < len; k += 32) near += abs(colidx[a + k] - colidx[b + k]) <= kNearCols;
+  near = __reduce_add_sync(0xffffffffu, near);
+  if (lane == 0 && len > 0) {
+    atomicAdd(cnt, (unsigned long long)near);
+    atomicAdd(cnt + 1, (unsigned long long)len);
+  }
+}
+
+// Whether neighbouring rows of A (row items) gather neighbouring entries of the
+// iterate; the pattern's, kept with the handle
+tbsla_status_t near_columns(tbsla_matrix *A, bool *near) {
+  if (!A->pr_near) {
+    unsigned long long *d = nullptr, h[2] = {0, 0};
+    if (A->rows >= 2) {
+      TB_TRY(pr_alloc((void **)&d, sizeof h));
+      cudaError_t e = cudaMemset(d, 0, sizeof h);
+      if (e == cudaSuccess)
+        near_columns_kernel<<<kNearSamples * 32 / 256, 256>>>(A->format == TBSLA_FMT_CSR ? A->idx0 : A->coo_rowptr,
+                                                              A->idx1, A->rows, d);
+      if (e == cudaSuccess) e = cudaMemcpy(h, d, sizeof h, cudaMemcpyDeviceToHost);
+      cudaFree(d);
+      TB_CUDA(e);
+    }
+    A->pr_near = h[1] && 2 * h[0] >= h[1] ? 1 : 2;
+  }
+  *near = A->pr_near == 1;
+  return TBSLA_OK;
+}
+
 struct PlanHolder {
   PrPlan p;
   ~PlanHolder() {
@@ -146,11 +184,19 @@ struct PlanHolder {
 // entries.  Large graphs: one lane a row of at most four entries (one batch),
 // 4 lanes up to 64, 8 up to 256, 32 up to half a lane's share of the sweep,
 // then chunks of eight warps: long walks by few lanes cost the fewest
-// reduction steps, but no row may outlast the sweep.  Small graphs, where a
-// warp takes an item or two a sweep: one lane up to 8, 4 up to 32, 8 up to
-// 128, 32 up to 512 entries, four batches at most (FP64 training step on
-// R-MAT 2^16 / 2^13: 1743 / 1384 us; half as long 1920 / 1546; FP32 solve on
-// 2^18 752 against 813).  Depends on the row structure only: kept with the
+// reduction steps, but no row may outlast the sweep.  Where rows of up to 16
+// entries (32, if nine tenths of the entries lie in such rows) hold half of
+// the entries, and neighbouring rows gather neighbouring entries or the rows are
+// short (of those above four entries, fewer than 10 on average), they take one
+// lane with 16-byte loads instead of four: the gathers hit L1 or L2 then, and four
+// lanes a row cost instructions, FP64 additions above all (cqmat, 2^22 rows of
+// 8, BF16: 13.1 ms with four lanes, 7.2 so; its adjoint 4.9 and 3.4; 2^22 random
+// rows of 6 on average, FP64: 4.5 and 3.8).  Random gathers of longer rows need the
+// four lanes' loads in flight (2^20 rows of 12, FP32: 1.60 ms, one lane 1.75).
+// Small graphs, where a warp takes an item or two a sweep: one lane up to 8, 4 up
+// to 32, 8 up to 128, 32 up to 512 entries, four batches at most (FP64 training
+// step on R-MAT 2^16 / 2^13: 1743 / 1384 us; half as long 1920 / 1546; FP32
+// solve on 2^18 752 against 813).  Depends on the pattern only: kept with the
 // handle across value changes.
 tbsla_status_t solver_plan(tbsla_matrix *A, const PrPlan **out) {
   if (A->pr_plan) {
@@ -161,22 +207,46 @@ tbsla_status_t solver_plan(tbsla_matrix *A, const PrPlan **out) {
   std::vector<int> rp((size_t)rows + 1);
   TB_CUDA(cudaMemcpy(rp.data(), A->format == TBSLA_FMT_CSR ? A->idx0 : A->coo_rowptr, rp.size() * sizeof(int),
                      cudaMemcpyDeviceToHost));
-  // longest row of classes 1 to 4 (32, 8, 4 lanes, one), and a chunk
   const int64_t share = A->stored / (152 * kPrThreads);
   const int per = (int)std::max<int64_t>(16, std::min<int64_t>(share / 2, 128));
   const bool small = share < 32;
-  const int limit[4] = {32 * per, small ? 128 : 256, small ? 32 : 64, small ? 8 : 4}, chunk = kPrSub * std::min(per, 32);
+  // wide items: rows of 5 to `wide` entries (none: wide = one)
+  const int one = small ? 8 : 4;
+  int wide = one;
+  if (!small) {
+    int64_t entries[2] = {0, 0}, count[2] = {0, 0};  // of rows up to 16, up to 32
+    int64_t upto32 = 0;
+    for (int r = 0; r < rows; ++r) {
+      const int len = rp[(size_t)r + 1] - rp[(size_t)r];
+      if (len > 32) continue;
+      upto32 += len;
+      for (int k = 0; k < 2; ++k)
+        if (len > one && len <= 16 << k) {
+          entries[k] += len;
+          ++count[k];
+        }
+    }
+    const int k = 10 * upto32 >= 9 * A->stored;
+    bool take = false;
+    if (2 * entries[k] >= A->stored) {
+      take = entries[k] < 10 * count[k];
+      if (!take) TB_TRY(near_columns(A, &take));
+    }
+    if (take) wide = 16 << k;
+  }
+  // longest row of 32, 8 and 4 lanes, a wide one, one of one lane, and a chunk
+  const int limit[5] = {32 * per, small ? 128 : 256, small ? 32 : 64, wide, one}, chunk = kPrSub * std::min(per, 32);
   std::vector<int4> chunk_items, chunks;
-  int count[4] = {0, 0, 0, 0};
-  auto bucket = [&](int len) { return len > limit[1] ? 0 : len > limit[2] ? 1 : len > limit[3] ? 2 : 3; };
+  int count[5] = {0, 0, 0, 0, 0};
+  auto bucket = [&](int len) { return len > limit[1] ? 0 : len > limit[2] ? 1 : len > limit[3] ? 2 : len > limit[4] ? 3 : 4; };
   int n_empty = 0;
   for (int r = 0; r < rows; ++r) {
     const int len = rp[(size_t)r + 1] - rp[(size_t)r];
     if (len == 0) ++n_empty;
     else if (len <= limit[0]) ++count[bucket(len)];
   }
-  int at[4], first[4], total = 0;
-  for (int b = 0; b < 4; ++b) {
+  int at[5], first[5], total = 0;
+  for (int b = 0; b < 5; ++b) {
     first[b] = at[b] = total;
     total += count[b];
   }
@@ -205,8 +275,11 @@ tbsla_status_t solver_plan(tbsla_matrix *A, const PrPlan **out) {
   const int nc = (int)chunk_items.size();
   p.start[0] = 0;
   p.start[1] = nc;
-  for (int c = 0; c < 3; ++c) p.start[c + 2] = nc + first[c + 1];
+  p.start[2] = nc + first[1];
+  p.start[3] = nc + first[2];
+  p.start[4] = nc + first[4];  // wide items are the last of the 4-lane class
   p.start[5] = nc + total;
+  p.n_wide = count[3];
   p.n_empty = n_empty;
   p.slots = (int)chunks.size();
   chunk_items.insert(chunk_items.end(), items.begin(), items.end());
@@ -290,15 +363,15 @@ template <typename V, typename T> unsigned barrier_polls(const tbsla_matrix *A, 
 
 constexpr int kRefProductRows = 1 << 22;
 
-template <int MODE, typename V, typename T, bool AA>
-tbsla_status_t launch_solver(const tbsla_matrix *A, const PrMat<V, T> &m, PrArgs<T> &a, const PrWork *W,
-                             cudaStream_t s) {
+template <bool kWide, int MODE, typename V, typename T, bool AA>
+tbsla_status_t launch_kind(const tbsla_matrix *A, const PrMat<V, T> &m, PrArgs<T> &a, const PrWork *W,
+                           cudaStream_t s) {
   static int per_sm[64], sms[64];
   static std::once_flag once[64];
   const int dev = A->device < 64 ? A->device : 63;
   std::call_once(once[dev], [&] {
     cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, A->device);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[dev], pr_solve_kernel<MODE, V, T, AA>, kPrThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[dev], pr_solve_kernel<kWide, MODE, V, T, AA>, kPrThreads, 0);
   });
   TB_CHECK(per_sm[dev] > 0, "the PageRank solver does not fit on the device");
   // four entries or one row per thread, all blocks resident at once
@@ -312,9 +385,16 @@ tbsla_status_t launch_solver(const tbsla_matrix *A, const PrMat<V, T> &m, PrArgs
   a.polls = barrier_polls(A, m);
   TB_CHECK(grid + (m.layout == kPrItems ? m.plan.n_chunked : 0) <= W->part_stride, "PageRank partials too small");
   void *args[] = {const_cast<PrMat<V, T> *>(&m), &a};
-  TB_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(pr_solve_kernel<MODE, V, T, AA>), dim3(grid),
+  TB_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(pr_solve_kernel<kWide, MODE, V, T, AA>), dim3(grid),
                                       dim3(kPrThreads), args, 0, s));
   return TBSLA_OK;
+}
+
+template <int MODE, typename V, typename T, bool AA>
+tbsla_status_t launch_solver(const tbsla_matrix *A, const PrMat<V, T> &m, PrArgs<T> &a, const PrWork *W,
+                             cudaStream_t s) {
+  if (m.layout == kPrItems && m.plan.n_wide > 0) return launch_kind<true, MODE, V, T, AA>(A, m, a, W, s);
+  return launch_kind<false, MODE, V, T, AA>(A, m, a, W, s);
 }
 
 // the partials: one slot per block of a full grid and per chunked row
@@ -473,11 +553,14 @@ tbsla_status_t run_f64(tbsla_matrix *A, PrWork *W, PrArgs<double> &a, int check_
   // their own labels the gathers go to DRAM, and the plain product, with twice
   // the warps per SM, is faster by more than its launch and the step cost.  R-MAT
   // of 2^20 / 2^21 / 2^22 / 2^23 / 2^24 vertices, 16 sweeps: walked 1.8 / 4.0 /
-  // 9.0 / 22.2 / 48.0 ms, by products 2.2 / 4.1 / 7.7 / 15.4 / 29.8; the ELL layout
-  // (even rows) is better walked at every size (2^24 rows, 205 sweeps: 118, 130 ms)
-  if (MODE == kSweepRef && A->n_row >= kRefProductRows && !walks_slots(A) &&
+  // 9.0 / 22.2 / 48.0 ms, by products 2.2 / 4.1 / 7.7 / 15.4 / 29.8; 2^22 random
+  // rows of 3 / 16 / 48 entries, 20 sweeps: 5.1 / 15.3 / 28.4 and 4.1 / 10.3 / 25.9.
+  // Where neighbouring rows gather neighbouring entries it is better walked at every
+  // size (2^22 banded rows of 8 / 24: 5.5 / 7.9 ms, 8.6 / 11.0 by products), as the
+  // ELL layout is (even rows; 2^24 of them, 205 sweeps: 118, 130 ms).
+  if (MODE == kSweepRef && A->n_row >= kRefProductRows && walked && !walks_slots(A) &&
       !(A->sell_width && A->values[0] && (A->short_mode == -1 || A->short_mode == 3)))
-    walked = false;
+    TB_TRY(near_columns(A, &walked));
   if (!walked && !W->prod) TB_TRY(pr_alloc((void **)&W->prod, (size_t)W->n * 8));
   PrMat<double, double> m;
   TB_TRY((solver_matrix<double, double>(A, static_cast<const double *>(A->values[0]), walked, W->prod, &m)));

@@ -13,9 +13,8 @@
 //
 // Work split: one block of 1024 threads per SM (64 registers a thread), so that
 // a barrier has few arrivals and few partial sums.  Rows are cut into classes
-// so that a lane never walks more than `per` entries (8 on small graphs, up to
-// 32 on large ones: PrPlan): 1, 4, 8 or 32 lanes a row, eight warps for a
-// chunk of a longer row.  Each class is dealt round robin over all warps of
+// so that a lane never walks more than a few batches of entries (solver_plan): 1,
+// 4, 8 or 32 lanes a row, eight warps for a chunk of a longer row.  Each class is dealt round robin over all warps of
 // the grid, beginning where the class before it ended.  A lane's entries go in
 // batches whose index loads, then gathers, are in flight together.  The groups
 // of a warp keep their sums until every lane holds a row, so the epilogue's
@@ -73,13 +72,14 @@ struct PrCtl {
 enum { kSweepRef = 0, kSweepDang = 1, kSweepInner = 2, kSweepTele = 3, kSweepAdj = 4 };
 
 // ------------------------------------------------------------ work list
-// Classes: 0 chunks of eight warps, 1 / 2 / 3: 32 / 8 / 4 lanes, 4: one lane
+// Classes: 0 chunks of eight warps, 1 / 2 / 3: 32 / 8 / 4 lanes, 4: one lane; of
+// class 3 the last n_wide items take one lane that reads 16 bytes at a time
 constexpr int kPrClasses = 5;
 struct PrPlan {
   int4 *items = nullptr;       // (row, begin, end, chunk slot or -1), class by class
   int start[kPrClasses + 1] = {0, 0, 0, 0, 0, 0};
   int *empty = nullptr;        // rows without entries
-  int n_empty = 0;
+  int n_empty = 0, n_wide = 0;
   int4 *chunks = nullptr;      // per chunk slot: (row, first slot of the row, chunks of the row, index of the row)
   int n_chunked = 0, slots = 0;
   int *arrived = nullptr;      // per chunked row: chunks summed so far (returns to 0 by itself)
@@ -320,6 +320,7 @@ template <int MODE, typename T, bool AA> struct PrEmit {
   static constexpr bool kSum = MODE == kSweepDang || MODE == kSweepInner;  // the sum is needed
   static constexpr int kBase = kSum || MODE == kSweepRef ? 3 : 2;
   static constexpr int NV = kBase + (AA ? 3 : 0);
+  static constexpr bool kAccel = AA;
   T *y;
   const T *xold;
   T *r0;
@@ -486,15 +487,107 @@ __device__ __forceinline__ void pr_sweep_groups(const PrMat<V, T> &m, const int4
   if (L > 1 && row >= 0) e.emit(row, val);
 }
 
+// Four entries from a multiple of four, those outside [a, b) with column -1 (the
+// arrays carry 64 bytes more than their entries)
+__device__ __forceinline__ void pr_ld4(const double *p, double (&v)[4]) {
+  const double2 a = __ldg(reinterpret_cast<const double2 *>(p)), b = __ldg(reinterpret_cast<const double2 *>(p + 2));
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__device__ __forceinline__ void pr_ld4(const float *p, float (&v)[4]) {
+  const float4 a = __ldg(reinterpret_cast<const float4 *>(p));
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+}
+__device__ __forceinline__ void pr_ld4(const __nv_bfloat16 *p, __nv_bfloat16 (&v)[4]) {
+  const uint2 a = __ldg(reinterpret_cast<const uint2 *>(p));
+  v[0] = __ushort_as_bfloat16((unsigned short)a.x);
+  v[1] = __ushort_as_bfloat16((unsigned short)(a.x >> 16));
+  v[2] = __ushort_as_bfloat16((unsigned short)a.y);
+  v[3] = __ushort_as_bfloat16((unsigned short)(a.y >> 16));
+}
+template <typename V>
+__device__ __forceinline__ void pr_load4(PrBatch<V> &q, const int *__restrict__ colidx, const V *__restrict__ values,
+                                         int k, int a, int b) {
+  static_assert(PrBatch<V>::U == 4, "four entries");
+  if (k < b) {
+    pr_ld4(values + k, q.v);
+    const int4 c = __ldg(reinterpret_cast<const int4 *>(colidx + k));
+    q.c[0] = c.x; q.c[1] = c.y; q.c[2] = c.z; q.c[3] = c.w;
+  }
+  #pragma unroll
+  for (int u = 0; u < 4; ++u)
+    if (k + u < a || k + u >= b) q.c[u] = -1;
+}
+
+// Short rows, one lane each, four entries with 16-byte loads at a time through L1,
+// which keeps the lines between the lanes of a warp.  FP32 and BF16 have the
+// next four (of this row or the warp's next) in flight with the gathers; in
+// FP64 and in accelerated FP32 sweeps their registers spill, the next row's
+// bounds alone are (rules and times: solver_plan).
+template <typename V, typename T, typename E>
+__device__ __forceinline__ void pr_sweep_rows(const PrMat<V, T> &m, const int4 *items, int n, int vw, int nw,
+                                              const T *x, E &e) {
+  constexpr bool kAhead = sizeof(V) < (E::kAccel ? 4 : 8);
+  const int lane = threadIdx.x & 31, step = nw * 32;
+  const int4 none = make_int4(-1, 0, 0, -1);
+  int i = vw * 32 + lane;
+  int4 it = i < n ? __ldg(items + i) : none;
+  i += step;
+  int4 nx = i < n ? __ldg(items + i) : none;
+  PrBatch<V> q;
+  T xv[4];
+  auto gather = [&]() {
+    #pragma unroll
+    for (int u = 0; u < 4; ++u) xv[u] = q.c[u] >= 0 ? x[q.c[u] - m.f_col] : T(0);
+  };
+  auto add = [&](T s) {
+    #pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (q.c[u] >= 0) s = fma_acc(to_acc(q.v[u], T()), xv[u], s);
+    return s;
+  };
+  if constexpr (kAhead) pr_load4<V>(q, m.colidx, m.values, it.y & ~3, it.y, it.z);
+  for (int base = vw * 32; base < n; base += step) {
+    T s = 0;
+    if constexpr (kAhead) {
+      i += step;
+      const int4 nn = i < n ? __ldg(items + i) : none;
+      for (int k = it.y & ~3;;) {
+        k += 4;
+        const bool more = k < it.z;
+        gather();
+        PrBatch<V> next;
+        pr_load4<V>(next, m.colidx, m.values, more ? k : nx.y & ~3, more ? it.y : nx.y, more ? it.z : nx.z);
+        s = add(s);
+        q = next;
+        if (!more) break;
+      }
+      if (it.x >= 0) e.emit(it.x, s);
+      it = nx;
+      nx = nn;
+    } else {
+      #pragma unroll 1
+      for (int k = it.y & ~3; k < it.z; k += 4) {
+        pr_load4<V>(q, m.colidx, m.values, k, it.y, it.z);
+        gather();
+        s = add(s);
+      }
+      if (it.x >= 0) e.emit(it.x, s);
+      it = nx;
+      i += step;
+      nx = i < n ? __ldg(items + i) : none;
+    }
+  }
+}
+
 // One sweep over the block's share: sums of rows to e.emit, partial sums to
 // the block's slot (chunked rows: to a slot per row after the blocks')
-template <int MODE, typename V, typename T, bool AA>
+template <bool kWide, int MODE, typename V, typename T, bool AA>
 __device__ __forceinline__ void pr_sweep(const PrMat<V, T> &m, const T *x, PrEmit<MODE, T, AA> &e, double *sh,
                                          double *partials, int stride) {
   constexpr int NV = PrEmit<MODE, T, AA>::NV;
   const int nb = gridDim.x, b = blockIdx.x;
   e.clear();
-  if (m.layout == kPrItems) {
+  if (kWide || m.layout == kPrItems) {
     const PrPlan &p = m.plan;
     // class 0: chunks, eight warps each.  The first warp of the eight adds the
     // threads' sums (in buffers used in turn, one barrier a chunk) and leaves
@@ -572,7 +665,7 @@ __device__ __forceinline__ void pr_sweep(const PrMat<V, T> &m, const T *x, PrEmi
     }
     // warp w of the grid lies in block w % nb: small classes spread over all SMs
     const int nw = nb * (kPrThreads / 32), w = (threadIdx.x >> 5) * nb + b;
-    const int n32 = p.start[2] - p.start[1], n8 = p.start[3] - p.start[2], n4 = p.start[4] - p.start[3],
+    const int n32 = p.start[2] - p.start[1], n8 = p.start[3] - p.start[2], n4 = p.start[4] - p.start[3] - (kWide ? p.n_wide : 0),
               n1 = p.start[5] - p.start[4];
     int off = (p.start[1] - p.start[0]) * (kPrSub / 32) % nw;
     auto begin = [&](int units) {  // this class's first warp is the one after the last class's last
@@ -584,6 +677,8 @@ __device__ __forceinline__ void pr_sweep(const PrMat<V, T> &m, const T *x, PrEmi
     if (n32) pr_sweep_groups<32, V, T>(m, p.items + p.start[1], n32, begin(n32), nw, x, e);
     if (n8) pr_sweep_groups<8, V, T>(m, p.items + p.start[2], n8, begin((n8 + 3) / 4), nw, x, e);
     if (n4) pr_sweep_groups<4, V, T>(m, p.items + p.start[3], n4, begin((n4 + 7) / 8), nw, x, e);
+    if constexpr (kWide)
+      pr_sweep_rows<V, T>(m, p.items + p.start[4] - p.n_wide, p.n_wide, begin((p.n_wide + 31) / 32), nw, x, e);
     if (n1) pr_sweep_groups<1, V, T>(m, p.items + p.start[4], n1, begin((n1 + 31) / 32), nw, x, e);
     const int lane = threadIdx.x & 31;
     for (int i = begin(0) * 32 + lane; i < p.n_empty; i += nw * 32) e.emit(__ldg(p.empty + i), T(0));
@@ -622,8 +717,12 @@ __device__ __forceinline__ void pr_sweep(const PrMat<V, T> &m, const T *x, PrEmi
 
 // ------------------------------------------------------------ the solver
 // MODE kSweepInner: T = float, the correction solve of the mixed-precision
-// solve; otherwise T = V = double.
-template <int MODE, typename V, typename T, bool AA>
+// solve; otherwise T = V = double.  kWide: row items with wide ones among them, in
+// a kernel of its own, since the registers of one walk cost the others (both in
+// one: R-MAT 2^23 adjoint 17.5 ms, 16.1 without).  The arguments of a launch are best
+// left in their places: four bytes more in front of the pointers of PrMat, and every
+// sweep of the 4-lane class took a tenth longer.
+template <bool kWide, int MODE, typename V, typename T, bool AA>
 __global__ void __launch_bounds__(kPrThreads, 1) pr_solve_kernel(const PrMat<V, T> m, const PrArgs<T> a) {
   constexpr bool kInner = MODE == kSweepInner;
   constexpr int NV = PrEmit<MODE, T, AA>::NV, NB = PrEmit<MODE, T, AA>::kBase;
@@ -710,7 +809,7 @@ __global__ void __launch_bounds__(kPrThreads, 1) pr_solve_kernel(const PrMat<V, 
     e.inv_n = c.inv_n;
     e.hist = MODE == kSweepRef ? !c.known : k;
     T *const yk = e.y;
-    pr_sweep<MODE, V, T, AA>(m, x, e, sh, buffer(), st);
+    pr_sweep<kWide, MODE, V, T, AA>(m, x, e, sh, buffer(), st);
     const int nparts = nb + (m.layout == kPrItems ? m.plan.n_chunked : 0);
     if (!meet(VN{}, nparts, MODE == kSweepRef, [&](const double (&v)[NV]) {
           if constexpr (MODE == kSweepRef) {
