@@ -12,7 +12,7 @@
 //     its stored order with one FMA per nonzero (the order of
 //     MatrixCSR::Ax, src/cpp/matrix/MatrixCSR.cpp:133-139).
 //   long (<= kChunk): a group of L lanes per row, L = 4, 8, 32 or a block of
-//     256 by length class (kGroupLimit), lanes striding the row, partial sums
+//     256 by length class (kGroupLimit, kManyLimit), lanes striding the row, partial sums
 //     combined in a fixed order inside the group.
 //   huge (> kChunk): the row is cut into chunks of kChunk nonzeros, a block
 //     per chunk writing a partial; csr_chunk_fixup_kernel adds the partials of
@@ -40,6 +40,13 @@ constexpr int kChunk = 8192;
 constexpr int kGroupClasses = 4;
 constexpr int kGroupLimit[kGroupClasses] = {96, 256, 1024, kChunk};
 constexpr int kGroupLanes[kGroupClasses] = {4, 8, 32, 256};
+// Rows of up to 1792 entries join the class of 32 lanes where there are as many as
+// fill the GPU with warps: a block a row leaves much of its time to the sums of
+// the lanes (rows of 1500 entries, 32 lanes / a block: 16384 of them 64 / 77 us in
+// FP64, 46 / 51 in FP32, 45 / 56 in BF16; 30000 168 / 155, 78 / 89, 75 / 98; 8000 34 /
+// 42 and 28 / 28; 4000 24 / 26 and 18 / 15).  Of 2000 entries 30000 rows take
+// 224 us in FP64 by 32 lanes, 206 by blocks.
+constexpr int kManyRows = 8192, kManyLimit = 1792;
 
 __device__ __forceinline__ float bf16_lo(unsigned w) { return __bfloat162float(__ushort_as_bfloat16((unsigned short)(w & 0xffffu))); }
 __device__ __forceinline__ float bf16_hi(unsigned w) { return __bfloat162float(__ushort_as_bfloat16((unsigned short)(w >> 16))); }
@@ -251,6 +258,23 @@ __global__ void __launch_bounds__(256) csr_tiny_kernel(int n_rows, const int *__
   }
 }
 
+// The same share without the next step's loads in flight, for FP64 and FP32 groups
+// of a whole warp where there are thousands (kPlainItems): the loads of the SM's other
+// warps overlap with it, and the shorter loop wins (16384 rows of 900 entries: 44
+// us against 49 in FP64, 31.5 / 34.2 in FP32).  With fewer of them, narrower
+// groups and BF16 the loads ahead stay (R-MAT 2^16 FP64: 15.3 us, 17.8 without; 2^20
+// banded rows of 48, FP32: 103, 121; 16384 rows of 900, BF16: 29.6, 31.5).
+template <int L, typename V, typename XT, typename Acc>
+__device__ __forceinline__ Acc range_sum_plain(const int *__restrict__ colidx, const V *__restrict__ values,
+                                               const XT *__restrict__ x, int f_col, int a, int b, int lane,
+                                               uint64_t keep) {
+  Acc acc = 0;
+  #pragma unroll 4
+  for (int64_t k = (int64_t)a + lane; k < b; k += L)
+    acc = fma_acc(to_acc(ld_stream(values + k), Acc()), to_acc(ld_keep(x + (ld_stream(colidx + k) - f_col), keep), Acc()), acc);
+  return acc;
+}
+
 // A lane's share of entries [a, b) of a group of L lanes: entries a + lane,
 // a + lane + L, ..., one FMA per entry in that order.  Four entries go
 // together, their gathers in flight with the next four's columns and values.
@@ -293,14 +317,15 @@ __device__ __forceinline__ Acc range_sum_lane(const int *__restrict__ colidx, co
 // first + n) dealt 256 / L to a block: items[i] = (row, begin, end, partial
 // slot or -1).  A warp holds 32/L groups, so its FP64 reduction steps and the
 // epilogue serve 32/L rows at once.
-template <int L, typename V, typename XT, typename Epi>
+template <int L, bool kPlain, typename V, typename XT, typename Epi>
 __device__ __forceinline__ void mixed_group(const int4 *__restrict__ items, int n, int block,
                                             const int *__restrict__ colidx, const V *__restrict__ values,
                                             const XT *__restrict__ x, int f_col, uint64_t keep, const Epi &epi) {
   using Acc = typename Epi::Acc;
   const int i = block * (256 / L) + (int)threadIdx.x / L, lane = threadIdx.x & (L - 1);
   const int4 it = i < n ? __ldg(items + i) : make_int4(-1, 0, 0, -1);
-  Acc s = range_sum_lane<L, V, XT, Acc>(colidx, values, x, f_col, it.y, it.z, lane, keep);
+  Acc s = kPlain ? range_sum_plain<L, V, XT, Acc>(colidx, values, x, f_col, it.y, it.z, lane, keep)
+                 : range_sum_lane<L, V, XT, Acc>(colidx, values, x, f_col, it.y, it.z, lane, keep);
   #pragma unroll
   for (int o = L / 2; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, L);
   if (lane == 0 && it.x >= 0) epi.emit(it.x, s);
@@ -322,7 +347,9 @@ struct MixedPlan {
   int n_short;
 };
 
-template <bool kPair, typename V, typename XT, typename Epi>
+constexpr int kPlainItems = 152 * 32;  // 32-lane items: a warp for half of the SMs' places
+
+template <bool kPair, bool kPlain, typename V, typename XT, typename Epi>
 __global__ void __launch_bounds__(256) csr_mixed_kernel(const MixedPlan p, const int *__restrict__ rowptr,
                                                        const int *__restrict__ colidx, const V *__restrict__ values,
                                                        const XT *__restrict__ x, int f_col, XKeep x_keep,
@@ -333,7 +360,11 @@ __global__ void __launch_bounds__(256) csr_mixed_kernel(const MixedPlan p, const
   const int b = blockIdx.x;
   if (b < p.first[2]) {
     const int4 it = __ldg(p.items + p.start[3] + b);
-    part[threadIdx.x] = range_sum_lane<256, V, XT, Acc>(colidx, values, x, f_col, it.y, it.z, threadIdx.x, keep);
+    // FP64 without the loads ahead (16384 rows of 5000 entries: 173 us, 188 with; FP32 130, 120)
+    if constexpr (sizeof(V) == 8)
+      part[threadIdx.x] = range_sum_plain<256, V, XT, Acc>(colidx, values, x, f_col, it.y, it.z, threadIdx.x, keep);
+    else
+      part[threadIdx.x] = range_sum_lane<256, V, XT, Acc>(colidx, values, x, f_col, it.y, it.z, threadIdx.x, keep);
     __syncthreads();
     if (threadIdx.x < 32) {
       Acc s = part[threadIdx.x];
@@ -347,11 +378,11 @@ __global__ void __launch_bounds__(256) csr_mixed_kernel(const MixedPlan p, const
       }
     }
   } else if (b < p.first[1]) {
-    mixed_group<32, V, XT, Epi>(p.items + p.start[2], p.start[3] - p.start[2], b - p.first[2], colidx, values, x, f_col, keep, epi);
+    mixed_group<32, kPlain, V, XT, Epi>(p.items + p.start[2], p.start[3] - p.start[2], b - p.first[2], colidx, values, x, f_col, keep, epi);
   } else if (b < p.first[0]) {
-    mixed_group<8, V, XT, Epi>(p.items + p.start[1], p.start[2] - p.start[1], b - p.first[1], colidx, values, x, f_col, keep, epi);
+    mixed_group<8, false, V, XT, Epi>(p.items + p.start[1], p.start[2] - p.start[1], b - p.first[1], colidx, values, x, f_col, keep, epi);
   } else if (b < p.first[4]) {
-    mixed_group<4, V, XT, Epi>(p.items + p.start[0], p.start[1] - p.start[0], b - p.first[0], colidx, values, x, f_col, keep, epi);
+    mixed_group<4, false, V, XT, Epi>(p.items + p.start[0], p.start[1] - p.start[0], b - p.first[0], colidx, values, x, f_col, keep, epi);
   } else if constexpr (kPair) {
     const int64_t t = ((int64_t)(b - p.first[4]) * 256 + threadIdx.x) >> 1;
     const int half = threadIdx.x & 1;

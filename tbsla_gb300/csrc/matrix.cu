@@ -626,6 +626,13 @@ tbsla_status_t csr_bins(tbsla_matrix *A, const std::vector<int> &rp) {
     bool all_short = true;
     int64_t short_nnz = 0;
     int short_max = 0;
+    int limit[kGroupClasses], many = 0;
+    std::copy(kGroupLimit, kGroupLimit + kGroupClasses, limit);
+    for (int r = 0; r < rows; ++r) {
+      const int len = rp[r + 1] - rp[r];
+      many += len > limit[2] && len <= kManyLimit;
+    }
+    if (many >= kManyRows) limit[2] = kManyLimit;
     for (int r = 0; r < rows; ++r) {
       const int len = rp[r + 1] - rp[r];
       if (len <= kShortRow) {
@@ -637,7 +644,7 @@ tbsla_status_t csr_bins(tbsla_matrix *A, const std::vector<int> &rp) {
       all_short = false;
       if (len <= kChunk) {
         int c = 0;
-        while (len > kGroupLimit[c]) ++c;
+        while (len > limit[c]) ++c;
         cls[c].push_back(make_int4(r, rp[r], rp[r + 1], -1));
         continue;
       }

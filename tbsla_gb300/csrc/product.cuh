@@ -168,12 +168,12 @@ tbsla_status_t launch_csr_direct(const tbsla_matrix *A, const int *rowptr, const
     p.first[kGroupClasses] = blocks;
     Acc *parts = chunk_partials_of<Acc>(A);
     if (A->n_short > 0) blocks += short_grid((pair ? 2 : 1) * (int64_t)A->n_short);
-    if (pair)
-      csr_mixed_kernel<true, V, XT, Epi><<<blocks, 256, 0, s>>>(p, rowptr, colidx, vals, x, A->f_col, xkeep_of<XT>(A),
-                                                               parts, epi);
-    else
-      csr_mixed_kernel<false, V, XT, Epi><<<blocks, 256, 0, s>>>(p, rowptr, colidx, vals, x, A->f_col, xkeep_of<XT>(A),
-                                                                parts, epi);
+    const bool plain = sizeof(V) >= 4 && p.start[3] - p.start[2] >= kPlainItems;
+    auto launch = [&](auto kernel) {
+      kernel<<<blocks, 256, 0, s>>>(p, rowptr, colidx, vals, x, A->f_col, xkeep_of<XT>(A), parts, epi);
+    };
+    if (pair) launch(plain ? csr_mixed_kernel<true, true, V, XT, Epi> : csr_mixed_kernel<true, false, V, XT, Epi>);
+    else launch(plain ? csr_mixed_kernel<false, true, V, XT, Epi> : csr_mixed_kernel<false, false, V, XT, Epi>);
   }
   kt.stop();
   if (A->n_chunk_rows > 0) {
