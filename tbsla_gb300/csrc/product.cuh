@@ -183,6 +183,29 @@ tbsla_status_t launch_csr_direct(const tbsla_matrix *A, const int *rowptr, const
   return TBSLA_OK;
 }
 
+// DENSE products by dense_rows_kernel: few columns, and for FP32 and BF16 64 rows an
+// SM (16 warps of four; with fewer the batches and splits of dense_kernel fill
+// the GPU as well or better: 5000 x 256 FP32 5.5 us, here 6.8).  FP32 and BF16 up
+// to 192 columns (10000 rows: 128 columns 5.9 us by dense_kernel, 5.4 here; 400 6.7 and
+// 7.7), from 16384 rows 320 (20000 x 256 7.9, 6.9; 384 9.0, 9.8), from 32768,
+// whose matrix leaves L2, 512 in FP32 (65536 rows 30.4, 26.5) and 400 in BF16 (384:
+// 17.0, 13.7); BF16 whose rows do not start on 16 bytes up to 2048 (20000 x 1500
+// 21.0, 16.0).  FP64, whose pipe is the bound, counts steps of 32 columns here and
+// pairs of them there, and loses occupancy to dense_kernel's registers: up to 192
+// columns (1500 x 128 7.9, 7.0; 256 7.3, 8.6), from 64 rows an SM 288 (20000 x 257
+// 25.6, 23.9; 10000 x 512 19.8, 21.5), from 32768 rows always (33554 x 1000 89.7,
+// 79.3; 20000 x 1500 70.5, 75.3), but not where the last, partial step is one of
+// few (335544 x 100 180, 232).
+template <typename V> inline bool dense_by_rows(int rows, int cols, bool vec) {
+  if (sizeof(V) == 8) {
+    if (cols % 32 != 0 && cols < 128 && 2 * ((cols + 63) / 64) == (cols + 31) / 32) return false;
+    return cols <= (rows < 64 * 152 ? 192 : 288) || rows >= 32768;
+  }
+  if (rows < 64 * 152) return false;
+  if (sizeof(V) == 2 && !vec) return cols <= 2048;
+  return cols <= (rows >= 32768 ? (sizeof(V) == 4 ? 512 : 400) : rows >= 16384 ? 320 : 192);
+}
+
 template <typename V, typename XT, typename Epi>
 tbsla_status_t launch_product(const tbsla_matrix *A, const V *vals, const XT *x, Epi epi,
                               cudaStream_t s) {
@@ -261,6 +284,12 @@ tbsla_status_t launch_product(const tbsla_matrix *A, const V *vals, const XT *x,
       // 16-byte loads when every row and x start on 16 bytes
       constexpr int VW = 16 / (int)sizeof(V);
       const bool vec = A->cols % VW == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+      KernelTimer kt(A, s);
+      if (dense_by_rows<V>(A->rows, A->cols, vec)) {
+        dense_rows_kernel<V, XT, Epi><<<(int)(((int64_t)A->rows + 31) / 32), 256, 0, s>>>(vals, x, A->rows, A->cols, epi);
+        kt.stop();
+        break;
+      }
       // warps per row group: as many as leave each four steps of columns, so
       // that blocks are short and many (8000 x 9001 FP64 in blocks of 35 steps,
       // one wave and a tenth: 281 us, against 175 with few, long blocks)
@@ -270,7 +299,6 @@ tbsla_status_t launch_product(const tbsla_matrix *A, const V *vals, const XT *x,
       while (splits < 8 && A->cols / (2 * splits) >= 4 * batch) splits *= 2;
       while (splits < 8 && groups * splits < 152 * 6 && A->cols / (2 * splits) >= 128) splits *= 2;
       const int grid = (int)((groups * splits + 7) / 8);
-      KernelTimer kt(A, s);
       if (vec) dense_kernel<VW, V, XT, Epi><<<grid, 256, 0, s>>>(vals, x, A->rows, A->cols, splits, epi);
       else dense_kernel<1, V, XT, Epi><<<grid, 256, 0, s>>>(vals, x, A->rows, A->cols, splits, epi);
       kt.stop();
