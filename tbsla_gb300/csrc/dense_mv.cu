@@ -231,27 +231,56 @@ __global__ void x_to_bf16_kernel(const float *__restrict__ x, int rows, int k, i
   }
 }
 
-// rows x cols row-major elements (ld src_ld) copied to ld dst_ld: a warp takes
-// 32 kPad consecutive elements of a row, kPad of a lane in flight.  A byte per
-// thread and step took 138 us for 65 MB (8094 x 2009 FP32), nine times the
-// product itself.
-constexpr int kPad = 8;
-template <typename E>
+// rows x cols row-major elements (ld src_ld) copied to ld dst_ld, kPad of a lane in
+// flight: a warp takes 32 kPad consecutive elements of a row.  A byte per thread
+// and step took 138 us for 65 MB (8094 x 2009 FP32), nine times the product
+// itself.  Rows under kNarrow elements would fill a few of its lanes: there it takes
+// 32 kPad consecutive elements whatever their rows (the product of 2000000 x 3
+// with 8 vectors, FP32: 417 us by rows, 207 byte by byte, 177 so; of 100000 x 17
+// 54 and 48; x 63 the same; x 130 72 by rows, 96 so: a division an element).
+constexpr int kPad = 8, kNarrow = 64;
+template <typename E, bool kFlat>
 __global__ void __launch_bounds__(256) pad_rows_kernel(const E *__restrict__ src, int64_t rows, int64_t cols,
                                                       int64_t src_ld, E *__restrict__ dst, int64_t dst_ld) {
-  const int64_t per_row = (cols + 32 * kPad - 1) / (32 * kPad), tasks = rows * per_row;
+  const int64_t per_row = (cols + 32 * kPad - 1) / (32 * kPad);
+  const int64_t tasks = kFlat ? (rows * cols + 32 * kPad - 1) / (32 * kPad) : rows * per_row;
   const int lane = threadIdx.x & 31;
   for (int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < tasks;
        t += ((int64_t)gridDim.x * blockDim.x) >> 5) {
-    const int64_t r = t / per_row, c0 = (t - r * per_row) * (32 * kPad) + lane;
     E v[kPad];
-    #pragma unroll
-    for (int u = 0; u < kPad; ++u)
-      if (c0 + 32 * u < cols) v[u] = __ldg(src + r * src_ld + c0 + 32 * u);
-    #pragma unroll
-    for (int u = 0; u < kPad; ++u)
-      if (c0 + 32 * u < cols) dst[r * dst_ld + c0 + 32 * u] = v[u];
+    if constexpr (kFlat) {
+      // the first element's row by one division, the others' from there
+      const int64_t e0 = t * (32 * kPad), r0 = e0 / cols;
+      const unsigned c0 = (unsigned)(e0 - r0 * cols) + lane, w = (unsigned)cols;
+      const int64_t left = rows * cols - e0;
+      #pragma unroll
+      for (int u = 0; u < kPad; ++u) {
+        const unsigned c = c0 + 32 * u;
+        if (lane + 32 * u < left) v[u] = __ldg(src + (r0 + c / w) * src_ld + c % w);
+      }
+      #pragma unroll
+      for (int u = 0; u < kPad; ++u) {
+        const unsigned c = c0 + 32 * u;
+        if (lane + 32 * u < left) dst[(r0 + c / w) * dst_ld + c % w] = v[u];
+      }
+    } else {
+      const int64_t r = t / per_row, c0 = (t - r * per_row) * (32 * kPad) + lane;
+      #pragma unroll
+      for (int u = 0; u < kPad; ++u)
+        if (c0 + 32 * u < cols) v[u] = __ldg(src + r * src_ld + c0 + 32 * u);
+      #pragma unroll
+      for (int u = 0; u < kPad; ++u)
+        if (c0 + 32 * u < cols) dst[r * dst_ld + c0 + 32 * u] = v[u];
+    }
   }
+}
+template <typename E>
+static void pad_rows(const void *src, int64_t rows, int64_t cols, int64_t src_ld, void *dst, int64_t dst_ld,
+                     cudaStream_t s) {
+  const E *a = static_cast<const E *>(src);
+  E *b = static_cast<E *>(dst);
+  if (cols < kNarrow) pad_rows_kernel<E, true><<<152 * 8, 256, 0, s>>>(a, rows, cols, src_ld, b, dst_ld);
+  else pad_rows_kernel<E, false><<<152 * 8, 256, 0, s>>>(a, rows, cols, src_ld, b, dst_ld);
 }
 
 tbsla_status_t encode_map(CUtensorMap *map, bool bf16, const void *base, int64_t inner, int64_t outer,
@@ -347,12 +376,8 @@ tbsla_status_t dense_spmm_tc(tbsla_matrix *A, bool bf16, int k, const float *X, 
   if ((K % align) != 0 || (reinterpret_cast<uintptr_t>(a) & 15) != 0) {
     lda = (K + align - 1) / align * align;
     TB_CUDA(cudaMallocAsync(&a_pad, (size_t)M * lda * es, s));
-    if (bf16)
-      pad_rows_kernel<uint16_t><<<152 * 8, 256, 0, s>>>(static_cast<const uint16_t *>(a), M, K, K,
-                                                        static_cast<uint16_t *>(a_pad), lda);
-    else
-      pad_rows_kernel<uint32_t><<<152 * 8, 256, 0, s>>>(static_cast<const uint32_t *>(a), M, K, K,
-                                                        static_cast<uint32_t *>(a_pad), lda);
+    if (bf16) pad_rows<uint16_t>(a, M, K, K, a_pad, lda, s);
+    else pad_rows<uint32_t>(a, M, K, K, a_pad, lda, s);
     a = a_pad;
   }
   // X: BF16 copy for the BF16 store; for F32 the caller's X when its vectors
@@ -368,8 +393,7 @@ tbsla_status_t dense_spmm_tc(tbsla_matrix *A, bool bf16, int k, const float *X, 
       x_to_bf16_kernel<<<dim3(gx, std::min(k, 65535)), 256, 0, s>>>(X, K, k, ldx,
                                                                     static_cast<__nv_bfloat16 *>(x_buf), ldxe, vec4);
     } else {
-      pad_rows_kernel<uint32_t><<<152 * 8, 256, 0, s>>>(reinterpret_cast<const uint32_t *>(X), k, K, ldx,
-                                                        static_cast<uint32_t *>(x_buf), ldxe);
+      pad_rows<uint32_t>(X, k, K, ldx, x_buf, ldxe, s);
     }
     x = x_buf;
   }
