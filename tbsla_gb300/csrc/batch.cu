@@ -42,7 +42,13 @@ constexpr int kBatchRows = 256;
 // The block-uniform item loop carries the next item's descriptor and member
 // entry (and its mask flag) one iteration ahead: their dependent loads
 // overlap the current rows' sums instead of preceding them.
-template <typename V, typename T>
+// kTwo: items of two rows per thread for members with an ELL-layout copy; else of
+// one, with eight slots of it in flight, since half of the two-row loop is left
+// idle by one row (two members of 60000 rows of 30 entries, FP64: 23.2 us by it,
+// 19.6 from the CSR arrays, 17.1 so).  Two kernels, since the registers of either loop
+// cost the other warps (8 members of 60000 rows of 16, both in one: 25 us became
+// 40).
+template <bool kTwo, typename V, typename T>
 __global__ void __launch_bounds__(256) batch_spmv_kernel(const BatchMember *__restrict__ members,
                                                         const int4 *__restrict__ items, int n_items,
                                                         const int *__restrict__ mask) {
@@ -67,7 +73,29 @@ __global__ void __launch_bounds__(256) batch_spmv_kernel(const BatchMember *__re
       T *y = static_cast<T *>(m.y);
       const T *x = static_cast<const T *>(m.x);
       const int ra = w.y + (int)threadIdx.x, rb = ra + kBatchRows;
-      if (m.sell_vals) {
+      if (!kTwo && m.sell_vals) {
+        const V *sv = static_cast<const V *>(m.sell_vals);
+        const bool ha = ra < w.z && ra < m.rows;
+        Acc sa = 0;
+        for (int j0 = 0; j0 < m.sell_width; j0 += 8) {
+          int c[8];
+          V v[8];
+          Acc xv[8];
+          #pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const bool in = ha && j0 + u < m.sell_width;
+            const size_t at = (size_t)(j0 + u) * m.sell_stride + ra;
+            c[u] = in ? ld_ell<false>(m.sell_cols + at) : -1;
+            v[u] = in ? ld_ell<false>(sv + at) : V(0);
+          }
+          #pragma unroll
+          for (int u = 0; u < 8; ++u) xv[u] = c[u] >= 0 ? to_acc(ld_keep(x + (c[u] - m.f_col), keep), Acc()) : Acc(0);
+          #pragma unroll
+          for (int u = 0; u < 8; ++u)
+            if (c[u] >= 0) sa = fma_acc(to_acc(v[u], Acc()), xv[u], sa);
+        }
+        if (ra < w.z) __stcs(y + ra, (T)sa);
+      } else if (m.sell_vals) {
         // rows ra and rb from the ELL-layout copy, slot by slot (padding and
         // rows past m.rows hold column -1 or are not read)
         const V *sv = static_cast<const V *>(m.sell_vals);
@@ -116,6 +144,7 @@ struct tbsla_batch {
   BatchMember *d_table = nullptr;
   int4 *d_items = nullptr;
   int n_items = 0;
+  bool two_rows = false;             // items of two rows per thread for members with an ELL-layout copy
   const int *d_mask = nullptr;       // caller's mask or NULL
   // persistent grid: 152 x blocks_per_sm (tbsla_batch_tune; 0: 12, or 6 when
   // there are fewer items than that holds).  64 cqmat matrices of up to 1e5
@@ -137,12 +166,10 @@ static tbsla_status_t batch_launch(tbsla_batch *B, tbsla_dtype_t store, cudaStre
   if (B->n_items == 0) return TBSLA_OK;
   const int per_sm = B->blocks_per_sm ? B->blocks_per_sm : B->n_items >= 152 * 12 ? 12 : 6;
   const int grid = std::max(1, std::min(B->n_items, 152 * per_sm));
-  if (store == TBSLA_F64)
-    batch_spmv_kernel<double, double><<<grid, 256, 0, s>>>(B->d_table, B->d_items, B->n_items, B->d_mask);
-  else if (store == TBSLA_F32)
-    batch_spmv_kernel<float, float><<<grid, 256, 0, s>>>(B->d_table, B->d_items, B->n_items, B->d_mask);
-  else
-    batch_spmv_kernel<__nv_bfloat16, float><<<grid, 256, 0, s>>>(B->d_table, B->d_items, B->n_items, B->d_mask);
+  auto launch = [&](auto kernel) { kernel<<<grid, 256, 0, s>>>(B->d_table, B->d_items, B->n_items, B->d_mask); };
+  if (store == TBSLA_F64) launch(B->two_rows ? batch_spmv_kernel<true, double, double> : batch_spmv_kernel<false, double, double>);
+  else if (store == TBSLA_F32) launch(B->two_rows ? batch_spmv_kernel<true, float, float> : batch_spmv_kernel<false, float, float>);
+  else launch(batch_spmv_kernel<true, __nv_bfloat16, float>);  // no copies: the CSR arrays
   TB_CUDA(cudaGetLastError());
   return TBSLA_OK;
 }
@@ -184,10 +211,11 @@ tbsla_status_t tbsla_batch_create(int count, const tbsla_matrix_t *const *member
   // batch would not give every SM a few items
   int64_t pairs = 0;
   for (const tbsla_matrix *A : B->members) pairs += (A->n_row + 2 * kBatchRows - 1) / (2 * kBatchRows);
+  B->two_rows = pairs >= 152 * 4;
   for (int m = 0; m < count; ++m) {
     const tbsla_matrix *A = B->members[(size_t)m];
     const int n_row = A->n_row;
-    const int span = (A->sell_width || batch_copy_wanted(A)) && pairs >= 152 * 4 ? 2 * kBatchRows : kBatchRows;
+    const int span = (A->sell_width || batch_copy_wanted(A)) && B->two_rows ? 2 * kBatchRows : kBatchRows;
     for (int r = 0; r < n_row; r += span) items.push_back(make_int4(m, r, std::min(r + span, n_row), 0));
   }
   B->n_items = (int)items.size();
