@@ -154,7 +154,8 @@ tbsla_status_t tbsla_matrix_destroy(tbsla_matrix_t *A);
  * over a derived row pointer, 1 = merge path.  ELL: 0 = warp tiles of 128
  * rows, lane l taking rows l, l+32, l+64, l+96, the default; 1 = four
  * consecutive rows per thread, bit-identical results).  Results agree within
- * the FP64 bound of the parity tests; the choice only changes speed. */
+ * the FP64 bound of the parity tests; the choice only changes speed.  PageRank
+ * solves walk the same arrays whatever it is. */
 tbsla_status_t tbsla_matrix_set_variant(tbsla_matrix_t *A, int variant);
 
 /* Tunable knobs of a handle's kernels (what the autotuner sets); results do

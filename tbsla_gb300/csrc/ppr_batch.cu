@@ -6,12 +6,12 @@
 // gather of a column index brings all KT values in one contiguous segment.
 // A group of G lanes sums a row, each lane VW consecutive vectors (16 bytes
 // of the tile row): no cross-lane reduction, every lane does useful
-// multiply-adds, and a warp sweeps 32 / G rows at once.  Rows longer than
-// kPprChunk entries are cut into chunks (partials + a fixup kernel) so that
+// multiply-adds, and a warp sweeps 32 / G rows at once.  Rows longer than a
+// chunk (PprPlan) are cut into chunks (partials + a fixup kernel) so that
 // hub rows of power-law graphs spread over many groups.  The FP64 sweeps are
-// bound by the FP64 pipe (2 operations per clock per SM): a 32-vector sweep
-// of R-MAT 2^20 (5.2e8 FMAs and the epilogue's FP64 work) keeps it 90 % busy
-// while DRAM runs at 10 %.
+// bound by the FP64 pipe (2 operations per clock per SM: 64 vectors of R-MAT 2^17
+// keep it 87 % busy, DRAM 12 %), the FP32 ones by the latency of their gathers
+// (FP64 pipe 57 %: the dangling mass; L1 46 %).
 //
 // Anderson acceleration (p->accel = 1), per vector as in the one-vector
 // solve: the sweep writes its output g and residual r = g - x into rings of
@@ -682,12 +682,6 @@ __global__ void ppr_seed_bits_kernel(unsigned *seeds, int n, const int2 *__restr
   }
 }
 
-// The work list of a handle's batched sweeps in decreasing length: rows, and
-// rows longer than a chunk cut into chunks; built once (it depends on the row
-// structure only) and kept on the handle.  A chunk is walked by one row group,
-// so it is a 16384th of the entries, 64 to 512: on small graphs a long chunk
-// outlasts the sweep (R-MAT 2^17, 32 FP32 vectors: 179 us a sweep with chunks
-// of 512 entries), on large ones short chunks only cost partial sums.
 // Device memory kept with the handle between solves (allocating and freeing a
 // solve's two dozen buffers took a third of a 64-vector solve on R-MAT 2^17:
 // six FP32 and FP64 solves of a refined one).  One solve holds it at a time,
@@ -760,6 +754,12 @@ class PprBuffers {
   std::vector<std::pair<void **, size_t>> req_;
 };
 
+// The work list of a handle's batched sweeps in decreasing length: rows, and
+// rows longer than a chunk cut into chunks; built once (it depends on the row
+// structure only) and kept on the handle.  A chunk is walked by one row group,
+// so it is a 16384th of the entries, 64 to 512: on small graphs a long chunk
+// outlasts the sweep (R-MAT 2^17, 32 FP32 vectors: 179 us a sweep with chunks
+// of 512 entries), on large ones short chunks only cost partial sums.
 struct PprPlan {
   PprMemory solve, refine;  // buffers of a solve, and of the refinement around it
   int4 *items = nullptr;  // (row, begin, end, chunk slot or -1)
