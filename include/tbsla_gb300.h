@@ -18,8 +18,12 @@
  *
  * Threading: a handle may be used from several threads for reads (spmv and
  * transposed products on device pointers, batched PageRank solves; the copies
- * and plans they build on first use are built once); the *_host entry points use the handle's own stream and
- * staging buffers and must not run concurrently on one handle.
+ * and plans they build on first use are built once).  Products of rows above
+ * 8192 entries and of the merge-path and row-block variants keep partial sums
+ * with the handle: on different streams they must not overlap.  The *_host entry
+ * points use the handle's own stream and staging buffers and must not run
+ * concurrently on one handle, nor must the one-vector PageRank solves, which
+ * use its workspace.
  */
 #ifndef TBSLA_GB300_H
 #define TBSLA_GB300_H
